@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/mf_patch.h"
+#include "mf_ieee64.cuh"
 
 namespace mf {
 
@@ -174,6 +175,9 @@ template <typename R> __device__ __forceinline__ R rmax(R a, R b) { return fmax(
 template <typename R> __device__ __forceinline__ R rmin(R a, R b) { return fmin(a, b); }
 template <typename R> __device__ __forceinline__ R rabs(R a) { return fabs(a); }
 template <typename R> __device__ __forceinline__ R sqrt_r(R a) { return sqrt(a); }
+template <typename R> __device__ __forceinline__ R half_r(R a);
+template <> __device__ __forceinline__ float half_r<float>(float a) { return 0.5f * a; }
+template <> __device__ __forceinline__ double half_r<double>(double a) { return ieee64::half(a); }
 
 // ---------------------------------------------------------------------------
 // VFRoe MHD flux: VFROE_FLUXES (src/VFRoeF.ChF:327-658) with arithmetic
@@ -302,28 +306,28 @@ __device__ __forceinline__ void vfroe_mhd(const DevParams& P, const R* wl, const
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cons_to_prim_plasma(const DevParams& P, const double* u,
                                                     double* w) {
-  double rho = (P.nf == 1) ? u[0] : fmax(u[0], P.smallr);
+  double rho = (P.nf == 1) ? u[0] : ieee64::maxnum(u[0], P.smallr);
   double ru = u[1], rv = u[2], rw = u[3];
-  double invrho = 1.0 / rho;
+  double invrho = ieee64::div(1.0, rho);
   double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
   double ke = ru * uu + rv * vv + rw * ww;
   double bx = u[5], by = u[6], bz = u[7];
   double b = kInv4Pi * (bx * bx + by * by + bz * bz);
-  double p = P.hgamma * (u[4] - 0.5 * (ke + b));
-  p = fmax(p, P.smallp);
+  double p = P.hgamma * (u[4] - ieee64::half(ke + b));
+  p = ieee64::maxnum(p, P.smallp);
   w[0] = rho; w[1] = uu; w[2] = vv; w[3] = ww; w[4] = p;
   w[5] = bx; w[6] = by; w[7] = bz;
 }
 
 __device__ __forceinline__ void cons_to_prim_euler(const DevParams& P, const double* u,
                                                    double* w) {
-  double rho = fmax(u[0], P.smallr);
+  double rho = ieee64::maxnum(u[0], P.smallr);
   double ru = u[1], rv = u[2], rw = u[3];
-  double invrho = 1.0 / rho;
+  double invrho = ieee64::div(1.0, rho);
   double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
   double ke = ru * uu + rv * vv + rw * ww;
-  double p = P.hgamma * (u[4] - 0.5 * ke);
-  p = fmax(p, P.smallp);
+  double p = P.hgamma * (u[4] - ieee64::half(ke));
+  p = ieee64::maxnum(p, P.smallp);
   w[0] = rho; w[1] = uu; w[2] = vv; w[3] = ww; w[4] = p;
 }
 
@@ -437,6 +441,14 @@ __device__ __forceinline__ void face_values(int lim, R wm1, R wp, R wp1, R& lo, 
       return;
     }
     default:  // MINMODFACEVALUES :126-155
+      if constexpr (sizeof(R) == sizeof(double)) {
+        // the limiter on the integer pipes; half the slope is exact, so the
+        // fused form rounds once, as the sum of the halved slope does
+        const R m = ieee64::minmod(dWR, dWL);
+        lo = fma(-0.5, m, wp);
+        hi = fma(0.5, m, wp);
+        return;
+      }
       slope = R(0.5) * minmod_<R>(dWR, dWL);
       break;
   }

@@ -414,7 +414,7 @@ __device__ __forceinline__ void flux_face(const DevParams& P, const double* __re
   // face-normal B (PatchMHDMF::computeBn, srcIdeal/PatchMHDMF.cpp:509-620)
   R bn = R(0);
   if (P.divb_method == 1) {
-    bn = R(0.5) * (wl[5 + DIR] + wr[5 + DIR]);
+    bn = half_r<R>(wl[5 + DIR] + wr[5 + DIR]);
     if (!P.periodic[DIR]) {
       const int f = (DIR == 0) ? i : (DIR == 1) ? j : k;
       if (f == RP.dlo[DIR]) bn = wr[5 + DIR];
@@ -536,7 +536,7 @@ __device__ __forceinline__ void riemann_face(const DevParams& P, const RunParams
   }
   R bn = R(0);
   if (P.divb_method == 1) {
-    bn = R(0.5) * (wl[5 + DIR] + wr[5 + DIR]);
+    bn = half_r<R>(wl[5 + DIR] + wr[5 + DIR]);
     if (!P.periodic[DIR]) {
       const int f = (DIR == 0) ? i : (DIR == 1) ? j : k;
       if (f == RP.dlo[DIR]) bn = wr[5 + DIR];

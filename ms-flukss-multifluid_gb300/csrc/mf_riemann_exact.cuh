@@ -16,244 +16,245 @@ namespace exact {
 // RIEMANN7F (src/Roe7WaveF.ChF:5-558).  wl/wr: rho,u,v,w,p,bx,by,bz in the
 // global frame; g: fluxes in the same order.  SEVEN drops the normal-B wave
 // (RIEMANN7F), whose normal-B flux is zero.
+//
+// Bound by the FP64 pipe, so everything else goes to the integer pipes
+// (mf_ieee64.cuh): divisions, roots, comparisons, signs and the factors 1/2
+// and 1/4.  Those factors and the signs are moved through the products they
+// stand in (exact: a power of two scales without rounding), which leaves one
+// product where the Fortran's coefficients repeat it with another factor:
+// e.g. so53 = -0.5 als as hyy sih / cc and sp35 = -als as hyy sih both come
+// from q1 = als as hyy.  The mirrored rows (fast and slow pairs) share their
+// partial sums: (-a) + (-b) = -(a + b) exactly.
 // ---------------------------------------------------------------------------
 template <typename R, int DIR, bool SEVEN>
 __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R* wr, R* g) {
+  static_assert(sizeof(R) == sizeof(double), "FP64 physics");
+  using namespace ieee64;
   constexpr int in = 1 + DIR, it1 = 1 + (DIR + 1) % 3, it2 = 1 + (DIR + 2) % 3;
   constexpr int inB = 5 + DIR, it1B = 5 + (DIR + 1) % 3, it2B = 5 + (DIR + 2) % 3;
-  const R gamma = R(P.gamma), hgamma = R(P.hgamma);
-  const R smallp = R(P.smallp), smallr = R(P.smallr);
-  const R i4pi = R(kInv4Pi), i8pi = R(kInv8Pi), sq2 = R(kSqrtHalf);
+  const double gamma = P.gamma, hgamma = P.hgamma;
+  const double smallp = P.smallp, smallr = P.smallr;
+  const double i4pi = kInv4Pi, i8pi = kInv8Pi, sq2 = kSqrtHalf;
 
-  R PGasL = rmax<R>(smallp, wl[4]), RhoL = rmax<R>(smallr, wl[0]);
-  R UL = wl[in], VL = wl[it1], WL = wl[it2];
-  R BXL = wl[inB], BYL = wl[it1B], BZL = wl[it2B];
-  R PGasR = rmax<R>(smallp, wr[4]), RhoR = rmax<R>(smallr, wr[0]);
-  R UR = wr[in], VR = wr[it1], WR = wr[it2];
-  R BXR = wr[inB], BYR = wr[it1B], BZR = wr[it2B];
+  const double PGasL = maxnum(smallp, wl[4]), RhoL = maxnum(smallr, wl[0]);
+  const double UL = wl[in], VL = wl[it1], WL = wl[it2];
+  const double BXL = wl[inB], BYL = wl[it1B], BZL = wl[it2B];
+  const double PGasR = maxnum(smallp, wr[4]), RhoR = maxnum(smallr, wr[0]);
+  const double UR = wr[in], VR = wr[it1], WR = wr[it2];
+  const double BXR = wr[inB], BYR = wr[it1B], BZR = wr[it2B];
 
-  R RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
-  R BxBL = i8pi * (BXL * BXL + BYL * BYL + BZL * BZL);
-  R RUxUL = R(0.5) * (RUL * UL + RVL * VL + RWL * WL);
-  R PL = PGasL + BxBL;
-  R EL = PGasL / hgamma + RUxUL + BxBL;
-  R AL2 = gamma * PGasL / RhoL;
+  const double RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
+  const double BxBL = i8pi * (BXL * BXL + BYL * BYL + BZL * BZL);
+  const double RUxUL = half(RUL * UL + RVL * VL + RWL * WL);
+  const double PL = PGasL + BxBL;
+  const double EL = div(PGasL, hgamma) + RUxUL + BxBL;
+  const double AL2 = div(gamma * PGasL, RhoL);
 
-  R RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
-  R BxBR = i8pi * (BXR * BXR + BYR * BYR + BZR * BZR);
-  R RUxUR = R(0.5) * (RUR * UR + RVR * VR + RWR * WR);
-  R PR = PGasR + BxBR;
-  R ER = PGasR / hgamma + RUxUR + BxBR;
-  R AR2 = gamma * PGasR / RhoR;
+  const double RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
+  const double BxBR = i8pi * (BXR * BXR + BYR * BYR + BZR * BZR);
+  const double RUxUR = half(RUR * UR + RVR * VR + RWR * WR);
+  const double PR = PGasR + BxBR;
+  const double ER = div(PGasR, hgamma) + RUxUR + BxBR;
+  const double AR2 = div(gamma * PGasR, RhoR);
 
-  R ccmi, ccma;
-  if (AL2 > AR2) { ccmi = AR2; ccma = AL2; } else { ccmi = AL2; ccma = AR2; }
+  const bool wide = lt(AR2, AL2);
+  const double ccmi = wide ? AR2 : AL2, ccma = wide ? AL2 : AR2;
 
-  R Rho, U, V, W, BX, BY, BZ, BX2, BYZ2, BxBH, kk, cc;
+  double Rho, U, V, W, BX, BY, BZ, BX2, BYZ2, BxBH, kk, cc;
   if (P.aver == 1) {
-    R HL = (EL + PL) / RhoL, HR = (ER + PR) / RhoR;
-    R coefRL = R(1) / (R(1) + sqrt_r<R>(RhoR / RhoL));
-    R coefRR = R(1) - coefRL;
+    const double HL = div(EL + PL, RhoL), HR = div(ER + PR, RhoR);
+    const double coefRL = div(1.0, 1.0 + root(div(RhoR, RhoL)));
+    const double coefRR = 1.0 - coefRL;
     Rho = RhoR * coefRL + RhoL * coefRR;
     U = UL * coefRL + UR * coefRR;
     V = VL * coefRL + VR * coefRR;
     W = WL * coefRL + WR * coefRR;
-    R HAV = HL * coefRL + HR * coefRR;
+    const double HAV = HL * coefRL + HR * coefRR;
     BX = BXR * coefRL + BXL * coefRR;
     BY = BYR * coefRL + BYL * coefRR;
     BZ = BZR * coefRL + BZL * coefRR;
-    R BXAV = R(0.5) * (BXL + BXR);
+    const double BXAV = half(BXL + BXR);
     BX2 = BXAV * BXAV;
-    R BY2 = BY * BY, BZ2 = BZ * BZ;
+    const double BY2 = BY * BY, BZ2 = BZ * BZ;
     BYZ2 = BY2 + BZ2;
     BxBH = i8pi * (BX2 + BYZ2);
-    kk = R(0.5) * (U * U + V * V + W * W);
-    R DBX = BXR - BXL, DBY = BYR - BYL, DBZ = BZR - BZL;
-    R X = i8pi * (DBX * DBX + DBY * DBY + DBZ * DBZ) * coefRL * coefRL / RhoL;
-    cc = hgamma * (HAV - kk - i4pi * (BX * BXAV + BYZ2) / Rho) + (R(2) - gamma) * X;
+    kk = half(U * U + V * V + W * W);
+    const double DBX = BXR - BXL, DBY = BYR - BYL, DBZ = BZR - BZL;
+    const double X = div(i8pi * (DBX * DBX + DBY * DBY + DBZ * DBZ) * coefRL * coefRL, RhoL);
+    cc = hgamma * (HAV - kk - div(i4pi * (BX * BXAV + BYZ2), Rho)) + (2.0 - gamma) * X;
   } else {
-    Rho = R(0.5) * (RhoL + RhoR);
-    U = R(0.5) * (UL + UR);
-    V = R(0.5) * (VL + VR);
-    W = R(0.5) * (WL + WR);
-    BX = R(0.5) * (BXL + BXR);
-    BY = R(0.5) * (BYL + BYR);
-    BZ = R(0.5) * (BZL + BZR);
-    R Pav = R(0.5) * (PL + PR);
+    Rho = half(RhoL + RhoR);
+    U = half(UL + UR);
+    V = half(VL + VR);
+    W = half(WL + WR);
+    BX = half(BXL + BXR);
+    BY = half(BYL + BYR);
+    BZ = half(BZL + BZR);
+    const double Pav = half(PL + PR);
     BX2 = BX * BX;
-    R BY2 = BY * BY, BZ2 = BZ * BZ;
+    const double BY2 = BY * BY, BZ2 = BZ * BZ;
     BYZ2 = BY2 + BZ2;
     BxBH = i8pi * (BX2 + BYZ2);
-    kk = R(0.5) * (U * U + V * V + W * W);
-    R PGas = Pav - BxBH;
-    cc = gamma * PGas / Rho;
+    kk = half(U * U + V * V + W * W);
+    const double PGas = Pav - BxBH;
+    cc = div(gamma * PGas, Rho);
   }
 
-  R bb = i4pi * BX2 / Rho;
-  R b = sqrt_r<R>(bb);
-  if (cc < ccmi) cc = ccmi;
-  if (cc > ccma) cc = ccma;
-  R c = sqrt_r<R>(cc);
+  const double bb = div(i4pi * BX2, Rho);
+  const double b = root(bb);
+  if (lt(cc, ccmi)) cc = ccmi;
+  if (lt(ccma, cc)) cc = ccma;
+  const double c = root(cc);
 
-  R hyy, hzz, aaf, aas, af, as;
-  const R smallB = R(P.smallB);
-  if (BYZ2 < smallB * smallB) {
+  double hyy, hzz, aaf, aas, af, as;
+  const double smallB = P.smallB;
+  if (lt(BYZ2, smallB * smallB)) {
     hyy = sq2;
     hzz = sq2;
-    if (bb > cc) { aaf = bb; aas = cc; af = b; as = c; }
-    else { aaf = cc; aas = bb; af = c; as = b; }
+    const bool alfven = lt(cc, bb);
+    aaf = alfven ? bb : cc;
+    aas = alfven ? cc : bb;
+    af = alfven ? b : c;
+    as = alfven ? c : b;
   } else {
-    R hyz = sqrt_r<R>(BYZ2);
-    hyy = BY / hyz;
-    hzz = BZ / hyz;
-    R szb = cc + (BxBH + BxBH) / Rho;
-    R h = sqrt_r<R>(szb * szb - R(4) * cc * bb);
-    aas = R(0.5) * (szb - h);
-    if (aas <= R(0)) { aas = R(0); as = R(0); }
-    else if (aas >= cc) { aas = cc; as = c; }
-    else { as = sqrt_r<R>(aas); }
-    aaf = R(0.5) * (szb + h);
-    if (aaf <= cc) { aaf = cc; af = c; }
-    else { af = sqrt_r<R>(aaf); }
+    const double hyz = root(BYZ2);
+    hyy = div(BY, hyz);
+    hzz = div(BZ, hyz);
+    const double szb = cc + div(scale<1>(BxBH), Rho);
+    const double h = root(szb * szb - scale<2>(cc) * bb);
+    aas = half(szb - h);
+    const bool gone = le(aas, 0.0), capped = le(cc, aas);
+    as = root(gone | capped ? 0.0 : aas);
+    if (capped) { aas = cc; as = c; }
+    if (gone) { aas = 0.0; as = 0.0; }
+    aaf = half(szb + h);
+    const bool low = le(aaf, cc);
+    af = root(low ? 0.0 : aaf);
+    if (low) { aaf = cc; af = c; }
   }
 
   // entropy-fixed speeds (Roe8 numbering: 1 entropy, 2 div-B, 3/4 Alfven,
   // 5/6 fast, 7/8 slow)
-  const R eigmax = rabs<R>(U) + rabs<R>(V) + rabs<R>(W) + af;
-  const R del = R(P.del2) * eigmax;
-  const R dell2 = del * del;
-  auto fix = [&](R e) -> R {
-    R z = rabs<R>(e);
-    return (z >= del) ? z : R(0.5) * (z * z + dell2) / del;
+  const double eigmax = absval(U) + absval(V) + absval(W) + af;
+  const double del = P.del2 * eigmax;
+  const double dell2 = del * del;
+  auto fix = [&](double e) -> double {
+    const double z = absval(e);
+    if (le(del, z)) return z;
+    return div(half(z * z + dell2), del);
   };
-  R A1 = fix(U);
-  R A2 = fix(U);
-  R A3 = fix(U + b), A4 = fix(U - b);
-  R A5 = fix(U + af), A6 = fix(U - af);
-  R A7 = fix(U + as), A8 = fix(U - as);
+  const double A1 = fix(U);
+  const double A2 = A1;
+  const double A3 = fix(U + b), A4 = fix(U - b);
+  const double A5 = fix(U + af), A6 = fix(U - af);
+  const double A7 = fix(U + as), A8 = fix(U - as);
 
-  R alf, als;
-  R dfs = aaf - aas;
-  if (dfs < R(1.0e-8)) { alf = R(1); als = R(0); }
-  else if ((cc - aas) <= R(0)) { alf = R(0); als = R(1); }
-  else if ((aaf - cc) <= R(0)) { alf = R(1); als = R(0); }
-  else { alf = sqrt_r<R>((cc - aas) / dfs); als = sqrt_r<R>((aaf - cc) / dfs); }
+  double alf, als;
+  const double dfs = aaf - aas;
+  const double dcs = cc - aas, dfc = aaf - cc;
+  if (lt(dfs, 1.0e-8)) { alf = 1.0; als = 0.0; }
+  else if (le(dcs, 0.0)) { alf = 0.0; als = 1.0; }
+  else if (le(dfc, 0.0)) { alf = 1.0; als = 0.0; }
+  else { alf = root(div(dcs, dfs)); als = root(div(dfc, dfs)); }
 
-  R sih = R(-1);
-  if (BX >= R(0)) sih = R(1);
+  // the sign bit of sih: clear where BX >= 0
+  const uint32_t sih = le(0.0, BX) ? 0u : 0x80000000u;
 
-  R fl1 = RUL;
-  R fl2 = UL * RUL - BXL * BXL * i4pi + PL;
-  R fl3 = UL * RVL - BXL * BYL * i4pi;
-  R fl4 = UL * RWL - BXL * BZL * i4pi;
-  R fl5 = UL * (EL + PL) - BXL * (UL * BXL + VL * BYL + WL * BZL) * i4pi;
-  R fl7 = UL * BYL - BXL * VL;
-  R fl8 = UL * BZL - BXL * WL;
-  R fr1 = RUR;
-  R fr2 = UR * RUR - BXR * BXR * i4pi + PR;
-  R fr3 = UR * RVR - BXR * BYR * i4pi;
-  R fr4 = UR * RWR - BXR * BZR * i4pi;
-  R fr5 = UR * (ER + PR) - BXR * (UR * BXR + VR * BYR + WR * BZR) * i4pi;
-  R fr7 = UR * BYR - BXR * VR;
-  R fr8 = UR * BZR - BXR * WR;
+  const double fl1 = RUL;
+  const double fl2 = UL * RUL - BXL * BXL * i4pi + PL;
+  const double fl3 = UL * RVL - BXL * BYL * i4pi;
+  const double fl4 = UL * RWL - BXL * BZL * i4pi;
+  const double fl5 = UL * (EL + PL) - BXL * (UL * BXL + VL * BYL + WL * BZL) * i4pi;
+  const double fl7 = UL * BYL - BXL * VL;
+  const double fl8 = UL * BZL - BXL * WL;
+  const double fr1 = RUR;
+  const double fr2 = UR * RUR - BXR * BXR * i4pi + PR;
+  const double fr3 = UR * RVR - BXR * BYR * i4pi;
+  const double fr4 = UR * RWR - BXR * BZR * i4pi;
+  const double fr5 = UR * (ER + PR) - BXR * (UR * BXR + VR * BYR + WR * BZR) * i4pi;
+  const double fr7 = UR * BYR - BXR * VR;
+  const double fr8 = UR * BZR - BXR * WR;
 
-  R du1 = RhoL - RhoR;
-  R du2 = RUL - RUR;
-  R du3 = RVL - RVR;
-  R du4 = RWL - RWR;
-  R du5 = EL - ER;
-  R du6 = BXL - BXR;
-  R du7 = BYL - BYR;
-  R du8 = BZL - BZR;
+  const double du1 = RhoL - RhoR;
+  double du2 = RUL - RUR;
+  double du3 = RVL - RVR;
+  double du4 = RWL - RWR;
+  double du5 = EL - ER;
+  const double du6 = BXL - BXR;
+  const double du7 = BYL - BYR;
+  const double du8 = BZL - BZR;
   if (SEVEN)
     du5 = -hgamma * (-kk * du1 + U * du2 + V * du3 + W * du4 - du5 + (BY * du7 + BZ * du8) * i4pi);
   else
     du5 = -hgamma *
           (-kk * du1 + U * du2 + V * du3 + W * du4 - du5 + (BX * du6 + BY * du7 + BZ * du8) * i4pi);
-  du2 = (-U * du1 + du2) / Rho;
-  du3 = (-V * du1 + du3) / Rho;
-  du4 = (-W * du1 + du4) / Rho;
+  du2 = div(-U * du1 + du2, Rho);
+  du3 = div(-V * du1 + du3, Rho);
+  du4 = div(-W * du1 + du4, Rho);
 
-  const R sqPiRho = sqrt_r<R>(R(kPi) * Rho);
-  const R sq2PiRho = sqrt_r<R>(R(k2Pi) * Rho);
+  const double sqPiRho = root(kPi * Rho);
+  const double sq2PiRho = root(k2Pi * Rho);
 
-  // left eigenvectors (non-zero entries only)
-  R so15 = -R(1) / cc;
-  R so33 = -hzz * sq2, so34 = hyy * sq2;
-  R so37 = R(0.5) * hzz * sih / sq2PiRho, so38 = -R(0.5) * hyy * sih / sq2PiRho;
-  // (-a)/b == -(a/b) exactly: the mirrored coefficients are negations
-  R so47 = -so37, so48 = -so38;
-  R so52 = R(0.5) * alf * af / cc;
-  R so53 = -R(0.5) * als * as * hyy * sih / cc;
-  R so54 = -R(0.5) * als * as * hzz * sih / cc;
-  R so55 = R(0.5) * alf / (cc * Rho);
-  R so57 = R(0.25) * als * hyy / (c * sqPiRho);
-  R so58 = R(0.25) * als * hzz / (c * sqPiRho);
-  R so62 = -so52;
-  R so63 = -so53;
-  R so64 = -so54;
-  R so72 = R(0.5) * als * as / cc;
-  R so73 = R(0.5) * alf * af * hyy * sih / cc;
-  R so74 = R(0.5) * alf * af * hzz * sih / cc;
-  R so75 = R(0.5) * als / (Rho * cc);
-  R so77 = -R(0.25) * alf * hyy / (c * sqPiRho);
-  R so78 = -R(0.25) * alf * hzz / (c * sqPiRho);
-  R so82 = -so72;
-  R so83 = -so73;
-  R so84 = -so74;
+  // products that the eigenvectors share
+  const double p1 = alf * af, p2 = als * as;
+  const double q1 = p2 * hyy, q2 = p2 * hzz, q3 = p1 * hyy, q4 = p1 * hzz;
+  const double ccr = cc * Rho, csq = c * sqPiRho;
+  const double h7 = half(du7), h8 = half(du8);
 
-  R lu1 = A1 * (du1 + so15 * du5);
-  R lu2 = A2 * du6;
-  R lu3 = A3 * (so33 * du3 + so34 * du4 + so37 * du7 + so38 * du8);
-  R lu4 = A4 * (so33 * du3 + so34 * du4 + so47 * du7 + so48 * du8);
-  R lu5 = A5 * (so52 * du2 + so53 * du3 + so54 * du4 + so55 * du5 + so57 * du7 + so58 * du8);
-  R lu6 = A6 * (so62 * du2 + so63 * du3 + so64 * du4 + so55 * du5 + so57 * du7 + so58 * du8);
-  R lu7 = A7 * (so72 * du2 + so73 * du3 + so74 * du4 + so75 * du5 + so77 * du7 + so78 * du8);
-  R lu8 = A8 * (so82 * du2 + so83 * du3 + so84 * du4 + so75 * du5 + so77 * du7 + so78 * du8);
+  const double lu1 = A1 * (du1 + flip(div(1.0, cc), 0x80000000u) * du5);
+  const double lu2 = A2 * du6;
+  const double s33 = hzz * sq2, s34 = hyy * sq2;
+  const double e34 = s34 * du4 - s33 * du3;
+  const double e37 = flip(div(hzz, sq2PiRho) * h7, sih), e38 = flip(div(hyy, sq2PiRho) * h8, sih);
+  const double lu3 = A3 * (e34 + e37 - e38);
+  const double lu4 = A4 * (e34 - e37 + e38);
+  // twice the amplitudes of the fast and slow waves' common parts
+  const double f234 = div(p1, cc) * du2 - flip(div(q1, cc), sih) * du3 - flip(div(q2, cc), sih) * du4;
+  const double f5 = div(alf, ccr) * du5;
+  const double f7 = div(als * hyy, csq) * h7, f8 = div(als * hzz, csq) * h8;
+  const double lu5 = half(A5 * (f234 + f5 + f7 + f8));
+  const double lu6 = half(A6 * (f5 - f234 + f7 + f8));
+  const double g234 = div(p2, cc) * du2 + flip(div(q3, cc), sih) * du3 + flip(div(q4, cc), sih) * du4;
+  const double g5 = div(als, ccr) * du5;
+  const double g7 = div(alf * hyy, csq) * h7, g8 = div(alf * hzz, csq) * h8;
+  const double lu7 = half(A7 * (g234 + g5 - g7 - g8));
+  const double lu8 = half(A8 * (g5 - g234 - g7 - g8));
 
   // right eigenvectors (non-zero entries only)
-  R sp15 = Rho * alf, sp17 = Rho * als;
-  R sp25 = alf * af, sp26 = -alf * af, sp27 = als * as, sp28 = -als * as;
-  R sp33 = -hzz * sq2;
-  R sp35 = -als * as * hyy * sih, sp36 = als * as * hyy * sih;
-  R sp37 = alf * af * hyy * sih, sp38 = -alf * af * hyy * sih;
-  R sp43 = hyy * sq2;
-  R sp45 = -als * as * hzz * sih, sp46 = als * as * hzz * sih;
-  R sp47 = alf * af * hzz * sih, sp48 = -alf * af * hzz * sih;
-  R sp55 = alf * Rho * cc, sp57 = als * Rho * cc;
-  R sp73 = hzz * sq2PiRho * sih, sp74 = -hzz * sq2PiRho * sih;
-  R sp75 = R(2) * als * sqPiRho * c * hyy;
-  R sp77 = -R(2) * alf * sqPiRho * c * hyy;
-  R sp83 = -hyy * sq2PiRho * sih, sp84 = hyy * sq2PiRho * sih;
-  R sp85 = R(2) * als * sqPiRho * c * hzz;
-  R sp87 = -R(2) * alf * sqPiRho * c * hzz;
-
-  R ra1 = lu1 + sp15 * lu5 + sp15 * lu6 + sp17 * lu7 + sp17 * lu8;
-  R ra2 = sp25 * lu5 + sp26 * lu6 + sp27 * lu7 + sp28 * lu8;
-  R ra3 = sp33 * lu3 + sp33 * lu4 + sp35 * lu5 + sp36 * lu6 + sp37 * lu7 + sp38 * lu8;
-  R ra4 = sp43 * lu3 + sp43 * lu4 + sp45 * lu5 + sp46 * lu6 + sp47 * lu7 + sp48 * lu8;
-  R ra5 = sp55 * lu5 + sp55 * lu6 + sp57 * lu7 + sp57 * lu8;
-  R ra6 = lu2;
-  R ra7 = sp73 * lu3 + sp74 * lu4 + sp75 * lu5 + sp75 * lu6 + sp77 * lu7 + sp77 * lu8;
-  R ra8 = sp83 * lu3 + sp84 * lu4 + sp85 * lu5 + sp85 * lu6 + sp87 * lu7 + sp87 * lu8;
+  const double sp15 = Rho * alf, sp17 = Rho * als;
+  double ra1 = lu1 + sp15 * lu5 + sp15 * lu6 + sp17 * lu7 + sp17 * lu8;
+  double ra2 = p1 * lu5 - p1 * lu6 + p2 * lu7 - p2 * lu8;
+  double ra3 = -(s33 * lu3) - s33 * lu4 - flip(q1 * lu5, sih) + flip(q1 * lu6, sih) +
+               flip(q3 * lu7, sih) - flip(q3 * lu8, sih);
+  double ra4 = s34 * lu3 + s34 * lu4 - flip(q2 * lu5, sih) + flip(q2 * lu6, sih) +
+               flip(q4 * lu7, sih) - flip(q4 * lu8, sih);
+  const double sp55 = sp15 * cc, sp57 = sp17 * cc;
+  double ra5 = sp55 * lu5 + sp55 * lu6 + sp57 * lu7 + sp57 * lu8;
+  const double ra6 = lu2;
+  const double sp73 = flip(hzz * sq2PiRho, sih), sp84 = flip(hyy * sq2PiRho, sih);
+  const double t5 = scale<1>(als * sqPiRho * c), t7 = scale<1>(alf * sqPiRho * c);
+  const double sp75 = t5 * hyy, sp77 = t7 * hyy, sp85 = t5 * hzz, sp87 = t7 * hzz;
+  const double ra7 = sp73 * lu3 - sp73 * lu4 + sp75 * lu5 + sp75 * lu6 - sp77 * lu7 - sp77 * lu8;
+  const double ra8 = sp84 * lu4 - sp84 * lu3 + sp85 * lu5 + sp85 * lu6 - sp87 * lu7 - sp87 * lu8;
 
   if (SEVEN)
-    ra5 = ra1 * kk + Rho * (U * ra2 + V * ra3 + W * ra4) + ra5 / hgamma + i4pi * (BY * ra7 + BZ * ra8);
+    ra5 = ra1 * kk + Rho * (U * ra2 + V * ra3 + W * ra4) + div(ra5, hgamma) +
+          i4pi * (BY * ra7 + BZ * ra8);
   else
-    ra5 = ra1 * kk + Rho * (U * ra2 + V * ra3 + W * ra4) + ra5 / hgamma +
+    ra5 = ra1 * kk + Rho * (U * ra2 + V * ra3 + W * ra4) + div(ra5, hgamma) +
           i4pi * (BX * ra6 + BY * ra7 + BZ * ra8);
   ra2 = U * ra1 + Rho * ra2;
   ra3 = V * ra1 + Rho * ra3;
   ra4 = W * ra1 + Rho * ra4;
 
-  g[0] = R(0.5) * (fl1 + fr1 + ra1);
-  g[in] = R(0.5) * (fl2 + fr2 + ra2);
-  g[it1] = R(0.5) * (fl3 + fr3 + ra3);
-  g[it2] = R(0.5) * (fl4 + fr4 + ra4);
-  g[4] = R(0.5) * (fl5 + fr5 + ra5);
-  g[inB] = SEVEN ? R(0) : R(0.5) * (R(0) + R(0) + ra6);
-  g[it1B] = R(0.5) * (fl7 + fr7 + ra7);
-  g[it2B] = R(0.5) * (fl8 + fr8 + ra8);
+  g[0] = half(fl1 + fr1 + ra1);
+  g[in] = half(fl2 + fr2 + ra2);
+  g[it1] = half(fl3 + fr3 + ra3);
+  g[it2] = half(fl4 + fr4 + ra4);
+  g[4] = half(fl5 + fr5 + ra5);
+  g[inB] = SEVEN ? 0.0 : half(ra6);
+  g[it1B] = half(fl7 + fr7 + ra7);
+  g[it2B] = half(fl8 + fr8 + ra8);
 }
 
 // RUSANOVF (src/RusanovF.ChF:4-197)
@@ -331,66 +332,69 @@ __device__ __forceinline__ void rusanov_mhd(const DevParams& P, const R* wl, con
 // DEDNER2X2F (src/DednerF.ChF:89-170): returns the Bn and psi fluxes.
 template <typename R>
 __device__ __forceinline__ void dedner_2x2(R ch, R bxl, R psil, R bxr, R psir, R& fbn, R& fpsi) {
-  R ch2 = ch * ch;
-  R so12 = -R(0.5) / ch, so22 = R(0.5) / ch;
-  R du1 = bxl - bxr, du2 = psil - psir;
-  R lu1 = ch * (R(0.5) * du1 + so12 * du2);
-  R lu2 = ch * (R(0.5) * du1 + so22 * du2);
-  R ra1 = lu1 + lu2;
-  R ra2 = -ch * lu1 + ch * lu2;
-  fbn = R(0.5) * (psil + psir + ra1);
-  fpsi = R(0.5) * (ch2 * bxl + ch2 * bxr + ra2);
+  using namespace ieee64;
+  const R ch2 = ch * ch;
+  const R hc = div(0.5, ch);
+  const R du1 = half(bxl - bxr), du2 = psil - psir;
+  const R lu1 = ch * (du1 - hc * du2);
+  const R lu2 = ch * (du1 + hc * du2);
+  const R ra1 = lu1 + lu2;
+  const R ra2 = ch * lu2 - ch * lu1;
+  fbn = half(psil + psir + ra1);
+  fpsi = half(ch2 * bxl + ch2 * bxr + ra2);
 }
 
 // VANLEERF (src/VanLeerRSF.ChF:4-130): wl/wr = rho,u,v,w,p of one Euler fluid.
+// Divisions, roots, comparisons and powers of two as in roe_mhd.
 template <typename R, int DIR>
 __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, const R* wr, R* g) {
+  using namespace ieee64;
   constexpr int in = 1 + DIR, it1 = 1 + (DIR + 1) % 3, it2 = 1 + (DIR + 2) % 3;
   const R gamma = R(P.gamma), hgamma = R(P.hgamma);
   R fl1, fl2, fl3, fl4, fl5, fr1, fr2, fr3, fr4, fr5;
-  R PGasL = rmax<R>(R(P.smallp), wl[4]), RhoL = rmax<R>(R(P.smallr), wl[0]);
-  R UL = wl[in], VL = wl[it1], WL = wl[it2];
-  R RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
-  R RUxUL = R(0.5) * (RUL * UL + RVL * VL + RWL * WL);
-  R EL = PGasL / hgamma + RUxUL;
-  R AL = sqrt_r<R>(gamma * PGasL / RhoL);
-  if (UL <= -AL) {
+  const R PGasL = maxnum(P.smallp, wl[4]), RhoL = maxnum(P.smallr, wl[0]);
+  const R UL = wl[in], VL = wl[it1], WL = wl[it2];
+  const R RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
+  const R RUxUL = half(RUL * UL + RVL * VL + RWL * WL);
+  const R EL = div(PGasL, hgamma) + RUxUL;
+  const R AL = root(div(gamma * PGasL, RhoL));
+  if (le(UL, -AL)) {
     fr1 = fr2 = fr3 = fr4 = fr5 = R(0);
-  } else if (UL >= AL) {
+  } else if (le(AL, UL)) {
     fr1 = RhoL * UL;
     fr2 = fr1 * UL + PGasL;
     fr3 = fr1 * VL;
     fr4 = fr1 * WL;
     fr5 = UL * (EL + PGasL);
   } else {
-    R UA = (-UL + (AL + AL)) / gamma;
-    R H = (EL + PGasL) / RhoL;
-    R HU = UL + AL;
-    fr1 = R(0.25) * RhoL * HU * HU / AL;
+    const R UA = div(scale<1>(AL) - UL, gamma);
+    const R H = div(EL + PGasL, RhoL);
+    const R HU = UL + AL;
+    fr1 = scale<-2>(div(RhoL * HU * HU, AL));
     fr2 = fr1 * (UL + UA);
     fr3 = fr1 * VL;
     fr4 = fr1 * WL;
     fr5 = fr1 * H;
   }
-  R PGasR = rmax<R>(R(P.smallp), wr[4]), RhoR = rmax<R>(R(P.smallr), wr[0]);
-  R UR = wr[in], VR = wr[it1], WR = wr[it2];
-  R RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
-  R RUxUR = R(0.5) * (RUR * UR + RVR * VR + RWR * WR);
-  R ER = PGasR / hgamma + RUxUR;
-  R AR = sqrt_r<R>(gamma * PGasR / RhoR);
-  if (UR >= AR) {
+  const R PGasR = maxnum(P.smallp, wr[4]), RhoR = maxnum(P.smallr, wr[0]);
+  const R UR = wr[in], VR = wr[it1], WR = wr[it2];
+  const R RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
+  const R RUxUR = half(RUR * UR + RVR * VR + RWR * WR);
+  const R ER = div(PGasR, hgamma) + RUxUR;
+  const R AR = root(div(gamma * PGasR, RhoR));
+  if (le(AR, UR)) {
     fl1 = fl2 = fl3 = fl4 = fl5 = R(0);
-  } else if (UR <= -AR) {
+  } else if (le(UR, -AR)) {
     fl1 = RhoR * UR;
     fl2 = fl1 * UR + PGasR;
     fl3 = fl1 * VR;
     fl4 = fl1 * WR;
     fl5 = UR * (ER + PGasR);
   } else {
-    R UA = (-UR - (AR + AR)) / gamma;
-    R H = (ER + PGasR) / RhoR;
-    R HU = UR - AR;
-    fl1 = -R(0.25) * RhoR * HU * HU / AR;
+    const R UA = div(-UR - scale<1>(AR), gamma);
+    const R H = div(ER + PGasR, RhoR);
+    const R HU = UR - AR;
+    fl1 = -scale<-2>(div(RhoR * HU * HU, AR));
     fl2 = fl1 * (UR + UA);
     fl3 = fl1 * VR;
     fl4 = fl1 * WR;

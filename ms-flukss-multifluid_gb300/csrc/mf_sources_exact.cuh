@@ -61,27 +61,28 @@ __device__ __forceinline__ int region_tracer_cell(const DevParams& P, double dx,
 __device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i, int j, int k,
                                            const double* w, double regtr) {
   if (P.reg_tracer) return region_tracer_cell(P, dx, i, j, k, w, regtr);
+  using namespace ieee64;
   double x = (i + 0.5) * dx - P.sun_c[0];
   double y = (j + 0.5) * dx - P.sun_c[1];
   double z = 0.0, r2, invr, ur;
   if (P.sd == 3) {
     z = (k + 0.5) * dx - P.sun_c[2];
     r2 = x * x + y * y + z * z;
-    invr = 1.0 / sqrt(r2);
+    invr = div(1.0, root(r2));
     ur = w[1] * (x * invr) + w[2] * (y * invr) + w[3] * (z * invr);
   } else {
     r2 = x * x + y * y;
-    invr = 1.0 / sqrt(r2);
+    invr = div(1.0, root(r2));
     ur = w[1] * (x * invr) + w[2] * (y * invr);
   }
-  double TEMP = P.t_coeff * w[4] / w[0];
+  double TEMP = div(P.t_coeff * w[4], w[0]);
   int reg;
-  bool zout = (P.sd == 3) && ((z < P.zbot) || (z > P.ztop));
-  if (fabs(ur) >= 0.6 * P.sun_v) {
-    reg = ((TEMP >= 1.0e6) && (r2 > P.sun_r * P.sun_r)) ? 2 : 3;
+  bool zout = (P.sd == 3) && (lt(z, P.zbot) || lt(P.ztop, z));
+  if (le(0.6 * P.sun_v, absval(ur))) {
+    reg = (le(1.0e6, TEMP) && lt(P.sun_r * P.sun_r, r2)) ? 2 : 3;
     if (zout) reg = 1;
   } else {
-    if (TEMP >= P.tmlim) {
+    if (le(P.tmlim, TEMP)) {
       reg = 2;
       if (zout) reg = 1;
     } else {
@@ -111,10 +112,15 @@ template <int IRHON, typename T = double, typename WA = const double*, int NN = 
 __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA& w, int reg,
                                                     double dt, double* u) {
   static_assert(sizeof(T) == sizeof(double), "FP64 physics");
+  using namespace ieee64;
   const int nN = NN > 0 ? NN : P.nf - 1;
-  double rho = w[0], ux = w[1], uy = w[2], uz = w[3], pp = w[4];
-  double U2 = ux * ux + uy * uy + uz * uz;
-  double VVTP = pp / rho;
+  const double rho = w[0], ux = w[1], uy = w[2], uz = w[3], pp = w[4];
+  const double U2 = ux * ux + uy * uy + uz * uz;
+  const double VVTP = div(pp, rho);
+  // plasma terms of the speeds, the same for every population; factors that
+  // are powers of two scale exactly
+  const double tp4 = scale<2>(VVTP), hU2 = half(U2);
+  const double tp16 = div(scale<4>(VVTP), kPi), tpc = 2.25 * kPi * VVTP, tp649 = div(scale<6>(VVTP), 9.0);
   double h2 = 0, h3 = 0, h4 = 0, h5 = 0, PPLUX = 0, PPLUY = 0, PPLUZ = 0, ENPLU = 0;
   double DENPLU[MF_MAX_FLUIDS], PMIX[MF_MAX_FLUIDS], PMIY[MF_MAX_FLUIDS], PMIZ[MF_MAX_FLUIDS],
       ENMI[MF_MAX_FLUIDS];
@@ -122,39 +128,42 @@ __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA
   for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
     if (f > nN) break;
     const double* wn = w + IRHON + (f - 1) * 5;
-    double rhoN = wn[0], uxN = wn[1], uyN = wn[2], uzN = wn[3], pN = wn[4];
-    double UH2 = uxN * uxN + uyN * uyN + uzN * uzN;
-    double DU2 = (ux - uxN) * (ux - uxN) + (uy - uyN) * (uy - uyN) + (uz - uzN) * (uz - uzN);
-    double VPHH = (ux - uxN) * uxN + (uy - uyN) * uyN + (uz - uzN) * uzN;
-    double VPHP = (ux - uxN) * ux + (uy - uyN) * uy + (uz - uzN) * uz;
-    double VVTH = 2.0 * pN / rhoN;
-    double UD = sqrt(4.0 * (VVTP + VVTH) / kPi + DU2);
-    double UPM = sqrt(16.0 * VVTP / kPi + 2.25 * kPi * VVTH + 4.0 * DU2);
-    double UHM = sqrt(2.25 * kPi * VVTP + 16.0 * VVTH / kPi + 4.0 * DU2);
-    double UPE = sqrt((4.0 * VVTP + 64.0 * VVTH / 9.0) / kPi + DU2);
-    double UHE = sqrt((64.0 * VVTP / 9.0 + 4.0 * VVTH) / kPi + DU2);
-    double UDS = P.ce_scale_vel * UD;
-    double t = P.ce_a - P.ce_b * log(UDS);
+    const double rhoN = wn[0], uxN = wn[1], uyN = wn[2], uzN = wn[3], pN = wn[4];
+    const double dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
+    const double UH2 = uxN * uxN + uyN * uyN + uzN * uzN;
+    const double DU2 = dx_ * dx_ + dy_ * dy_ + dz_ * dz_, DU24 = scale<2>(DU2);
+    const double VPHH = dx_ * uxN + dy_ * uyN + dz_ * uzN;
+    const double VPHP = dx_ * ux + dy_ * uy + dz_ * uz;
+    const double VVTH = div(scale<1>(pN), rhoN);
+    const double th4 = scale<2>(VVTH);
+    const double UD = root(div(scale<2>(VVTP + VVTH), kPi) + DU2);
+    const double UPM = root(tp16 + 2.25 * kPi * VVTH + DU24);
+    const double UHM = root(tpc + div(scale<4>(VVTH), kPi) + DU24);
+    const double UPE = root(div(tp4 + div(scale<6>(VVTH), 9.0), kPi) + DU2);
+    const double UHE = root(div(tp649 + th4, kPi) + DU2);
+    const double UDS = P.ce_scale_vel * UD;
+    const double t = P.ce_a - P.ce_b * log(UDS);
     double SIG = t * t;
     if (P.ce_damp_c > 0.0) SIG = SIG * pow(1.0 - exp(-P.ce_damp_c / UDS), P.ce_damp_pow);
     SIG = P.ce_sigma_scale * SIG;
-    double ARR = SIG * rhoN * rho;
-    double VVTHU = VVTH / UPM;
-    h2 = h2 + ARR * (ux - uxN) * (UD + VVTHU + VVTP / UHM);
-    h3 = h3 + ARR * (uy - uyN) * (UD + VVTHU + VVTP / UHM);
-    h4 = h4 + ARR * (uz - uzN) * (UD + VVTHU + VVTP / UHM);
-    h5 = h5 + 0.5 * ARR *
-                  (1.5 * (UHE * VVTP - UPE * VVTH) + UD * (U2 - UH2) +
-                   2.0 * (VVTHU * VPHH + VVTP * VPHP / UHM));
+    const double ARR = SIG * rhoN * rho;
+    const double VVTHU = div(VVTH, UPM);
+    const double hs = UD + VVTHU + div(VVTP, UHM);
+    h2 = h2 + ARR * dx_ * hs;
+    h3 = h3 + ARR * dy_ * hs;
+    h4 = h4 + ARR * dz_ * hs;
+    h5 = h5 + half(ARR) * (1.5 * (UHE * VVTP - UPE * VVTH) + UD * (U2 - UH2) +
+                           scale<1>(VVTHU * VPHH + div(VVTP * VPHP, UHM)));
     DENPLU[f] = -ARR * UD;
-    PPLUX = PPLUX - ARR * (ux * UD - (uxN - ux) * VVTP / UHM);
-    PPLUY = PPLUY - ARR * (uy * UD - (uyN - uy) * VVTP / UHM);
-    PPLUZ = PPLUZ - ARR * (uz * UD - (uzN - uz) * VVTP / UHM);
-    ENPLU = ENPLU - ARR * (0.5 * U2 * UD + VVTP * (VPHP / UHM + 0.75 * UHE));
-    PMIX[f] = ARR * (uxN * UD + (uxN - ux) * VVTHU);
-    PMIY[f] = ARR * (uyN * UD + (uyN - uy) * VVTHU);
-    PMIZ[f] = ARR * (uzN * UD + (uzN - uz) * VVTHU);
-    ENMI[f] = ARR * (0.5 * UH2 * UD - VPHH * VVTHU + 0.75 * VVTH * UPE);
+    // -(uxN - ux) == ux - uxN exactly
+    PPLUX = PPLUX - ARR * (ux * UD + div(dx_ * VVTP, UHM));
+    PPLUY = PPLUY - ARR * (uy * UD + div(dy_ * VVTP, UHM));
+    PPLUZ = PPLUZ - ARR * (uz * UD + div(dz_ * VVTP, UHM));
+    ENPLU = ENPLU - ARR * (hU2 * UD + VVTP * (div(VPHP, UHM) + 0.75 * UHE));
+    PMIX[f] = ARR * (uxN * UD - dx_ * VVTHU);
+    PMIY[f] = ARR * (uyN * UD - dy_ * VVTHU);
+    PMIZ[f] = ARR * (uzN * UD - dz_ * VVTHU);
+    ENMI[f] = ARR * (half(UH2) * UD - VPHH * VVTHU + 0.75 * VVTH * UPE);
   }
   u[1] = u[1] + (-dt * h2);
   u[2] = u[2] + (-dt * h3);
@@ -287,17 +296,18 @@ __device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double 
 // (srcIdeal/PatchMHDMFF.ChF:301-511).
 template <int IRHON>
 __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
+  using namespace ieee64;
   const double hg = P.hgamma, smallR = P.smallr, smallP = P.smallp;
   if (P.nf == 1) {
     double Rho = u[0];
     bool was = false;
-    if (Rho < smallR) { Rho = smallR; was = true; }
-    double invRho = 1.0 / Rho;
+    if (lt(Rho, smallR)) { Rho = smallR; was = true; }
+    double invRho = div(1.0, Rho);
     double Ux = u[1] * invRho, Uy = u[2] * invRho, Uz = u[3] * invRho;
     double BxB = kInv8Pi * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]);
-    double UxU = 0.5 * (Ux * Ux + Uy * Uy + Uz * Uz);
+    double UxU = half(Ux * Ux + Uy * Uy + Uz * Uz);
     double Pr = hg * (u[4] - BxB - Rho * UxU);
-    if (Pr < smallP) { Pr = smallP; was = true; }
+    if (lt(Pr, smallP)) { Pr = smallP; was = true; }
     if (was) {
       u[0] = Rho;
       u[4] = Pr / hg + Rho * UxU + BxB;
@@ -306,14 +316,14 @@ __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
   }
   {
     double Rho = u[0];
-    double invRho = 1.0 / Rho;
+    double invRho = div(1.0, Rho);
     double Ux = u[1] * invRho, Uy = u[2] * invRho, Uz = u[3] * invRho;
     double BxB = kInv8Pi * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]);
-    double UxU = 0.5 * (Ux * Ux + Uy * Uy + Uz * Uz);
+    double UxU = half(Ux * Ux + Uy * Uy + Uz * Uz);
     double Pr = hg * (u[4] - BxB - Rho * UxU);
     bool was = false;
-    if (Rho < smallR) { Rho = smallR; was = true; }
-    if (Pr < smallP) { Pr = smallP; was = true; }
+    if (lt(Rho, smallR)) { Rho = smallR; was = true; }
+    if (lt(Pr, smallP)) { Pr = smallP; was = true; }
     if (was) {
       u[0] = Rho;
       u[1] = Rho * Ux;
@@ -329,13 +339,13 @@ __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
     double fp = (f == 1) ? smallP : (f == 3) ? kNet3Pres : kNet2Pres;
     double* un = u + IRHON + (f - 1) * 5;
     double Rho = un[0];
-    double invRho = 1.0 / Rho;
+    double invRho = div(1.0, Rho);
     double Ux = un[1] * invRho, Uy = un[2] * invRho, Uz = un[3] * invRho;
-    double UxU = 0.5 * (Ux * Ux + Uy * Uy + Uz * Uz);
+    double UxU = half(Ux * Ux + Uy * Uy + Uz * Uz);
     double Pr = hg * (un[4] - Rho * UxU);
     bool was = false;
-    if (Rho < fd) { Rho = fd; was = true; }
-    if (Pr < fp) { Pr = fp; was = true; }
+    if (lt(Rho, fd)) { Rho = fd; was = true; }
+    if (lt(Pr, fp)) { Pr = fp; was = true; }
     if (was) {
       un[0] = Rho;
       un[1] = Rho * Ux;
@@ -351,42 +361,43 @@ __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
 template <int IRHON, typename T = double>
 __device__ __forceinline__ double max_wave_speed(const DevParams& P, const double* u) {
   static_assert(sizeof(T) == sizeof(double), "FP64 physics");
+  using namespace ieee64;
   double cmax = 0.0;
   {
     double rho = u[0];
-    double invrho = 1.0 / rho;
+    double invrho = div(1.0, rho);
     double ru = u[1], rv = u[2], rw = u[3];
     double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
     double ke = ru * uu + rv * vv + rw * ww;
     double bx = u[5], by = u[6], bz = u[7];
     double b = kInv4Pi * (bx * bx + by * by + bz * bz);
-    double p = P.hgamma * (u[4] - 0.5 * (ke + b));
-    p = fmax(p, P.smallp);
+    double p = P.hgamma * (u[4] - half(ke + b));
+    p = maxnum(p, P.smallp);
     double a2 = P.gamma * p * invrho;
-    double as2 = 0.5 * (a2 + invrho * b);
+    double as2 = half(a2 + invrho * b);
     double as4 = as2 * as2;
     double bn2 = kInv4Pi * bx * bx * invrho;
-    double umax = fabs(uu) + sqrt(as2 + sqrt(as4 - a2 * bn2));
+    double umax = absval(uu) + root(as2 + root(as4 - a2 * bn2));
     bn2 = kInv4Pi * by * by * invrho;
-    umax = fmax(fabs(vv) + sqrt(as2 + sqrt(as4 - a2 * bn2)), umax);
+    umax = maxnum(absval(vv) + root(as2 + root(as4 - a2 * bn2)), umax);
     bn2 = kInv4Pi * bz * bz * invrho;
-    umax = fmax(fabs(ww) + sqrt(as2 + sqrt(as4 - a2 * bn2)), umax);
-    cmax = fmax(umax, cmax);
+    umax = maxnum(absval(ww) + root(as2 + root(as4 - a2 * bn2)), umax);
+    cmax = maxnum(umax, cmax);
   }
 #pragma unroll
   for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
     if (f >= P.nf) break;
     const double* un = u + IRHON + (f - 1) * 5;
-    double rho = fmax(un[0], P.smallr);
-    double invrho = 1.0 / rho;
+    double rho = maxnum(un[0], P.smallr);
+    double invrho = div(1.0, rho);
     double ru = un[1], rv = un[2], rw = un[3];
     double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
     double ke = ru * uu + rv * vv + rw * ww;
-    double p = P.hgamma * (un[4] - 0.5 * ke);
-    p = fmax(p, P.smallp);
-    double a = sqrt(P.gamma * p * invrho);
-    double umax = fmax(fmax(fabs(uu), fabs(vv)), fabs(ww)) + a;
-    cmax = fmax(umax, cmax);
+    double p = P.hgamma * (un[4] - half(ke));
+    p = maxnum(p, P.smallp);
+    double a = root(P.gamma * p * invrho);
+    double umax = maxnum(maxnum(absval(uu), absval(vv)), absval(ww)) + a;
+    cmax = maxnum(umax, cmax);
   }
   return cmax;
 }

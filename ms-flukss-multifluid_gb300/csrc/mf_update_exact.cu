@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kMaxBlock)
 #pragma unroll
     for (int q = 0; q < MF_MAX_COMP; ++q)
       if (q < P.nc) u[q] = U[base + q * cs];
-    dtc = runs[D.run].dx / max_wave_speed<IRHON>(P, u);
+    dtc = ieee64::div(runs[D.run].dx, max_wave_speed<IRHON>(P, u));
     myidx = g;
   }
   block_dt_min(dtc, myidx, descs, ndesc, partials, blockIdx.x);

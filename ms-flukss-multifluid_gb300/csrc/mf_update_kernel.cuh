@@ -173,7 +173,7 @@ __device__ __forceinline__ void update_tail(const DevParams& P, const StageBuffe
   const auto& w = w_arg(ws);
   if (P.use8) {
     // SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES
-    const double dtbydx = dt / RP.dx;
+    const double dtbydx = ieee64::div(dt, RP.dx);
     const double dB = -divB * dtbydx;
     const double Ux = w[1], Uy = w[2], Uz = w[3];
     const double Bx = kInv4Pi * w[5], By = kInv4Pi * w[6], Bz = kInv4Pi * w[7];
@@ -215,7 +215,8 @@ __device__ __forceinline__ void update_tail(const DevParams& P, const StageBuffe
   if (FLAGS & kStageAverage) {  // AVERAGESTATE (src/PatchMHDAMF.ChF:289-316), every state
 #pragma unroll
     for (int q = 0; q < MF_MAX_COMP; ++q)
-      if (q < P.nc) u[q] = u[q] + 0.5 * (B.uold[base + q * cs] - B.uin[base + q * cs]);
+      if (q < P.nc)  // half the difference is exact: the fused form rounds once, like the sum
+        u[q] = fma(0.5, B.uold[base + q * cs] - B.uin[base + q * cs], u[q]);
   }
   bool finite = true;
 #pragma unroll
@@ -227,7 +228,7 @@ __device__ __forceinline__ void update_tail(const DevParams& P, const StageBuffe
     }
   if (!finite) atomicOr(&ss->flags, kFlagNonFinite);
   if (FLAGS & kStageDt) {
-    dtc = RP.dx / max_wave_speed<IRHON, R>(P, u);
+    dtc = ieee64::div(RP.dx, max_wave_speed<IRHON, R>(P, u));
     myidx = g;
     if (B.divb && P.use8) B.divb[loc(B.divb_lo, B.divb_n, i, j, k)] = divB;
   }
