@@ -407,6 +407,9 @@ static void count_launches(mf_level* L) {
   L->fused_saving = L->fused ? per * sd : 0;
   L->launches = L->base_launches + per * (int)L->gathers.size() - (fused ? per * sd : 0) +
                 (overlap ? per * (L->nchunks - sd) : 0);
+  if (p.time_approximation != MF_TA_HANCOCK)  // (Hancock: one flux launch per direction)
+    L->launches += per * (mf::flux_launches(L->ctx->dp, p.precision,
+                                            L->flux_form == MF_FLUX_LINES) - sd);
 }
 
 // Work list of the fused kernel: each desc's valueBox cut into tiles of the
@@ -1411,6 +1414,7 @@ static mf_status enqueue_level_step(mf_level* L, int advance, cudaEvent_t* ev = 
   // chunked flux / update overlap of the split mixed-precision stages
   const bool overlap = L->nchunks > 1 && !L->fused && L->gathers.empty() && !c->dp.ct;
   const bool lines = L->flux_form == MF_FLUX_LINES;
+  const int nflux = mf::flux_launches(c->dp, p.precision, lines);
   auto stage_marks = [&](int n0) {
     if (!ev) return;
     kinds[n0] = 1;
@@ -1425,9 +1429,9 @@ static mf_status enqueue_level_step(mf_level* L, int advance, cudaEvent_t* ev = 
       ne = n0 + np0 + L->nchunks + 1;
       return;
     }
-    for (int d = 0; d < sd; ++d) kinds[n0 + np0 + d] = 2;
-    kinds[n0 + np0 + sd] = 3;
-    ne = n0 + np0 + 1 + sd;
+    for (int q = 0; q < nflux; ++q) kinds[n0 + np0 + q] = 2;
+    kinds[n0 + np0 + nflux] = 3;
+    ne = n0 + np0 + 1 + nflux;
   };
   if (!lean) {
     MF_CHECK_CUDA(
@@ -1762,14 +1766,12 @@ mf_status mf_level_create(mf_ctx* c, int npatch, const mf_box* valid, mf_level**
     if (p.time_approximation == MF_TA_RK2 && L->ntwo) L->launches -= 1;
     L->launches += stages * (mf::prim_launches(&L->lp, mixed) - 1);
   }
-  // one fused kernel instead of the fluxes and the update (while no gathers)
-  L->fused_saving = L->fused ? ((p.time_approximation == MF_TA_RK2) ? 2 : 1) * sd : 0;
   if (L->nsun) L->launches += 1;
   // constrained transport: edge field + recalculation per stage, the dt after
   // them, and the level's recalculation
   if (c->dp.ct) L->launches += (p.time_approximation == MF_TA_RK2) ? 6 : 4;
   L->base_launches = L->launches;
-  L->launches -= L->fused_saving;
+  count_launches(L);
   *out = L;
   return MF_OK;
 }
@@ -2151,6 +2153,7 @@ static mf_status level_set_flux_form(mf_level* L, int form) {
     }
   }
   L->flux_form = form;
+  count_launches(L);
   if (L->gsync) cudaGraphExecDestroy(L->gsync);
   if (L->gasync) cudaGraphExecDestroy(L->gasync);
   L->gsync = L->gasync = nullptr;
@@ -2255,16 +2258,8 @@ static mf_status time_kind(mf_level* L, int kind, int reps, cudaEvent_t e0, cuda
     } else if (kind == 1) {
       const mf::LinePlan& lp = (p.time_approximation == MF_TA_RK2) ? L->lp1 : L->lp2;
       const bool lines = L->flux_form == MF_FLUX_LINES;
-      for (int d = 0; d < sd && e == cudaSuccess; ++d) {
-        if (p.precision == MF_PREC_MIXED)
-          e = mf::launch_flux_fast<float>(c->dp, d, B.w, B.f[d], B.bn[d], b, ds, L->s, B.wf);
-        else if (p.precision == MF_PREC_FP64_FAST)
-          e = lines ? mf::launch_flux_lines_fast(c->dp, d, B.w, B.f[d], B.bn[d], b, lp, ds, L->s)
-                    : mf::launch_flux_fast<double>(c->dp, d, B.w, B.f[d], B.bn[d], b, ds, L->s);
-        else
-          e = lines ? mf::launch_flux_lines_exact(c->dp, d, B.w, B.f[d], B.bn[d], b, lp, ds, L->s)
-                    : mf::launch_flux_exact(c->dp, d, B.w, B.f[d], B.bn[d], b, ds, L->s);
-      }
+      B.lines = lines ? &lp : nullptr;
+      e = mf::launch_fluxes(c->dp, p.precision, B, b, ds, L->s, nullptr);
     } else if (kind == 4) {  // fluxes + update of stage 1 in the level's chunks, overlapped
       StageBuffers Bo = B;
       Bo.overlap = (p.time_approximation == MF_TA_RK2) ? &L->op1 : &L->op2;

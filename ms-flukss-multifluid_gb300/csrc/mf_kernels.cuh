@@ -271,6 +271,30 @@ cudaError_t launch_flux_exact(const DevParams& P, int dir, const double* w, void
 cudaError_t launch_update_exact(const DevParams& P, const StageBuffers& B, const Batch& b,
                                 int flags, double dt_scale, StepState* state,
                                 DtPartial* partials, int* nblocks_v, cudaStream_t s);
+// FP64 face fluxes of every direction with the plasma and the neutral
+// populations in launches of their own (mf_face_kernel.cuh): every option but
+// characteristic reconstruction, HELIOBC and tracking surfaces, whose plasma
+// and neutral parts share more than the face.  launch_fluxes picks it.
+inline bool flux_split(const DevParams& P, int precision) {
+  return precision != MF_PREC_MIXED && !P.char_rec && !P.helio_bc && P.nls == 0;
+}
+cudaError_t launch_plasma_exact(const DevParams& P, const double* w, void* const f[3],
+                                void* const bn[3], const Batch& b, const StepState* state,
+                                cudaStream_t s);
+cudaError_t launch_neutral_exact(const DevParams& P, const double* w, void* const f[3],
+                                 const Batch& b, cudaStream_t s);
+cudaError_t launch_plasma_fast(const DevParams& P, const double* w, void* const f[3],
+                               void* const bn[3], const Batch& b, const StepState* state,
+                               cudaStream_t s);
+cudaError_t launch_neutral_fast(const DevParams& P, const double* w, void* const f[3],
+                                const Batch& b, cudaStream_t s);
+// The face fluxes and Bn of every direction of a stage from B.w / B.wf, in
+// flux_launches launches, with B.ev's events from *ne on after each.
+cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers& B,
+                          const Batch& b, const StepState* state, cudaStream_t s, int* ne);
+inline int flux_launches(const DevParams& P, int precision, bool lines) {
+  return (!lines && flux_split(P, precision)) ? 1 + (P.nf > 1 ? 1 : 0) : P.sd;
+}
 // fast physics: R = float (mixed precision) or double (fast FP64)
 // wf (R = float only, nullable): the FP32 copy of w the prim kernel wrote
 // face fluxes by lines (k_lflux), FP64 paths; *_prepare once per device

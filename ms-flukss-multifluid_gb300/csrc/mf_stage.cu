@@ -4,6 +4,35 @@
 
 namespace mf {
 
+cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers& B,
+                          const Batch& b, const StepState* state, cudaStream_t s, int* ne) {
+  cudaError_t e = cudaSuccess;
+  auto done = [&]() {
+    if (e == cudaSuccess && B.ev) cudaEventRecord(B.ev[(*ne)++], s);
+    return e;
+  };
+  if (!B.lines && flux_split(P, precision)) {
+    const bool fast = precision == MF_PREC_FP64_FAST;
+    e = fast ? launch_plasma_fast(P, B.w, B.f, B.bn, b, state, s)
+             : launch_plasma_exact(P, B.w, B.f, B.bn, b, state, s);
+    if (done() != cudaSuccess || P.nf < 2) return e;
+    e = fast ? launch_neutral_fast(P, B.w, B.f, b, s) : launch_neutral_exact(P, B.w, B.f, b, s);
+    return done();
+  }
+  for (int d = 0; d < P.sd; ++d) {
+    if (precision == MF_PREC_MIXED)
+      e = launch_flux_fast<float>(P, d, B.w, B.f[d], B.bn[d], b, state, s, B.wf);
+    else if (precision == MF_PREC_FP64_FAST)
+      e = B.lines ? launch_flux_lines_fast(P, d, B.w, B.f[d], B.bn[d], b, *B.lines, state, s)
+                  : launch_flux_fast<double>(P, d, B.w, B.f[d], B.bn[d], b, state, s);
+    else
+      e = B.lines ? launch_flux_lines_exact(P, d, B.w, B.f[d], B.bn[d], b, *B.lines, state, s)
+                  : launch_flux_exact(P, d, B.w, B.f[d], B.bn[d], b, state, s);
+    if (done() != cudaSuccess) return e;
+  }
+  return e;
+}
+
 cudaError_t launch_stage(const DevParams& P, int precision, const StageBuffers& B,
                          const Batch& b, int flags, double dt_scale, StepState* state,
                          DtPartial* partials, int* nblocks_v, cudaStream_t s) {
@@ -50,18 +79,8 @@ cudaError_t launch_stage(const DevParams& P, int precision, const StageBuffers& 
     if (B.ev) cudaEventRecord(B.ev[ne++], s);
     return cudaSuccess;
   }
-  for (int d = 0; d < P.sd; ++d) {
-    if (precision == MF_PREC_MIXED)
-      e = launch_flux_fast<float>(P, d, B.w, B.f[d], B.bn[d], b, state, s, B.wf);
-    else if (precision == MF_PREC_FP64_FAST)
-      e = B.lines ? launch_flux_lines_fast(P, d, B.w, B.f[d], B.bn[d], b, *B.lines, state, s)
-                  : launch_flux_fast<double>(P, d, B.w, B.f[d], B.bn[d], b, state, s);
-    else
-      e = B.lines ? launch_flux_lines_exact(P, d, B.w, B.f[d], B.bn[d], b, *B.lines, state, s)
-                  : launch_flux_exact(P, d, B.w, B.f[d], B.bn[d], b, state, s);
-    if (e != cudaSuccess) return e;
-    if (B.ev) cudaEventRecord(B.ev[ne++], s);
-  }
+  e = launch_fluxes(P, precision, B, b, state, s, &ne);
+  if (e != cudaSuccess) return e;
   if (precision == MF_PREC_MIXED)
     e = launch_update_fast<float>(P, B, b, flags, dt_scale, state, partials, nblocks_v, s);
   else if (precision == MF_PREC_FP64_FAST)
