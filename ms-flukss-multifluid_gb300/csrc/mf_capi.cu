@@ -766,7 +766,7 @@ static mf_status patch_update_impl(mf_ctx* c, mf_fab* U, const mf_box* valid, do
   MF_CHECK_CUDA(c->state.ensure(sizeof(StepState)));
   MF_CHECK_CUDA(c->hstate.ensure(sizeof(StepState)));
   const long long vmax = box_cells(v2);
-  const long long nparts = (vmax + 127) / 128 + 1;
+  const long long nparts = (vmax + mf::kCellBlock - 1) / mf::kCellBlock + 1;
   MF_CHECK_CUDA(c->partials.ensure(sizeof(DtPartial) * nparts));
 
   SingleBlock* hb = (SingleBlock*)c->hdesc.p;
@@ -892,7 +892,8 @@ static mf_status patch_update_impl(mf_ctx* c, mf_fab* U, const mf_box* valid, do
       MF_CHECK_CUDA(mf::launch_dt(c->dp, U->data, b2, parts, &nb, s));
     }
   }
-  MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, b2, b2.nt[2], ds, 0, s));
+  MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, b2, mf::update_cells(c->dp, p.precision, b2),
+                                    ds, 0, s));
   if (ct && E)  // updateState's E: the step average (RK2) or the one stage's field
     MF_CHECK_CUDA(
         mf::launch_edges_out(sd, rk2 ? (const double*)c->ct_eo.p : e2, U->box, *valid, E, s));
@@ -1551,7 +1552,8 @@ static mf_status enqueue_level_step(mf_level* L, int advance, cudaEvent_t* ev = 
     }
     if ((gst = gather(2)) != MF_OK) return gst;
   }
-  MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, L->b2, L->b2.nt[2], ds, advance, s,
+  MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, L->b2,
+                                    mf::update_cells(c->dp, p.precision, L->b2), ds, advance, s,
                                     fused ? L->fp2.ntiles : 0));
   mark(4);
   // HeliosphericProblem::postTimeStep (swlism/HeliosphericProblem.cpp:2472-2535),

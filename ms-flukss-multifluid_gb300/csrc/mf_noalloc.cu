@@ -193,10 +193,15 @@ extern "C" mf_status mf_patch_update_noalloc(mf_ctx* ctx, mf_fab* U, const mf_bo
   off += up256(sizeof(StageDesc) * 2 + sizeof(mf::RunParams));
   const size_t o_state = off;
   off += up256(sizeof(StepState));
-  const long long nparts = (cells(v2) + mf::kBlock - 1) / mf::kBlock + 1;
+  const auto parts_bytes = [&](int per) {
+    return up256(sizeof(DtPartial) * ((cells(v2) + per - 1) / per + 1));
+  };
   const size_t o_parts = off;
-  off += up256(sizeof(DtPartial) * nparts);
-  if (off > (size_t)MF_NOALLOC_SCRATCH_BYTES) return MF_ERR_SCRATCH_LIMIT;
+  if (off + parts_bytes(mf::kBlock) > (size_t)MF_NOALLOC_SCRATCH_BYTES)
+    return MF_ERR_SCRATCH_LIMIT;
+  // a patch that fills the array leaves no room for the finer partials of the
+  // update by fluid: it takes the update by cell
+  const int whole = off + parts_bytes(mf::kCellBlock) > (size_t)MF_NOALLOC_SCRATCH_BYTES;
 
   void* basev = nullptr;
   mf_status st = scratch_base(&basev);
@@ -244,6 +249,7 @@ extern "C" mf_status mf_patch_update_noalloc(mf_ctx* ctx, mf_fab* U, const mf_bo
 
   StageBuffers B;
   std::memset(&B, 0, sizeof(B));
+  B.by_cell = whole;
   B.w = (double*)(base + o_w);
   int nb = 0;
   if (divB && divB->data) {
@@ -283,7 +289,8 @@ extern "C" mf_status mf_patch_update_noalloc(mf_ctx* ctx, mf_fab* U, const mf_bo
     B.divb = (divB && divB->data) ? divB->data : nullptr;
     NA_CUDA(mf::launch_stage(*cv.dp, p.precision, B, b2, mf::kStageDt, 1.0, ds, parts, &nb, s));
   }
-  NA_CUDA(mf::launch_finalize(*cv.dp, parts, b2, b2.nt[2], ds, 0, s));
+  NA_CUDA(mf::launch_finalize(*cv.dp, parts, b2,
+                              mf::update_cells(*cv.dp, p.precision, b2, whole), ds, 0, s));
   if (F) {
     const void* f2p[3] = {nullptr, nullptr, nullptr};
     const void* f1p[3] = {nullptr, nullptr, nullptr};

@@ -15,8 +15,9 @@ namespace exact {
 // are the routine's literals.  Its x > 650 test reads the x of the last
 // solar-wind cell the routine visited (x is assigned in that branch only);
 // here the cell's own x, the same on every domain within x <= 650.
+template <typename WA>
 __device__ __forceinline__ int region_tracer_cell(const DevParams& P, double dx, int i, int j,
-                                                  int k, const double* w, double regtr) {
+                                                  int k, const WA& w, double regtr) {
   const double x = (i + 0.5) * dx - P.sun_c[0];
   const double ux = w[1], uy = w[2], uz = w[3];
   int reg;
@@ -58,8 +59,9 @@ __device__ __forceinline__ int region_tracer_cell(const DevParams& P, double dx,
 // DEFINE_REGIONS_2F (swlism/SWLISMF.ChF:654-742), Cartesian branch, or the
 // tracer variant above (HeliosphericProblem::defineRegions,
 // swlism/HeliosphericProblem.cpp:2538-2575).
+template <typename WA>
 __device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i, int j, int k,
-                                           const double* w, double regtr) {
+                                           const WA& w, double regtr) {
   if (P.reg_tracer) return region_tracer_cell(P, dx, i, j, k, w, regtr);
   using namespace ieee64;
   double x = (i + 0.5) * dx - P.sun_c[0];
@@ -101,116 +103,134 @@ __device__ __forceinline__ int ce_recipient(int nN, int reg) {
   return (reg >= 1 && reg <= nN) ? reg : 0;
 }
 
-// Pauls & Zank charge-exchange rates of one cell; adds S = -dt*H to u
-// (HeliosphericProblem::explicitSource, swlism/HeliosphericProblem.cpp:1394-1539).
-// T names the arithmetic type for interface symmetry with the fast physics;
-// the parity physics is FP64 only.
-// NN > 0: the number of neutral populations fixed at compile time (the same
-// operations in the same order; the loops run a known count, so the
-// populations' independent chains can be scheduled together); 0: P.nf - 1.
+// Pauls & Zank charge exchange of the plasma with one neutral population
+// (HeliosphericProblem::explicitSource, swlism/HeliosphericProblem.cpp:1394-1539;
+// CHARGE_EXCHANGE_*, swlism/ChargeExchange2F.ChF:294-1149).
+struct CeTerms {
+  static constexpr int kShared = 9;
+  // what the plasma sums over the populations: the terms of h2..h5, ARR UD
+  // (-DENPLU) and the terms of PPLUX, PPLUY, PPLUZ, ENPLU
+  double shared[kShared];
+  double pmi[3], enmi;  // PMIX, PMIY, PMIZ, ENMI
+};
+
+// w: the stage-start primitive state; o: the population's first component.
+// Factors that are powers of two scale exactly and move out of the products.
+template <typename WA>
+__device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const WA& w, int o,
+                                                      CeTerms& c) {
+  using namespace ieee64;
+  const double rho = w[0], ux = w[1], uy = w[2], uz = w[3], pp = w[4];
+  const double rhoN = w[o], uxN = w[o + 1], uyN = w[o + 2], uzN = w[o + 3], pN = w[o + 4];
+  const double U2 = ux * ux + uy * uy + uz * uz;
+  const double VVTP = div(pp, rho);
+  const double dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
+  const double UH2 = uxN * uxN + uyN * uyN + uzN * uzN;
+  const double DU2 = dx_ * dx_ + dy_ * dy_ + dz_ * dz_, DU24 = scale<2>(DU2);
+  const double VPHH = dx_ * uxN + dy_ * uyN + dz_ * uzN;
+  const double VPHP = dx_ * ux + dy_ * uy + dz_ * uz;
+  const double VVTH = div(scale<1>(pN), rhoN);
+  const double UD = root(div(scale<2>(VVTP + VVTH), kPi) + DU2);
+  const double UPM = root(div(scale<4>(VVTP), kPi) + 2.25 * kPi * VVTH + DU24);
+  const double UHM = root(2.25 * kPi * VVTP + div(scale<4>(VVTH), kPi) + DU24);
+  const double UPE = root(div(scale<2>(VVTP) + div(scale<6>(VVTH), 9.0), kPi) + DU2);
+  const double UHE = root(div(div(scale<6>(VVTP), 9.0) + scale<2>(VVTH), kPi) + DU2);
+  const double UDS = P.ce_scale_vel * UD;
+  const double t = P.ce_a - P.ce_b * log(UDS);
+  double SIG = t * t;
+  if (P.ce_damp_c > 0.0) SIG = SIG * pow(1.0 - exp(-P.ce_damp_c / UDS), P.ce_damp_pow);
+  SIG = P.ce_sigma_scale * SIG;
+  const double ARR = SIG * rhoN * rho;
+  const double VVTHU = div(VVTH, UPM);
+  const double hs = UD + VVTHU + div(VVTP, UHM);
+  c.shared[0] = ARR * dx_ * hs;
+  c.shared[1] = ARR * dy_ * hs;
+  c.shared[2] = ARR * dz_ * hs;
+  c.shared[3] = half(ARR) * (1.5 * (UHE * VVTP - UPE * VVTH) + UD * (U2 - UH2) +
+                             scale<1>(VVTHU * VPHH + div(VVTP * VPHP, UHM)));
+  c.shared[4] = ARR * UD;
+  // -(uxN - ux) == ux - uxN exactly
+  c.shared[5] = ARR * (ux * UD + div(dx_ * VVTP, UHM));
+  c.shared[6] = ARR * (uy * UD + div(dy_ * VVTP, UHM));
+  c.shared[7] = ARR * (uz * UD + div(dz_ * VVTP, UHM));
+  c.shared[8] = ARR * (half(U2) * UD + VVTP * (div(VPHP, UHM) + 0.75 * UHE));
+  c.pmi[0] = ARR * (uxN * UD - dx_ * VVTHU);
+  c.pmi[1] = ARR * (uyN * UD - dy_ * VVTHU);
+  c.pmi[2] = ARR * (uzN * UD - dz_ * VVTHU);
+  c.enmi = ARR * (half(UH2) * UD - VPHH * VVTHU + 0.75 * VVTH * UPE);
+}
+
+// S = -dt H of the plasma (momentum and energy; the magnetic field's and
+// psi's S is zero).  at(f, q): CeTerms::shared[q] of population f (from 0);
+// NN populations, or nN at run time with NN = 0.
+template <int NN, typename AT>
+__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at,
+                                                       int nN = NN) {
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    double h = 0.0;
+#pragma unroll
+    for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
+      if (f < (NN > 0 ? NN : nN)) h = h + at(f, q);
+    u[1 + q] = u[1 + q] + (-dt * h);
+  }
+}
+
+// S = -dt H of population f (from 0) with terms c; rec: it receives the
+// newly created neutrals.
+template <int NN, typename AT>
+__device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const CeTerms& c,
+                                                        double dt, double* un, const AT& at,
+                                                        int nN_ = NN) {
+  const int nN = NN > 0 ? NN : nN_;
+  double H1 = c.shared[4], H2 = c.pmi[0], H3 = c.pmi[1], H4 = c.pmi[2], H5 = c.enmi;
+  if (rec) {
+    double X = 0.0, Y = 0.0, Z = 0.0, E = 0.0, sum = 0.0;
+    bool first = true;
+#pragma unroll
+    for (int q = 0; q < MF_MAX_FLUIDS - 1; ++q) {
+      if (q < nN) {
+        X = X - at(q, 5);
+        Y = Y - at(q, 6);
+        Z = Z - at(q, 7);
+        E = E - at(q, 8);
+        if (nN > 3 || q != f) {
+          sum = first ? -at(q, 4) : sum - at(q, 4);
+          first = false;
+        }
+      }
+    }
+    H1 = (nN > 3) ? sum + c.shared[4] : sum;
+    H2 = X + H2;
+    H3 = Y + H3;
+    H4 = Z + H4;
+    H5 = E + H5;
+  }
+  un[0] = un[0] + (-dt * H1);
+  un[1] = un[1] + (-dt * H2);
+  un[2] = un[2] + (-dt * H3);
+  un[3] = un[3] + (-dt * H4);
+  un[4] = un[4] + (-dt * H5);
+}
+
+// All populations of one cell by one thread.  T names the arithmetic type for
+// interface symmetry with the fast physics; the parity physics is FP64 only.
+// NN > 0: the number of populations fixed at compile time; 0: P.nf - 1.
 template <int IRHON, typename T = double, typename WA = const double*, int NN = 0>
 __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA& w, int reg,
                                                     double dt, double* u) {
   static_assert(sizeof(T) == sizeof(double), "FP64 physics");
-  using namespace ieee64;
   const int nN = NN > 0 ? NN : P.nf - 1;
-  const double rho = w[0], ux = w[1], uy = w[2], uz = w[3], pp = w[4];
-  const double U2 = ux * ux + uy * uy + uz * uz;
-  const double VVTP = div(pp, rho);
-  // plasma terms of the speeds, the same for every population; factors that
-  // are powers of two scale exactly
-  const double tp4 = scale<2>(VVTP), hU2 = half(U2);
-  const double tp16 = div(scale<4>(VVTP), kPi), tpc = 2.25 * kPi * VVTP, tp649 = div(scale<6>(VVTP), 9.0);
-  double h2 = 0, h3 = 0, h4 = 0, h5 = 0, PPLUX = 0, PPLUY = 0, PPLUZ = 0, ENPLU = 0;
-  double DENPLU[MF_MAX_FLUIDS], PMIX[MF_MAX_FLUIDS], PMIY[MF_MAX_FLUIDS], PMIZ[MF_MAX_FLUIDS],
-      ENMI[MF_MAX_FLUIDS];
+  CeTerms c[MF_MAX_FLUIDS - 1];
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f > nN) break;
-    const double* wn = w + IRHON + (f - 1) * 5;
-    const double rhoN = wn[0], uxN = wn[1], uyN = wn[2], uzN = wn[3], pN = wn[4];
-    const double dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
-    const double UH2 = uxN * uxN + uyN * uyN + uzN * uzN;
-    const double DU2 = dx_ * dx_ + dy_ * dy_ + dz_ * dz_, DU24 = scale<2>(DU2);
-    const double VPHH = dx_ * uxN + dy_ * uyN + dz_ * uzN;
-    const double VPHP = dx_ * ux + dy_ * uy + dz_ * uz;
-    const double VVTH = div(scale<1>(pN), rhoN);
-    const double th4 = scale<2>(VVTH);
-    const double UD = root(div(scale<2>(VVTP + VVTH), kPi) + DU2);
-    const double UPM = root(tp16 + 2.25 * kPi * VVTH + DU24);
-    const double UHM = root(tpc + div(scale<4>(VVTH), kPi) + DU24);
-    const double UPE = root(div(tp4 + div(scale<6>(VVTH), 9.0), kPi) + DU2);
-    const double UHE = root(div(tp649 + th4, kPi) + DU2);
-    const double UDS = P.ce_scale_vel * UD;
-    const double t = P.ce_a - P.ce_b * log(UDS);
-    double SIG = t * t;
-    if (P.ce_damp_c > 0.0) SIG = SIG * pow(1.0 - exp(-P.ce_damp_c / UDS), P.ce_damp_pow);
-    SIG = P.ce_sigma_scale * SIG;
-    const double ARR = SIG * rhoN * rho;
-    const double VVTHU = div(VVTH, UPM);
-    const double hs = UD + VVTHU + div(VVTP, UHM);
-    h2 = h2 + ARR * dx_ * hs;
-    h3 = h3 + ARR * dy_ * hs;
-    h4 = h4 + ARR * dz_ * hs;
-    h5 = h5 + half(ARR) * (1.5 * (UHE * VVTP - UPE * VVTH) + UD * (U2 - UH2) +
-                           scale<1>(VVTHU * VPHH + div(VVTP * VPHP, UHM)));
-    DENPLU[f] = -ARR * UD;
-    // -(uxN - ux) == ux - uxN exactly
-    PPLUX = PPLUX - ARR * (ux * UD + div(dx_ * VVTP, UHM));
-    PPLUY = PPLUY - ARR * (uy * UD + div(dy_ * VVTP, UHM));
-    PPLUZ = PPLUZ - ARR * (uz * UD + div(dz_ * VVTP, UHM));
-    ENPLU = ENPLU - ARR * (hU2 * UD + VVTP * (div(VPHP, UHM) + 0.75 * UHE));
-    PMIX[f] = ARR * (uxN * UD - dx_ * VVTHU);
-    PMIY[f] = ARR * (uyN * UD - dy_ * VVTHU);
-    PMIZ[f] = ARR * (uzN * UD - dz_ * VVTHU);
-    ENMI[f] = ARR * (half(UH2) * UD - VPHH * VVTHU + 0.75 * VVTH * UPE);
-  }
-  u[1] = u[1] + (-dt * h2);
-  u[2] = u[2] + (-dt * h3);
-  u[3] = u[3] + (-dt * h4);
-  u[4] = u[4] + (-dt * h5);
-  // S of the magnetic field (and of psi) is zero: u + 0 == u
+  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
+    if (f < nN) charge_exchange_terms(P, w, IRHON + f * 5, c[f]);
+  auto at = [&](int f, int q) { return c[f].shared[q]; };
+  charge_exchange_plasma<NN>(dt, u, at, nN);
   const int rk = ce_recipient(nN, reg);
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f > nN) break;
-    double H1, H2, H3, H4, H5;
-    if (f == rk) {
-      if (nN <= 3) {
-        bool first = true;
-        H1 = 0.0;
-#pragma unroll
-        for (int q = 1; q < MF_MAX_FLUIDS; ++q) {
-          if (q > nN) break;
-          if (q == f) continue;
-          H1 = first ? DENPLU[q] : H1 + DENPLU[q];
-          first = false;
-        }
-      } else {
-        double sum = DENPLU[1];
-#pragma unroll
-        for (int q = 2; q < MF_MAX_FLUIDS; ++q)
-          if (q <= nN) sum = sum + DENPLU[q];
-        H1 = sum - DENPLU[f];
-      }
-      H2 = PPLUX + PMIX[f];
-      H3 = PPLUY + PMIY[f];
-      H4 = PPLUZ + PMIZ[f];
-      H5 = ENPLU + ENMI[f];
-    } else {
-      H1 = -DENPLU[f];
-      H2 = PMIX[f];
-      H3 = PMIY[f];
-      H4 = PMIZ[f];
-      H5 = ENMI[f];
-    }
-    double* un = u + IRHON + (f - 1) * 5;
-    un[0] = un[0] + (-dt * H1);
-    un[1] = un[1] + (-dt * H2);
-    un[2] = un[2] + (-dt * H3);
-    un[3] = un[3] + (-dt * H4);
-    un[4] = un[4] + (-dt * H5);
-  }
+  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
+    if (f < nN) charge_exchange_neutral<NN>(f + 1 == rk, f, c[f], dt, u + IRHON + f * 5, at, nN);
 }
 
 // HELIOREINIT_DEFAULT (swlism/HeliosphericPlasmaBCF.ChF:1435-1566) at time t
@@ -271,16 +291,22 @@ static __device__ __host__ __forceinline__ void reinit_state(const ReinitIn P, d
 }
 
 // The reset of one cell: the membership test, then the wind state.
-__device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double dx, int i, int j, int k,
-                                            double t, double* u) {
+__device__ __host__ __forceinline__ bool reinit_wind(const DevParams& P, double dx, int i, int j,
+                                                     int k, double t, ReinitState& o) {
   double x = (i + 0.5) * dx - P.sun_c[0];
   double y = (j + 0.5) * dx - P.sun_c[1];
   double z = 0.0;
   if (P.sd == 3) z = (k + 0.5) * dx - P.sun_c[2];
   double r2 = (P.sd == 3) ? (x * x + y * y + z * z) : (x * x + y * y);
-  if (!(r2 <= P.r0 * P.r0)) return;
-  ReinitState o;
+  if (!(r2 <= P.r0 * P.r0)) return false;
   reinit_state(reinit_in(P), x, y, z, r2, t, o);
+  return true;
+}
+
+__device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double dx, int i, int j, int k,
+                                            double t, double* u) {
+  ReinitState o;
+  if (!reinit_wind(P, dx, i, j, k, t, o)) return;
 #pragma unroll
   for (int q = 0; q < 8; ++q) u[q] = o.u[q];
   if (!P.monopolar) {
@@ -292,10 +318,18 @@ __device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double 
   }
 }
 
+// The plasma alone (no tracking surfaces).
+__device__ __forceinline__ void reinit_plasma(const DevParams& P, double dx, int i, int j, int k,
+                                              double t, double* u) {
+  ReinitState o;
+  if (!reinit_wind(P, dx, i, j, k, t, o)) return;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) u[q] = o.u[q];
+}
+
 // POSTPROCESSING (srcIdeal/PatchIdealMHDF.ChF:1019-1070) and POSTPROCESSING_MF
 // (srcIdeal/PatchMHDMFF.ChF:301-511).
-template <int IRHON>
-__device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
+__device__ __forceinline__ void positivity_plasma(const DevParams& P, double* u) {
   using namespace ieee64;
   const double hg = P.hgamma, smallR = P.smallr, smallP = P.smallp;
   if (P.nf == 1) {
@@ -332,73 +366,83 @@ __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
       u[4] = Pr / hg + Rho * UxU + BxB;
     }
   }
-#pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f >= P.nf) break;
-    double fd = (f == 1) ? smallR : (f == 3) ? kNet3Dens : kNet2Dens;
-    double fp = (f == 1) ? smallP : (f == 3) ? kNet3Pres : kNet2Pres;
-    double* un = u + IRHON + (f - 1) * 5;
-    double Rho = un[0];
-    double invRho = div(1.0, Rho);
-    double Ux = un[1] * invRho, Uy = un[2] * invRho, Uz = un[3] * invRho;
-    double UxU = half(Ux * Ux + Uy * Uy + Uz * Uz);
-    double Pr = hg * (un[4] - Rho * UxU);
-    bool was = false;
-    if (lt(Rho, fd)) { Rho = fd; was = true; }
-    if (lt(Pr, fp)) { Pr = fp; was = true; }
-    if (was) {
-      un[0] = Rho;
-      un[1] = Rho * Ux;
-      un[2] = Rho * Uy;
-      un[3] = Rho * Uz;
-      un[4] = Pr / hg + Rho * UxU;
-    }
+}
+
+// neutral fluid f (from 1)
+__device__ __forceinline__ void positivity_neutral(const DevParams& P, int f, double* un) {
+  using namespace ieee64;
+  const double hg = P.hgamma, smallR = P.smallr, smallP = P.smallp;
+  double fd = (f == 1) ? smallR : (f == 3) ? kNet3Dens : kNet2Dens;
+  double fp = (f == 1) ? smallP : (f == 3) ? kNet3Pres : kNet2Pres;
+  double Rho = un[0];
+  double invRho = div(1.0, Rho);
+  double Ux = un[1] * invRho, Uy = un[2] * invRho, Uz = un[3] * invRho;
+  double UxU = half(Ux * Ux + Uy * Uy + Uz * Uz);
+  double Pr = hg * (un[4] - Rho * UxU);
+  bool was = false;
+  if (lt(Rho, fd)) { Rho = fd; was = true; }
+  if (lt(Pr, fp)) { Pr = fp; was = true; }
+  if (was) {
+    un[0] = Rho;
+    un[1] = Rho * Ux;
+    un[2] = Rho * Uy;
+    un[3] = Rho * Uz;
+    un[4] = Pr / hg + Rho * UxU;
   }
+}
+
+template <int IRHON>
+__device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
+  positivity_plasma(P, u);
+#pragma unroll
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f)
+    if (f < P.nf) positivity_neutral(P, f, u + IRHON + (f - 1) * 5);
 }
 
 // MAXWAVESPEED (srcIdeal/PatchIdealMHDF.ChF:5-63) + MAXWAVESPEED_E
 // (srcIdeal/PatchEulerF.ChF:5-50) of one cell.
+__device__ __forceinline__ double wave_speed_plasma(const DevParams& P, const double* u) {
+  using namespace ieee64;
+  double rho = u[0];
+  double invrho = div(1.0, rho);
+  double ru = u[1], rv = u[2], rw = u[3];
+  double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
+  double ke = ru * uu + rv * vv + rw * ww;
+  double bx = u[5], by = u[6], bz = u[7];
+  double b = kInv4Pi * (bx * bx + by * by + bz * bz);
+  double p = P.hgamma * (u[4] - half(ke + b));
+  p = maxnum(p, P.smallp);
+  double a2 = P.gamma * p * invrho;
+  double as2 = half(a2 + invrho * b);
+  double as4 = as2 * as2;
+  double bn2 = kInv4Pi * bx * bx * invrho;
+  double umax = absval(uu) + root(as2 + root(as4 - a2 * bn2));
+  bn2 = kInv4Pi * by * by * invrho;
+  umax = maxnum(absval(vv) + root(as2 + root(as4 - a2 * bn2)), umax);
+  bn2 = kInv4Pi * bz * bz * invrho;
+  return maxnum(absval(ww) + root(as2 + root(as4 - a2 * bn2)), umax);
+}
+
+__device__ __forceinline__ double wave_speed_neutral(const DevParams& P, const double* un) {
+  using namespace ieee64;
+  double rho = maxnum(un[0], P.smallr);
+  double invrho = div(1.0, rho);
+  double ru = un[1], rv = un[2], rw = un[3];
+  double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
+  double ke = ru * uu + rv * vv + rw * ww;
+  double p = P.hgamma * (un[4] - half(ke));
+  p = maxnum(p, P.smallp);
+  double a = root(P.gamma * p * invrho);
+  return maxnum(maxnum(absval(uu), absval(vv)), absval(ww)) + a;
+}
+
 template <int IRHON, typename T = double>
 __device__ __forceinline__ double max_wave_speed(const DevParams& P, const double* u) {
   static_assert(sizeof(T) == sizeof(double), "FP64 physics");
-  using namespace ieee64;
-  double cmax = 0.0;
-  {
-    double rho = u[0];
-    double invrho = div(1.0, rho);
-    double ru = u[1], rv = u[2], rw = u[3];
-    double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
-    double ke = ru * uu + rv * vv + rw * ww;
-    double bx = u[5], by = u[6], bz = u[7];
-    double b = kInv4Pi * (bx * bx + by * by + bz * bz);
-    double p = P.hgamma * (u[4] - half(ke + b));
-    p = maxnum(p, P.smallp);
-    double a2 = P.gamma * p * invrho;
-    double as2 = half(a2 + invrho * b);
-    double as4 = as2 * as2;
-    double bn2 = kInv4Pi * bx * bx * invrho;
-    double umax = absval(uu) + root(as2 + root(as4 - a2 * bn2));
-    bn2 = kInv4Pi * by * by * invrho;
-    umax = maxnum(absval(vv) + root(as2 + root(as4 - a2 * bn2)), umax);
-    bn2 = kInv4Pi * bz * bz * invrho;
-    umax = maxnum(absval(ww) + root(as2 + root(as4 - a2 * bn2)), umax);
-    cmax = maxnum(umax, cmax);
-  }
+  double cmax = ieee64::maxnum(wave_speed_plasma(P, u), 0.0);
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f >= P.nf) break;
-    const double* un = u + IRHON + (f - 1) * 5;
-    double rho = maxnum(un[0], P.smallr);
-    double invrho = div(1.0, rho);
-    double ru = un[1], rv = un[2], rw = un[3];
-    double uu = ru * invrho, vv = rv * invrho, ww = rw * invrho;
-    double ke = ru * uu + rv * vv + rw * ww;
-    double p = P.hgamma * (un[4] - half(ke));
-    p = maxnum(p, P.smallp);
-    double a = root(P.gamma * p * invrho);
-    double umax = maxnum(maxnum(absval(uu), absval(vv)), absval(ww)) + a;
-    cmax = maxnum(umax, cmax);
-  }
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f)
+    if (f < P.nf) cmax = ieee64::maxnum(wave_speed_neutral(P, u + IRHON + (f - 1) * 5), cmax);
   return cmax;
 }
 

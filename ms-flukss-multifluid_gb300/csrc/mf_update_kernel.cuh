@@ -75,8 +75,10 @@ __device__ __forceinline__ void block_dt_min(double dtc, int myidx,
       myidx = oi;
     }
   }
-  __shared__ double sdt[kMaxBlock / 32];
-  __shared__ int sidx[kMaxBlock / 32];
+  constexpr int kWarps = kCellBlock * MF_MAX_FLUIDS / 32;  // the largest block
+  static_assert(kWarps >= kMaxBlock / 32, "a slot per warp");
+  __shared__ double sdt[kWarps];
+  __shared__ int sidx[kWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) {
     sdt[wid] = dtc;

@@ -13,14 +13,16 @@ from helpers import rel_err, to_device, to_host, valid_view
 pytestmark = pytest.mark.gpu
 RTOL = 1e-12  # per step and conserved variable, the parity path's bar
 
+PLAIN = dict(divb_cleaning=0, use_8wave=1)
 FORMS = {
-    "roe7": dict(flux=1),
-    "roe7_roe_average": dict(flux=13),
-    "rusanov": dict(flux=2),
-    "roe8": dict(flux=3, divb_cleaning=0, use_8wave=1),
-    "vfroe": dict(flux=5, divb_cleaning=0, use_8wave=1),
+    "glm": dict(flux=1),
+    "glm_roe_average": dict(flux=3),
+    "roe8": dict(PLAIN, flux=1),
+    "roe7_roe_average": dict(PLAIN, flux=13),
+    "rusanov": dict(PLAIN, flux=2),
+    "vfroe": dict(PLAIN, flux=5),
     "limiters_positivity": dict(flux=1, limiters=True, check_positivity=1),
-    "central_bn": dict(flux=1, divb_method=2),
+    "central_bn": dict(PLAIN, flux=1, divb_method=2),
 }
 
 
