@@ -892,7 +892,7 @@ static mf_status patch_update_impl(mf_ctx* c, mf_fab* U, const mf_box* valid, do
       MF_CHECK_CUDA(mf::launch_dt(c->dp, U->data, b2, parts, &nb, s));
     }
   }
-  MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, b2, mf::update_cells(c->dp, p.precision, b2),
+  MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, b2, mf::update_cells(c->dp, b2),
                                     ds, 0, s));
   if (ct && E)  // updateState's E: the step average (RK2) or the one stage's field
     MF_CHECK_CUDA(
@@ -1553,7 +1553,7 @@ static mf_status enqueue_level_step(mf_level* L, int advance, cudaEvent_t* ev = 
     if ((gst = gather(2)) != MF_OK) return gst;
   }
   MF_CHECK_CUDA(mf::launch_finalize(c->dp, parts, L->b2,
-                                    mf::update_cells(c->dp, p.precision, L->b2), ds, advance, s,
+                                    mf::update_cells(c->dp, L->b2, overlap), ds, advance, s,
                                     fused ? L->fp2.ntiles : 0));
   mark(4);
   // HeliosphericProblem::postTimeStep (swlism/HeliosphericProblem.cpp:2472-2535),

@@ -9,7 +9,7 @@ namespace mf {
 cudaError_t launch_cells_exact(const DevParams& P, const StageBuffers& B, const Batch& b,
                                int flags, double dt_scale, StepState* state,
                                DtPartial* partials, int* nblocks_v, cudaStream_t s) {
-  return launch_cells_t(P, B, b, flags, dt_scale, state, partials, nblocks_v, s);
+  return launch_cells_t<double, double>(P, B, b, flags, dt_scale, state, partials, nblocks_v, s);
 }
 
 }  // namespace mf

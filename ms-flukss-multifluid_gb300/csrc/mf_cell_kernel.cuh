@@ -1,5 +1,4 @@
-// mf_cell_kernel.cuh - the update kernel of the FP64 paths with one thread
-// per cell and fluid.  Included by mf_cell_exact.cu (parity physics) and
+// mf_cell_kernel.cuh - the update kernel with one thread per cell and fluid.  Included by mf_cell_exact.cu (parity physics) and
 // mf_cell.cu (fast physics); MF_PHYS names the physics namespace.
 //
 // Bound by the FP64 pipe while enough warps are resident.  With one thread
@@ -29,15 +28,17 @@ constexpr int kCells = kCellBlock;
 #endif
 constexpr int cell_blocks(int nf) { return 65536 / (MF_CELL_REGS * kCells * nf); }
 
-template <int NF>
+// R: type of the face fluxes and wave speeds; T: type of the charge-exchange rates.
+template <int NF, typename R, typename T>
 __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     k_cells(const __grid_constant__ DevParams P, const __grid_constant__ StageBuffers B,
             const StageDesc* __restrict__ descs, int ndesc, int total, int flags,
             const RunParams* __restrict__ runs, StepState* __restrict__ states,
             const double dt_scale, DtPartial* __restrict__ partials) {
   constexpr int NN = NF - 1;
-  __shared__ double terms[NN > 0 ? NN : 1][CeTerms::kShared][kCells];
-  __shared__ double speed[NF][kCells];
+  using Terms = CeTermsT<T>;
+  __shared__ T terms[NN > 0 ? NN : 1][Terms::kShared][kCells];
+  __shared__ R speed[NF][kCells];
   __shared__ int region[kCells];
   const int role = threadIdx.x / kCells, lane = threadIdx.x % kCells;  // role 0: the plasma
   const bool plasma = NN == 0 || role == 0;
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
   int i = 0, j = 0, k = 0;
   long long cs = 0, base = 0;
   double dt = 0.0, u[9];
-  CeTerms t;
+  Terms t;
   if (Dp) {
     const StageDesc& D = *Dp;
     const RunParams& RP = runs[D.run];
@@ -69,7 +70,10 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     for (int q = 0; q < 9; ++q)
       if (q < 5 || (plasma && (q < 8 || P.glm))) u[q] = B.uin[base + (s + q) * cs];
     // UPDATECONS (src/PatchMHDAMF.ChF:542-587), one direction after another
+    // (FP32 fluxes: the differences of the directions are summed in FP32 and
+    // enter the FP64 state once, as in update_cells)
     double divB = 0.0;
+    R sum[sizeof(R) == 4 ? 9 : 1];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       if (d < P.sd) {
@@ -78,38 +82,42 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
         const long long fcs = (long long)n[0] * n[1] * n[2];
         const long long sf = (d == 0) ? 1 : (d == 1) ? (long long)n[0] : (long long)n[0] * n[1];
         const long long fo = loc(D.vlo, n, i, j, k);
-        const double* __restrict__ F = (const double*)B.f[d] + D.f_off[d] + fo + s * fcs;
+        const R* __restrict__ F = (const R*)B.f[d] + D.f_off[d] + fo + s * fcs;
 #pragma unroll
-        for (int q = 0; q < 9; ++q)
-          if (q < 5 || (plasma && (q < 8 || P.glm)))
-            u[q] = u[q] - dtinv * (F[q * fcs + sf] - F[q * fcs]);
+        for (int q = 0; q < 9; ++q) {
+          if (q < 5 || (plasma && (q < 8 || P.glm))) {
+            const R diff = F[q * fcs + sf] - F[q * fcs];
+            if constexpr (sizeof(R) == 4)
+              sum[q] = (d == 0) ? diff : sum[q] + diff;
+            else
+              u[q] = u[q] - dtinv * diff;
+          }
+        }
         if (plasma && P.use8) {  // COMPUTEDIVB
-          const double* __restrict__ b = (const double*)B.bn[d] + D.bn_off[d] + fo;
-          divB = divB + b[sf] - b[0];
+          const R* __restrict__ b = (const R*)B.bn[d] + D.bn_off[d] + fo;
+          if constexpr (sizeof(R) == 4)
+            divB = divB + fp64::f2d(b[sf] - b[0]);
+          else
+            divB = divB + b[sf] - b[0];
         }
       }
     }
+    if constexpr (sizeof(R) == 4) {
+#pragma unroll
+      for (int q = 0; q < 9; ++q)
+        if (q < 5 || (plasma && (q < 8 || P.glm))) u[q] = fma(-dtinv, fp64::f2d(sum[q]), u[q]);
+    }
     if (plasma) {
       if (P.use8) {
-        // SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES
-        const double dB = -divB * ieee64::div(dt, RP.dx);
-        const double Ux = w[1], Uy = w[2], Uz = w[3];
-        const double Bx = kInv4Pi * w[5], By = kInv4Pi * w[6], Bz = kInv4Pi * w[7];
-        u[1] = u[1] + dB * Bx;
-        u[2] = u[2] + dB * By;
-        u[3] = u[3] + dB * Bz;
-        u[4] = u[4] + dB * (Bx * Ux + By * Uy + Bz * Uz);
-        u[5] = u[5] + dB * Ux;
-        u[6] = u[6] + dB * Uy;
-        u[7] = u[7] + dB * Uz;
+        source_8wave(w, divB, ieee64::div(dt, RP.dx), u);
         if ((flags & kStageDt) && B.divb) B.divb[loc(B.divb_lo, B.divb_n, i, j, k)] = divB;
       }
       if (P.glm) u[8] = psi_damp * u[8];  // PSIPARABOLIC (src/DednerF.ChF:65-87)
       if (ce) region[lane] = region_cell(P, RP.dx, i, j, k, w, 0.0);
     } else if (ce) {
-      charge_exchange_terms(P, w, s, t);
+      charge_exchange_terms<T>(P, w, s, t);
 #pragma unroll
-      for (int q = 0; q < CeTerms::kShared; ++q) terms[role - 1][q][lane] = t.shared[q];
+      for (int q = 0; q < Terms::kShared; ++q) terms[role - 1][q][lane] = t.shared[q];
     }
   }
   if (ce) __syncthreads();
@@ -120,13 +128,20 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     // (src/PatchMHDAM.cpp:705-707); with constrained transport these follow
     // the recalculation of B
     if (plasma) {
-      if (ce) charge_exchange_plasma<NN>(dt, u, at);
+      if constexpr (NN > 0) {
+        if (ce) charge_exchange_plasma<NN, T>(dt, u, at);
+      }
       if (!P.ct) {
         if (P.reinit) reinit_plasma(P, runs[Dp->run].dx, i, j, k, stage_time(states[Dp->run], dt), u);
         positivity_plasma(P, u);
       }
     } else {
-      if (ce) charge_exchange_neutral<NN>(ce_recipient(NN, region[lane]) == role, role - 1, t, dt, u, at);
+      if constexpr (NN > 0) {
+        if (ce) {
+          const bool rec = ce_recipient(NN, region[lane]) == role;
+          charge_exchange_neutral<NN, T>(rec, role - 1, WColumn{B.w + base, cs}, t, dt, u, at);
+        }
+      }
       if (!P.ct) positivity_neutral(P, role, u);
     }
     // AVERAGESTATE (src/PatchMHDAMF.ChF:289-316): half the difference is
@@ -142,7 +157,7 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     }
     if (!finite) atomicOr(&states[Dp->run].flags, kFlagNonFinite);
     if (flags & kStageDt)
-      speed[role][lane] = plasma ? wave_speed_plasma(P, u) : wave_speed_neutral(P, u);
+      speed[role][lane] = plasma ? wave_speed_plasma<R>(P, u) : wave_speed_neutral<R>(P, u);
   }
   if (flags & kStageDt) {
     __syncthreads();
@@ -151,7 +166,7 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     if (plasma && Dp) {
       double cmax = 0.0;
 #pragma unroll
-      for (int f = 0; f < NF; ++f) cmax = ieee64::maxnum(speed[f][lane], cmax);
+      for (int f = 0; f < NF; ++f) cmax = ieee64::maxnum((double)speed[f][lane], cmax);
       dtc = ieee64::div(runs[Dp->run].dx, cmax);
       idx = g;
     }
@@ -159,15 +174,16 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
   }
 }
 
-inline cudaError_t launch_cells_t(const DevParams& P, const StageBuffers& B, const Batch& b,
+template <typename R, typename T>
+cudaError_t launch_cells_t(const DevParams& P, const StageBuffers& B, const Batch& b,
                                   int flags, double dt_scale, StepState* state,
                                   DtPartial* partials, int* nblocks_v, cudaStream_t s) {
   const unsigned nb = flat_blocks(b.tot_v, kCells);
   if (nblocks_v) *nblocks_v = (int)nb;
   if (b.tot_v <= 0) return cudaSuccess;
 #define MF_CELLS(NF)                                                                             \
-  k_cells<NF><<<nb, kCells * NF, 0, s>>>(P, B, b.desc, b.ndesc, b.tot_v, flags, b.runs, state, \
-                                         dt_scale, partials)
+  k_cells<NF, R, T><<<nb, kCells * NF, 0, s>>>(P, B, b.desc, b.ndesc, b.tot_v, flags, b.runs, \
+                                               state, dt_scale, partials)
   switch (P.nf) {
     case 1: MF_CELLS(1); break;
     case 2: MF_CELLS(2); break;

@@ -234,7 +234,7 @@ struct StageBuffers {
   const FusedPlan* fused;  // optional (mixed precision): fluxes + update in one kernel
   const OverlapPlan* overlap;  // optional (mixed precision): chunked, overlapped flux + update
   const LinePlan* lines;       // optional (FP64 paths): face fluxes by lines
-  int by_cell;  // FP64 update with one thread per cell (StageBuffers users with little scratch)
+  int by_cell;  // update with one thread per cell (callers without room for its finer partials)
 };
 
 enum StageFlags : int { kStageAverage = 1, kStageDt = 2 };
@@ -335,19 +335,23 @@ inline unsigned flat_blocks(long long n, int nt) {
   return (unsigned)(n > 0 ? (n + nt - 1) / nt : 1);
 }
 
-// The FP64 update with a thread per cell and fluid (mf_cell_kernel.cuh; blocks
-// of kCellBlock cells): every option but tracking surfaces.
+// The update with a thread per cell and fluid (mf_cell_kernel.cuh; blocks of
+// kCellBlock cells): every option but tracking surfaces.
 constexpr int kCellBlock = 64;
-inline bool update_by_fluid(const DevParams& P, int precision) {
-  return precision == MF_PREC_FP64 && P.nls == 0;
-}
+inline bool update_by_fluid(const DevParams& P) { return P.nls == 0; }
+template <typename R>
+cudaError_t launch_cells_fast(const DevParams& P, const StageBuffers& B, const Batch& b,
+                              int flags, double dt_scale, StepState* state,
+                              DtPartial* partials, int* nblocks_v, cudaStream_t s);
 cudaError_t launch_cells_exact(const DevParams& P, const StageBuffers& B, const Batch& b,
                                int flags, double dt_scale, StepState* state,
                                DtPartial* partials, int* nblocks_v, cudaStream_t s);
 // Cells per dt partial of the update kernel (with constrained transport the
 // dt comes from the dt kernel), and room for the partials of any kernel.
-inline int update_cells(const DevParams& P, int precision, const Batch& b, int by_cell = 0) {
-  return (!by_cell && !P.ct && update_by_fluid(P, precision)) ? kCellBlock : b.nt[2];
+// by_cell: the update ran with one thread per cell (StageBuffers::by_cell, or
+// the overlapped flux and update launches).
+inline int update_cells(const DevParams& P, const Batch& b, int by_cell = 0) {
+  return (!by_cell && !P.ct && update_by_fluid(P)) ? kCellBlock : b.nt[2];
 }
 inline int dt_partials(const Batch& b) {
   return (int)flat_blocks(b.tot_v, b.nt[2] < kCellBlock ? b.nt[2] : kCellBlock);

@@ -290,7 +290,7 @@ extern "C" mf_status mf_patch_update_noalloc(mf_ctx* ctx, mf_fab* U, const mf_bo
     NA_CUDA(mf::launch_stage(*cv.dp, p.precision, B, b2, mf::kStageDt, 1.0, ds, parts, &nb, s));
   }
   NA_CUDA(mf::launch_finalize(*cv.dp, parts, b2,
-                              mf::update_cells(*cv.dp, p.precision, b2, whole), ds, 0, s));
+                              mf::update_cells(*cv.dp, b2, whole), ds, 0, s));
   if (F) {
     const void* f2p[3] = {nullptr, nullptr, nullptr};
     const void* f1p[3] = {nullptr, nullptr, nullptr};

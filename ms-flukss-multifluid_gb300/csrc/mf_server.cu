@@ -343,7 +343,7 @@ mf_status enqueue_step(mf_server* S) {
     B.uout = (double*)S->U.p;
     SV_CUDA(mf::launch_stage(P, p.precision, B, S->b2, mf::kStageDt, 1.0, ds, parts, &nb, S->s));
   }
-  SV_CUDA(mf::launch_finalize(P, parts, S->b2, mf::update_cells(P, p.precision, S->b2), ds, 1, S->s));
+  SV_CUDA(mf::launch_finalize(P, parts, S->b2, mf::update_cells(P, S->b2), ds, 1, S->s));
   // neutral pass-through at the sun of every run (NEUTRALS_SUNBC)
   SV_CUDA(mf::launch_sun_copy((double*)S->U.p, (const mf::SunPair*)S->sun.p, S->nsun, P.irhon,
                               P.nf, S->s));

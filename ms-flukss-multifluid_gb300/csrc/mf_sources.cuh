@@ -112,134 +112,210 @@ __device__ __forceinline__ int ce_recipient(int nN, int reg) {
   return (reg >= 1 && reg <= nN) ? reg : 0;
 }
 
-// Arithmetic type of the charge-exchange rates: FP64, or FP32 in the opt-in
-// MF_PREC_MIXED_CE32 mode (the rates scale a source that is a small fraction
-// of the state per step).  The FP64 forms take the reciprocal and logarithm
-// of mf_fp64.cuh (within a few units of 2^-53 of the library's).  The state
-// update itself is FP64 either way.
-__device__ __forceinline__ double ce_rsqrt(double x) { return rsqrt(x); }
-__device__ __forceinline__ float ce_rsqrt(float x) { return rsqrtf(x); }
+// Arithmetic type of the charge-exchange rates and wave speeds: FP64, or FP32
+// (the rates in the opt-in MF_PREC_MIXED_CE32 mode, the wave speeds in every
+// mixed mode; both scale what is a small fraction of the state per step).
+// The FP64 forms take division and square root from the integer pipes
+// (mf_ieee64.cuh) and the logarithm of mf_fp64.cuh.  Products and sums are
+// written as fused operations (mad), or the product by prod() where it must
+// not fuse, so that every kernel that inlines these routines rounds alike.  The state update itself is
+// FP64 either way.
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double prod(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float prod(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double quotient(double a, double b) { return ieee64::div(a, b); }
+__device__ __forceinline__ float quotient(float a, float b) { return a * (1.0f / b); }
+// sqrt(x) and a / sqrt(x) for x > 0
+__device__ __forceinline__ double root_of(double x) { return ieee64::root(x); }
+__device__ __forceinline__ float root_of(float x) { return x * rsqrtf(x); }
+__device__ __forceinline__ double over_root(double a, double x) {
+  return ieee64::div(a, ieee64::root(x));
+}
+__device__ __forceinline__ float over_root(float a, float x) { return a * rsqrtf(x); }
+template <int K>
+__device__ __forceinline__ double pow2(double x) { return ieee64::scale<K>(x); }
+template <int K>
+__device__ __forceinline__ float pow2(float x) {
+  return x * (K < 0 ? 1.0f / (1 << (K < 0 ? -K : 0)) : (float)(1 << (K < 0 ? 0 : K)));
+}
 __device__ __forceinline__ double ce_log(double x) { return fp64::log64(x); }
 __device__ __forceinline__ float ce_log(float x) { return logf(x); }
-__device__ __forceinline__ double ce_rcp(double x) { return fp64::rcp64(x); }
-__device__ __forceinline__ float ce_rcp(float x) { return 1.0f / x; }
 __device__ __forceinline__ double ce_exp(double x) { return exp(x); }
 __device__ __forceinline__ float ce_exp(float x) { return expf(x); }
 __device__ __forceinline__ double ce_pow(double x, double y) { return pow(x, y); }
 __device__ __forceinline__ float ce_pow(float x, float y) { return powf(x, y); }
-// conversions between the FP64 state and the rates' type T (identities for
-// T = double).  The conversion instructions: their integer forms
-// (fp64::d2f / f2d) made the FP32-rate update 10% slower (more registers
-// and branches in a kernel bounded at 128 registers), measured.
+// conversions between the FP64 state and the type T of the rates, off the
+// FP64 pipe (identities for T = double)
 template <typename T>
-__device__ __forceinline__ T to_t(double x) {
-  return static_cast<T>(x);
-}
-__device__ __forceinline__ double to_d(float x) { return static_cast<double>(x); }
+__device__ __forceinline__ T to_t(double x);
+template <> __device__ __forceinline__ double to_t<double>(double x) { return x; }
+template <> __device__ __forceinline__ float to_t<float>(double x) { return fp64::d2f(x); }
+__device__ __forceinline__ double to_d(float x) { return fp64::f2d(x); }
 __device__ __forceinline__ double to_d(double x) { return x; }
 
-// Pauls & Zank charge-exchange rates of one cell; adds S = -dt*H to u
+// Pauls & Zank charge exchange of the plasma with one neutral population
 // (HeliosphericProblem::explicitSource, swlism/HeliosphericProblem.cpp:1394-1539,
 // CHARGE_EXCHANGE_4F swlism/ChargeExchange2F.ChF:673-993 and _MF :995-1149).
-// T is the arithmetic type of the rates (double, or float in the opt-in
-// FP32-rate mode).  The plasma's thermal-speed terms that every neutral
-// population shares are formed once per cell.
-// w: the stage-start primitive state (an array, or a column view that
-// loads each component where it is used).
-// NN > 0: the number of neutral populations fixed at compile time (the
-// loops run a known count, so the populations' independent chains can be
-// scheduled together); 0: P.nf - 1 at run time.
+// T: arithmetic type of the rates.  The products ARR UD, ARR VVTHU and
+// ARR VP_UHM that several terms share are formed once; the plasma's terms
+// that carry a cell factor (ux, U2/2) are summed without it and scaled after
+// the sum: the reference's H in another order.
+template <typename T>
+struct CeTermsT {
+  static constexpr int kShared = 9;
+  // what the plasma sums over the populations: h2..h4, the S of PPLUX..Z,
+  // ARR UD (-DENPLU), G (in the energy source and the recipient's energy
+  // gain) and the rest of h5
+  T shared[kShared];
+  T own[4];  // PMIX, PMIY, PMIZ, ENMI
+};
+using CeTerms = CeTermsT<double>;
+
+// w: the stage-start primitive state; o: the population's first component
+template <typename T, typename WA>
+__device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const WA& w, int o,
+                                                      CeTermsT<T>& c) {
+  constexpr T c4p = T(4.0 * kInvPi), c16p = T(16.0 * kInvPi), c94pi = T(2.25 * kPi);
+  constexpr T c649ip = T(64.0 / 9.0 * kInvPi);
+  const T rho = to_t<T>(w[0]), ux = to_t<T>(w[1]), uy = to_t<T>(w[2]), uz = to_t<T>(w[3]);
+  const T rhoN = to_t<T>(w[o]), uxN = to_t<T>(w[o + 1]), uyN = to_t<T>(w[o + 2]), uzN = to_t<T>(w[o + 3]);
+  const T VVTP = quotient(to_t<T>(w[4]), rho);
+  const T VVTH = quotient(pow2<1>(to_t<T>(w[o + 4])), rhoN);
+  const T dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
+  const T hU2 = pow2<-1>(mad(uz, uz, mad(uy, uy, ux * ux)));
+  const T hUH2 = pow2<-1>(mad(uzN, uzN, mad(uyN, uyN, uxN * uxN)));
+  const T DU2 = mad(dz_, dz_, mad(dy_, dy_, dx_ * dx_)), DU24 = pow2<2>(DU2);
+  const T VPHH = mad(dz_, uzN, mad(dy_, uyN, dx_ * uxN));
+  const T VPHP = mad(dz_, uz, mad(dy_, uy, dx_ * ux));
+  // thermal + relative speeds; every radicand is > 0
+  const T UD = root_of(mad(c4p, VVTH, mad(c4p, VVTP, DU2)));
+  const T VVTHU = over_root(VVTH, mad(c94pi, VVTH, mad(c16p, VVTP, DU24)));
+  const T VP_UHM = over_root(VVTP, mad(c16p, VVTH, mad(c94pi, VVTP, DU24)));
+  const T UPE = root_of(mad(c649ip, VVTH, mad(c4p, VVTP, DU2)));
+  const T UHE = root_of(mad(c4p, VVTH, mad(c649ip, VVTP, DU2)));
+  const T UDS = to_t<T>(P.ce_scale_vel) * UD;
+  const T t = mad(-to_t<T>(P.ce_b), ce_log(UDS), to_t<T>(P.ce_a));
+  T SIG = t * t;
+  const T damp_c = to_t<T>(P.ce_damp_c);
+  if (damp_c > T(0)) SIG = SIG * ce_pow(T(1) - ce_exp(-damp_c / UDS), to_t<T>(P.ce_damp_pow));
+  const T ARR = SIG * (rhoN * (to_t<T>(P.ce_sigma_scale) * rho));
+  const T aU = prod(ARR, UD), aT = prod(ARR, VVTHU), aV = prod(ARR, VP_UHM);
+  const T Y = T(0.75) * ((ARR * UPE) * VVTH);
+  const T hv = aU + aT + aV;
+  c.shared[0] = prod(hv, dx_);
+  c.shared[1] = prod(hv, dy_);
+  c.shared[2] = prod(hv, dz_);
+  c.shared[3] = prod(aV, dx_);
+  c.shared[4] = prod(aV, dy_);
+  c.shared[5] = prod(aV, dz_);
+  c.shared[6] = aU;
+  c.shared[7] = mad(aV, VPHP, (T(0.75) * VVTP) * (ARR * UHE));
+  c.shared[8] = mad(aT, VPHH, mad(aU, hU2 - hUH2, -Y));
+  c.own[0] = mad(uxN, aU, -(dx_ * aT));
+  c.own[1] = mad(uyN, aU, -(dy_ * aT));
+  c.own[2] = mad(uzN, aU, -(dz_ * aT));
+  c.own[3] = mad(hUH2, aU, mad(-VPHH, aT, Y));
+}
+
+// S = -dt H of the plasma (momentum and energy; the magnetic field's and
+// psi's S is zero) from the sums over the populations, sum[q] of shared[q].
+template <typename T>
+__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const T* sum) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q) u[1 + q] = fma(-dt, to_d(sum[q]), u[1 + q]);
+  u[4] = fma(-dt, to_d(sum[7] + sum[8]), u[4]);
+}
+
+// S = -dt H of a population's own loss and gain
+template <typename T>
+__device__ __forceinline__ void charge_exchange_own(const CeTermsT<T>& c, double dt, double* un) {
+  un[0] = fma(-dt, to_d(c.shared[6]), un[0]);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) un[1 + q] = fma(-dt, to_d(c.own[q]), un[1 + q]);
+}
+
+// The newly created neutrals that the recipient gains (its own loss, already
+// applied, cancels): from the sums; w: the plasma's primitive state.
+template <typename T, typename WA>
+__device__ __forceinline__ void charge_exchange_gain(const WA& w, const T* sum, double dt,
+                                                     double* un) {
+  const T ux = to_t<T>(w[1]), uy = to_t<T>(w[2]), uz = to_t<T>(w[3]), D = sum[6];
+  const T hU2 = pow2<-1>(mad(uz, uz, mad(uy, uy, ux * ux)));
+  un[0] = fma(dt, to_d(D), un[0]);
+  un[1] = fma(dt, to_d(mad(ux, D, sum[3])), un[1]);
+  un[2] = fma(dt, to_d(mad(uy, D, sum[4])), un[2]);
+  un[3] = fma(dt, to_d(mad(uz, D, sum[5])), un[3]);
+  un[4] = fma(dt, to_d(mad(hU2, D, sum[7])), un[4]);
+}
+
+// The same for a thread per fluid; at(f, q): shared[q] of population f (from 0)
+template <int NN, typename T, typename AT>
+__device__ __forceinline__ void charge_exchange_sums(T* sum, const AT& at) {
+#pragma unroll
+  for (int q = 0; q < CeTermsT<T>::kShared; ++q) {
+    sum[q] = at(0, q);
+#pragma unroll
+    for (int f = 1; f < NN; ++f) sum[q] = sum[q] + at(f, q);
+  }
+}
+template <int NN, typename T, typename AT>
+__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at) {
+  T sum[CeTermsT<T>::kShared];
+  charge_exchange_sums<NN>(sum, at);
+  charge_exchange_plasma(dt, u, sum);
+}
+template <int NN, typename T, typename WA, typename AT>
+__device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const WA& w,
+                                                        const CeTermsT<T>& c, double dt,
+                                                        double* un, const AT& at) {
+  charge_exchange_own(c, dt, un);
+  if (!rec) return;
+  T sum[CeTermsT<T>::kShared];
+  charge_exchange_sums<NN>(sum, at);
+  charge_exchange_gain(w, sum, dt, un);
+}
+
+// All populations of one cell by one thread.  w: the stage-start primitive
+// state (an array, or a column view that loads each component where it is
+// used).  NN > 0: the number of populations fixed at compile time (their
+// independent chains can be scheduled together); 0: P.nf - 1 at run time.
 template <int IRHON, typename T = double, typename WA = const double*, int NN = 0>
 __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA& w, int reg,
                                                     double dt, double* u) {
   const int nN = NN > 0 ? NN : P.nf - 1;
-  constexpr T c4p = T(4.0 * kInvPi), c16p = T(16.0 * kInvPi), c94pi = T(2.25 * kPi);
-  constexpr T c4ip = T(4.0 * kInvPi), c649ip = T(64.0 / 9.0 * kInvPi);
-  const T rho = to_t<T>(w[0]), ux = to_t<T>(w[1]), uy = to_t<T>(w[2]), uz = to_t<T>(w[3]);
-  const T U2 = ux * ux + uy * uy + uz * uz, hU2 = T(0.5) * U2;
-  const T VVTP = to_t<T>(w[4]) * ce_rcp(rho);
-  // plasma thermal-speed terms of the five speed arguments
-  const T aUDp = c4p * VVTP, aUPMp = c16p * VVTP, aUHMp = c94pi * VVTP;
-  const T aPEp = c4ip * VVTP, aHEp = c649ip * VVTP, q75VP = T(0.75) * VVTP;
-  const T scale_vel = to_t<T>(P.ce_scale_vel), ce_a = to_t<T>(P.ce_a), ce_b = to_t<T>(P.ce_b);
-  const T damp_c = to_t<T>(P.ce_damp_c), damp_pow = to_t<T>(P.ce_damp_pow);
-  const T srho = to_t<T>(P.ce_sigma_scale) * rho;
-  // Each population's own loss / gain is applied inside the loop; the
-  // recipient of the newly created neutrals (region-dependent) then also
-  // receives the plasma's totals.  The products ARR*UD, ARR*VVTHU and
-  // ARR*VP_UHM that several terms share are formed once, and the plasma's
-  // terms that carry a cell factor (ux, U2/2, 3 VVTP/4) are summed without it
-  // and scaled after the loop: the reference's H, summed in another order.
-  // G: the sum of ARR (VPHP VP_UHM + 3 VVTP UHE / 4), which both the energy
-  // source and the recipient's energy gain hold; H5: the rest of h5.
-  T h2 = 0, h3 = 0, h4 = 0, DSUM = 0, S1x = 0, S1y = 0, S1z = 0, G = 0, H5 = 0;
+  T sum[CeTermsT<T>::kShared];
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f > nN) break;
-    const int o = IRHON + (f - 1) * 5;
-    const T rhoN = to_t<T>(w[o]), uxN = to_t<T>(w[o + 1]), uyN = to_t<T>(w[o + 2]), uzN = to_t<T>(w[o + 3]);
-    const T dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
-    const T UH2 = uxN * uxN + uyN * uyN + uzN * uzN;
-    const T DU2 = dx_ * dx_ + dy_ * dy_ + dz_ * dz_, DU2x4 = T(4) * DU2;
-    const T VPHH = dx_ * uxN + dy_ * uyN + dz_ * uzN;
-    const T VPHP = dx_ * ux + dy_ * uy + dz_ * uz;
-    const T VVTH = T(2) * (to_t<T>(w[o + 4]) * ce_rcp(rhoN));
-    // thermal + relative speeds; every argument is > 0, so sqrt(a) = a*rsqrt(a)
-    const T aUD = (aUDp + c4p * VVTH) + DU2;
-    const T UD = aUD * ce_rsqrt(aUD);
-    const T iUPM = ce_rsqrt((aUPMp + c94pi * VVTH) + DU2x4);
-    const T iUHM = ce_rsqrt((aUHMp + c16p * VVTH) + DU2x4);
-    const T aPE = (aPEp + c649ip * VVTH) + DU2;
-    const T UPE = aPE * ce_rsqrt(aPE);
-    const T aHE = (aHEp + c4ip * VVTH) + DU2;
-    const T UHE = aHE * ce_rsqrt(aHE);
-    const T UDS = scale_vel * UD;
-    const T t = ce_a - ce_b * ce_log(UDS);
-    T SIG = t * t;
-    if (damp_c > T(0)) SIG = SIG * ce_pow(T(1) - ce_exp(-damp_c / UDS), damp_pow);
-    const T ARR = SIG * (rhoN * srho);
-    const T aU = ARR * UD;                  // -DENPLU
-    const T aT = ARR * (VVTH * iUPM);       // ARR*VVTHU
-    const T aV = ARR * (VVTP * iUHM);       // ARR*VP_UHM
-    const T Y = (ARR * UPE) * VVTH;
-    const T hv = aU + aT + aV;
-    h2 = h2 + hv * dx_;
-    h3 = h3 + hv * dy_;
-    h4 = h4 + hv * dz_;
-    S1x = S1x + aV * dx_;
-    S1y = S1y + aV * dy_;
-    S1z = S1z + aV * dz_;
-    DSUM = DSUM - aU;
-    G = G + aV * VPHP + q75VP * (ARR * UHE);
-    H5 = H5 + aT * VPHH + aU * (hU2 - T(0.5) * UH2) - T(0.75) * Y;
-    double* un = u + IRHON + (f - 1) * 5;
-    un[0] = un[0] - dt * to_d(aU);
-    un[1] = un[1] - dt * to_d(uxN * aU - dx_ * aT);
-    un[2] = un[2] - dt * to_d(uyN * aU - dy_ * aT);
-    un[3] = un[3] - dt * to_d(uzN * aU - dz_ * aT);
-    un[4] = un[4] - dt * to_d((T(0.5) * UH2) * aU - VPHH * aT + T(0.75) * Y);
+  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f) {
+    if (f < nN) {
+      CeTermsT<T> c;
+      charge_exchange_terms<T>(P, w, IRHON + f * 5, c);
+      charge_exchange_own(c, dt, u + IRHON + f * 5);
+#pragma unroll
+      for (int q = 0; q < CeTermsT<T>::kShared; ++q)
+        sum[q] = (f == 0) ? c.shared[q] : sum[q] + c.shared[q];
+    }
   }
-  const T h5 = G + H5;
-  const T PPLUX = ux * DSUM - S1x, PPLUY = uy * DSUM - S1y, PPLUZ = uz * DSUM - S1z;
-  const T ENPLU = hU2 * DSUM - G;
-  u[1] = u[1] - dt * to_d(h2);
-  u[2] = u[2] - dt * to_d(h3);
-  u[3] = u[3] - dt * to_d(h4);
-  u[4] = u[4] - dt * to_d(h5);
-  // S of the magnetic field (and of psi) is zero; the recipient gets the
-  // other populations' lost density (DSUM less its own, already applied)
+  charge_exchange_plasma(dt, u, sum);
   const int rk = ce_recipient(nN, reg);
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f > nN) break;
-    const bool rec = (f == rk);
-    double* un = u + IRHON + (f - 1) * 5;
-    un[0] = rec ? un[0] - dt * to_d(DSUM) : un[0];
-    un[1] = rec ? un[1] - dt * to_d(PPLUX) : un[1];
-    un[2] = rec ? un[2] - dt * to_d(PPLUY) : un[2];
-    un[3] = rec ? un[3] - dt * to_d(PPLUZ) : un[3];
-    un[4] = rec ? un[4] - dt * to_d(ENPLU) : un[4];
-  }
+  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
+    if (f < nN && f + 1 == rk) charge_exchange_gain(w, sum, dt, u + IRHON + f * 5);
+}
+
+// SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES
+template <typename WA>
+__device__ __forceinline__ void source_8wave(const WA& w, double divB, double dtbydx, double* u) {
+  const double dB = -divB * dtbydx;
+  const double Ux = w[1], Uy = w[2], Uz = w[3];
+  const double Bx = kInv4Pi * w[5], By = kInv4Pi * w[6], Bz = kInv4Pi * w[7];
+  u[1] = mad(dB, Bx, u[1]);
+  u[2] = mad(dB, By, u[2]);
+  u[3] = mad(dB, Bz, u[3]);
+  u[4] = mad(dB, mad(Bz, Uz, mad(By, Uy, Bx * Ux)), u[4]);
+  u[5] = mad(dB, Ux, u[5]);
+  u[6] = mad(dB, Uy, u[6]);
+  u[7] = mad(dB, Uz, u[7]);
 }
 
 // HELIOREINIT_DEFAULT (swlism/HeliosphericPlasmaBCF.ChF:1435-1566): the
@@ -299,8 +375,8 @@ static __device__ __host__ __forceinline__ void reinit_state(const ReinitIn P, d
 
 // The reset of one cell: the membership test in non-fused arithmetic (host
 // and device agree exactly), then the wind state.
-__device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double dx, int i, int j, int k,
-                                            double t, double* u) {
+__device__ __host__ __forceinline__ bool reinit_wind(const DevParams& P, double dx, int i, int j,
+                                                     int k, double t, ReinitState& o) {
 #ifdef __CUDA_ARCH__
   const double x = __dadd_rn(__dmul_rn(i + 0.5, dx), -P.sun_c[0]);
   const double y = __dadd_rn(__dmul_rn(j + 0.5, dx), -P.sun_c[1]);
@@ -308,16 +384,22 @@ __device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double 
   const double r2 = (P.sd == 3)
                         ? __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z))
                         : __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
-  if (!(r2 <= __dmul_rn(P.r0, P.r0))) return;
+  if (!(r2 <= __dmul_rn(P.r0, P.r0))) return false;
 #else
   const double x = (i + 0.5) * dx - P.sun_c[0];
   const double y = (j + 0.5) * dx - P.sun_c[1];
   const double z = (P.sd == 3) ? (k + 0.5) * dx - P.sun_c[2] : 0.0;
   const double r2 = (P.sd == 3) ? (x * x + y * y + z * z) : (x * x + y * y);
-  if (!(r2 <= P.r0 * P.r0)) return;
+  if (!(r2 <= P.r0 * P.r0)) return false;
 #endif
-  ReinitState o;
   reinit_state(reinit_in(P), x, y, z, r2, t, o);
+  return true;
+}
+
+__device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double dx, int i, int j, int k,
+                                            double t, double* u) {
+  ReinitState o;
+  if (!reinit_wind(P, dx, i, j, k, t, o)) return;
 #pragma unroll
   for (int q = 0; q < 8; ++q) u[q] = o.u[q];
   if (!P.monopolar) {
@@ -329,69 +411,70 @@ __device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double 
   }
 }
 
+// The plasma alone (no tracking surfaces).
+__device__ __forceinline__ void reinit_plasma(const DevParams& P, double dx, int i, int j, int k,
+                                              double t, double* u) {
+  ReinitState o;
+  if (!reinit_wind(P, dx, i, j, k, t, o)) return;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) u[q] = o.u[q];
+}
+
 // POSTPROCESSING (srcIdeal/PatchIdealMHDF.ChF:1019-1070) and POSTPROCESSING_MF
 // (srcIdeal/PatchMHDMFF.ChF:301-511).
-template <int IRHON>
-__device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
+__device__ __forceinline__ void positivity_plasma(const DevParams& P, double* u) {
+  using namespace ieee64;
   const double hg = P.hgamma, ihg = P.invhgamma, smallR = P.smallr, smallP = P.smallp;
-  if (P.nf == 1) {
-    double Rho = u[0];
-    bool was = false;
-    if (Rho < smallR) { Rho = smallR; was = true; }
-    const double invRho = fp64::rcp64(Rho);
-    const double Ux = u[1] * invRho, Uy = u[2] * invRho, Uz = u[3] * invRho;
-    const double BxB = kInv8Pi * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]);
-    const double UxU = 0.5 * (Ux * Ux + Uy * Uy + Uz * Uz);
-    double Pr = hg * (u[4] - BxB - Rho * UxU);
-    if (Pr < smallP) { Pr = smallP; was = true; }
-    if (was) {
-      u[0] = Rho;
-      u[4] = Pr * ihg + Rho * UxU + BxB;
-    }
-    return;
-  }
-  {
-    const double Rho0 = u[0];
-    const double invRho = fp64::rcp64(Rho0);
-    const double Ux = u[1] * invRho, Uy = u[2] * invRho, Uz = u[3] * invRho;
-    const double BxB = kInv8Pi * (u[5] * u[5] + u[6] * u[6] + u[7] * u[7]);
-    const double UxU = 0.5 * (Ux * Ux + Uy * Uy + Uz * Uz);
-    double Pr = hg * (u[4] - BxB - Rho0 * UxU);
-    double Rho = Rho0;
-    bool was = false;
-    if (Rho < smallR) { Rho = smallR; was = true; }
-    if (Pr < smallP) { Pr = smallP; was = true; }
-    if (was) {
-      u[0] = Rho;
+  double Rho = u[0];
+  bool was = lt(Rho, smallR);
+  if (P.nf == 1 && was) Rho = smallR;  // one fluid: the velocities of the floored density
+  const double invRho = div(1.0, Rho);
+  const double Ux = u[1] * invRho, Uy = u[2] * invRho, Uz = u[3] * invRho;
+  const double BxB = prod(kInv8Pi, mad(u[7], u[7], mad(u[6], u[6], u[5] * u[5])));
+  const double UxU = half(mad(Uz, Uz, mad(Uy, Uy, Ux * Ux)));
+  double Pr = hg * mad(-Rho, UxU, u[4] - BxB);
+  if (was) Rho = smallR;
+  if (lt(Pr, smallP)) { Pr = smallP; was = true; }
+  if (was) {
+    u[0] = Rho;
+    if (P.nf > 1) {
       u[1] = Rho * Ux;
       u[2] = Rho * Uy;
       u[3] = Rho * Uz;
-      u[4] = Pr * ihg + Rho * UxU + BxB;
     }
+    u[4] = mad(Pr, ihg, mad(Rho, UxU, BxB));
   }
+}
+
+// neutral fluid f (from 1)
+__device__ __forceinline__ void positivity_neutral(const DevParams& P, int f, double* un) {
+  using namespace ieee64;
+  const double hg = P.hgamma, ihg = P.invhgamma;
+  const double fd = (f == 1) ? P.smallr : (f == 3) ? kNet3Dens : kNet2Dens;
+  const double fp = (f == 1) ? P.smallp : (f == 3) ? kNet3Pres : kNet2Pres;
+  double Rho = un[0];
+  const double invRho = div(1.0, Rho);
+  const double Ux = un[1] * invRho, Uy = un[2] * invRho, Uz = un[3] * invRho;
+  const double UxU = half(mad(Uz, Uz, mad(Uy, Uy, Ux * Ux)));
+  double Pr = hg * mad(-Rho, UxU, un[4]);
+  bool was = false;
+  if (lt(Rho, fd)) { Rho = fd; was = true; }
+  if (lt(Pr, fp)) { Pr = fp; was = true; }
+  if (was) {
+    un[0] = Rho;
+    un[1] = Rho * Ux;
+    un[2] = Rho * Uy;
+    un[3] = Rho * Uz;
+    un[4] = mad(Pr, ihg, Rho * UxU);
+  }
+}
+
+template <int IRHON>
+__device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
+  positivity_plasma(P, u);
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f >= P.nf) break;
-    const double fd = (f == 1) ? smallR : (f == 3) ? kNet3Dens : kNet2Dens;
-    const double fp = (f == 1) ? smallP : (f == 3) ? kNet3Pres : kNet2Pres;
-    double* un = u + IRHON + (f - 1) * 5;
-    const double Rho0 = un[0];
-    const double invRho = fp64::rcp64(Rho0);
-    const double Ux = un[1] * invRho, Uy = un[2] * invRho, Uz = un[3] * invRho;
-    const double UxU = 0.5 * (Ux * Ux + Uy * Uy + Uz * Uz);
-    double Pr = hg * (un[4] - Rho0 * UxU);
-    double Rho = Rho0;
-    bool was = false;
-    if (Rho < fd) { Rho = fd; was = true; }
-    if (Pr < fp) { Pr = fp; was = true; }
-    if (was) {
-      un[0] = Rho;
-      un[1] = Rho * Ux;
-      un[2] = Rho * Uy;
-      un[3] = Rho * Uz;
-      un[4] = Pr * ihg + Rho * UxU;
-    }
-  }
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f)
+    if (f < P.nf) positivity_neutral(P, f, u + IRHON + (f - 1) * 5);
 }
 
 // MAXWAVESPEED (srcIdeal/PatchIdealMHDF.ChF:5-63) + MAXWAVESPEED_E
@@ -399,46 +482,53 @@ __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
 // from the total energy in FP64 (E minus kinetic minus magnetic cancels in
 // cold, low-beta flow); the speeds are formed in T (FP64, or FP32 in the
 // mixed precision modes, whose time step then carries FP32 rounding).
-__device__ __forceinline__ double ws_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double ws_sqrt(double x) { return ieee64::root(x); }
 __device__ __forceinline__ float ws_sqrt(float x) { return sqrtf(x); }
+__device__ __forceinline__ double ws_max(double a, double b) { return ieee64::maxnum(a, b); }
+__device__ __forceinline__ float ws_max(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double ws_abs(double a) { return ieee64::absval(a); }
+__device__ __forceinline__ float ws_abs(float a) { return fabsf(a); }
+
+template <typename T = double>
+__device__ __forceinline__ T wave_speed_plasma(const DevParams& P, const double* u) {
+  const T i4pi = T(kInv4Pi), gam = to_t<T>(P.gamma);
+  const double rinv = ieee64::div(1.0, u[0]);
+  const double m1 = u[1], m2 = u[2], m3 = u[3], bx = u[5], by = u[6], bz = u[7];
+  const double ke = prod(mad(m3, m3, mad(m2, m2, m1 * m1)), rinv);
+  const double bb = prod(kInv4Pi, mad(bz, bz, mad(by, by, bx * bx)));
+  const double p = ieee64::maxnum(P.hgamma * mad(-0.5, ke + bb, u[4]), P.smallp);
+  const T invrho = to_t<T>(rinv), b = to_t<T>(bb);
+  const T uu = to_t<T>(m1) * invrho, vv = to_t<T>(m2) * invrho, ww = to_t<T>(m3) * invrho;
+  const T bxt = to_t<T>(bx), byt = to_t<T>(by), bzt = to_t<T>(bz);
+  const T a2 = gam * to_t<T>(p) * invrho;
+  const T as2 = pow2<-1>(mad(invrho, b, a2));
+  const T as4 = as2 * as2;
+  const T k4 = i4pi * invrho * a2;
+  // as4 - k4 b^2 >= 0 exactly; contracted rounding can push it below 0
+  T umax = ws_abs(uu) + ws_sqrt(as2 + ws_sqrt(ws_max(T(0), mad(-(k4 * bxt), bxt, as4))));
+  umax = ws_max(ws_abs(vv) + ws_sqrt(as2 + ws_sqrt(ws_max(T(0), mad(-(k4 * byt), byt, as4)))), umax);
+  return ws_max(ws_abs(ww) + ws_sqrt(as2 + ws_sqrt(ws_max(T(0), mad(-(k4 * bzt), bzt, as4)))), umax);
+}
+
+template <typename T = double>
+__device__ __forceinline__ T wave_speed_neutral(const DevParams& P, const double* un) {
+  const T gam = to_t<T>(P.gamma);
+  const double rinv = ieee64::div(1.0, ieee64::maxnum(un[0], P.smallr));
+  const double m1 = un[1], m2 = un[2], m3 = un[3];
+  const double ke = prod(mad(m3, m3, mad(m2, m2, m1 * m1)), rinv);
+  const double p = ieee64::maxnum(P.hgamma * mad(-0.5, ke, un[4]), P.smallp);
+  const T invrho = to_t<T>(rinv);
+  const T uu = to_t<T>(m1) * invrho, vv = to_t<T>(m2) * invrho, ww = to_t<T>(m3) * invrho;
+  const T a = ws_sqrt(gam * to_t<T>(p) * invrho);
+  return ws_max(ws_max(ws_abs(uu), ws_abs(vv)), ws_abs(ww)) + a;
+}
 
 template <int IRHON, typename T = double>
 __device__ __forceinline__ double max_wave_speed(const DevParams& P, const double* u) {
-  const T i4pi = T(kInv4Pi), gam = to_t<T>(P.gamma);
-  T cmax = 0;
-  {
-    const double rinv = fp64::rcp64(u[0]);
-    const double m1 = u[1], m2 = u[2], m3 = u[3], bx = u[5], by = u[6], bz = u[7];
-    const double ke = (m1 * m1 + m2 * m2 + m3 * m3) * rinv;
-    const double bb = kInv4Pi * (bx * bx + by * by + bz * bz);
-    const double p = fmax(P.hgamma * (u[4] - 0.5 * (ke + bb)), P.smallp);
-    const T invrho = to_t<T>(rinv), b = to_t<T>(bb);
-    const T uu = to_t<T>(m1) * invrho, vv = to_t<T>(m2) * invrho, ww = to_t<T>(m3) * invrho;
-    const T bxt = to_t<T>(bx), byt = to_t<T>(by), bzt = to_t<T>(bz);
-    const T a2 = gam * to_t<T>(p) * invrho;
-    const T as2 = T(0.5) * (a2 + invrho * b);
-    const T as4 = as2 * as2;
-    const T k4 = i4pi * invrho * a2;
-    // as4 - k4 b^2 >= 0 exactly; contracted rounding can push it below 0
-    T umax = fabs(uu) + ws_sqrt(as2 + ws_sqrt(fmax(T(0), as4 - k4 * bxt * bxt)));
-    umax = fmax(fabs(vv) + ws_sqrt(as2 + ws_sqrt(fmax(T(0), as4 - k4 * byt * byt))), umax);
-    umax = fmax(fabs(ww) + ws_sqrt(as2 + ws_sqrt(fmax(T(0), as4 - k4 * bzt * bzt))), umax);
-    cmax = fmax(umax, cmax);
-  }
+  T cmax = ws_max(wave_speed_plasma<T>(P, u), T(0));
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f >= P.nf) break;
-    const double* un = u + IRHON + (f - 1) * 5;
-    const double rinv = fp64::rcp64(fmax(un[0], P.smallr));
-    const double m1 = un[1], m2 = un[2], m3 = un[3];
-    const double ke = (m1 * m1 + m2 * m2 + m3 * m3) * rinv;
-    const double p = fmax(P.hgamma * (un[4] - 0.5 * ke), P.smallp);
-    const T invrho = to_t<T>(rinv);
-    const T uu = to_t<T>(m1) * invrho, vv = to_t<T>(m2) * invrho, ww = to_t<T>(m3) * invrho;
-    const T a = ws_sqrt(gam * to_t<T>(p) * invrho);
-    const T umax = fmax(fmax(fabs(uu), fabs(vv)), fabs(ww)) + a;
-    cmax = fmax(umax, cmax);
-  }
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f)
+    if (f < P.nf) cmax = ws_max(wave_speed_neutral<T>(P, u + IRHON + (f - 1) * 5), cmax);
   return to_d(cmax);
 }
 

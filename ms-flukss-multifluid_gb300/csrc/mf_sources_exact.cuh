@@ -113,10 +113,12 @@ struct CeTerms {
   double shared[kShared];
   double pmi[3], enmi;  // PMIX, PMIY, PMIZ, ENMI
 };
+template <typename T>
+using CeTermsT = CeTerms;
 
 // w: the stage-start primitive state; o: the population's first component.
 // Factors that are powers of two scale exactly and move out of the products.
-template <typename WA>
+template <typename T = double, typename WA>
 __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const WA& w, int o,
                                                       CeTerms& c) {
   using namespace ieee64;
@@ -163,7 +165,7 @@ __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const 
 // S = -dt H of the plasma (momentum and energy; the magnetic field's and
 // psi's S is zero).  at(f, q): CeTerms::shared[q] of population f (from 0);
 // NN populations, or nN at run time with NN = 0.
-template <int NN, typename AT>
+template <int NN, typename T = double, typename AT>
 __device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at,
                                                        int nN = NN) {
 #pragma unroll
@@ -178,10 +180,10 @@ __device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, con
 
 // S = -dt H of population f (from 0) with terms c; rec: it receives the
 // newly created neutrals.
-template <int NN, typename AT>
-__device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const CeTerms& c,
-                                                        double dt, double* un, const AT& at,
-                                                        int nN_ = NN) {
+template <int NN, typename T = double, typename WA, typename AT>
+__device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const WA&,
+                                                        const CeTerms& c, double dt, double* un,
+                                                        const AT& at, int nN_ = NN) {
   const int nN = NN > 0 ? NN : nN_;
   double H1 = c.shared[4], H2 = c.pmi[0], H3 = c.pmi[1], H4 = c.pmi[2], H5 = c.enmi;
   if (rec) {
@@ -230,7 +232,22 @@ __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA
   const int rk = ce_recipient(nN, reg);
 #pragma unroll
   for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
-    if (f < nN) charge_exchange_neutral<NN>(f + 1 == rk, f, c[f], dt, u + IRHON + f * 5, at, nN);
+    if (f < nN) charge_exchange_neutral<NN>(f + 1 == rk, f, w, c[f], dt, u + IRHON + f * 5, at, nN);
+}
+
+// SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES
+template <typename WA>
+__device__ __forceinline__ void source_8wave(const WA& w, double divB, double dtbydx, double* u) {
+  const double dB = -divB * dtbydx;
+  const double Ux = w[1], Uy = w[2], Uz = w[3];
+  const double Bx = kInv4Pi * w[5], By = kInv4Pi * w[6], Bz = kInv4Pi * w[7];
+  u[1] = u[1] + dB * Bx;
+  u[2] = u[2] + dB * By;
+  u[3] = u[3] + dB * Bz;
+  u[4] = u[4] + dB * (Bx * Ux + By * Uy + Bz * Uz);
+  u[5] = u[5] + dB * Ux;
+  u[6] = u[6] + dB * Uy;
+  u[7] = u[7] + dB * Uz;
 }
 
 // HELIOREINIT_DEFAULT (swlism/HeliosphericPlasmaBCF.ChF:1435-1566) at time t
@@ -401,6 +418,7 @@ __device__ __forceinline__ void positivity_cell(const DevParams& P, double* u) {
 
 // MAXWAVESPEED (srcIdeal/PatchIdealMHDF.ChF:5-63) + MAXWAVESPEED_E
 // (srcIdeal/PatchEulerF.ChF:5-50) of one cell.
+template <typename T = double>
 __device__ __forceinline__ double wave_speed_plasma(const DevParams& P, const double* u) {
   using namespace ieee64;
   double rho = u[0];
@@ -423,6 +441,7 @@ __device__ __forceinline__ double wave_speed_plasma(const DevParams& P, const do
   return maxnum(absval(ww) + root(as2 + root(as4 - a2 * bn2)), umax);
 }
 
+template <typename T = double>
 __device__ __forceinline__ double wave_speed_neutral(const DevParams& P, const double* un) {
   using namespace ieee64;
   double rho = maxnum(un[0], P.smallr);

@@ -11,8 +11,10 @@ cudaError_t launch_update_fast(const DevParams& P, const StageBuffers& B, const 
                                int flags, double dt_scale, StepState* state,
                                DtPartial* partials, int* nblocks_v, cudaStream_t s, int first,
                                int end) {
-  const int nt = b.nt[2];
   if (end < 0) end = b.tot_v;
+  if (!B.by_cell && first == 0 && end == b.tot_v && update_by_fluid(P))
+    return launch_cells_fast<R>(P, B, b, flags, dt_scale, state, partials, nblocks_v, s);
+  const int nt = b.nt[2];
   if (nblocks_v) *nblocks_v = (int)flat_blocks(b.tot_v, nt);
   if (first % nt != 0) return cudaErrorInvalidValue;
   if (end - first <= 0) return cudaSuccess;

@@ -205,7 +205,7 @@ __global__ void k_flux_out(int nc, const R* __restrict__ f2, int l20, int l21, i
 cudaError_t launch_update_exact(const DevParams& P, const StageBuffers& B, const Batch& b,
                                 int flags, double dt_scale, StepState* state,
                                 DtPartial* partials, int* nblocks_v, cudaStream_t s) {
-  if (!B.by_cell && update_by_fluid(P, MF_PREC_FP64))
+  if (!B.by_cell && update_by_fluid(P))
     return launch_cells_exact(P, B, b, flags, dt_scale, state, partials, nblocks_v, s);
   const int nt = b.nt[2];
   const unsigned gv = flat_blocks(b.tot_v, nt);

@@ -173,20 +173,7 @@ __device__ __forceinline__ void update_tail(const DevParams& P, const StageBuffe
       if (q < P.ils) ws.v[q] = B.w[base + q * cs];
   }
   const auto& w = w_arg(ws);
-  if (P.use8) {
-    // SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES
-    const double dtbydx = ieee64::div(dt, RP.dx);
-    const double dB = -divB * dtbydx;
-    const double Ux = w[1], Uy = w[2], Uz = w[3];
-    const double Bx = kInv4Pi * w[5], By = kInv4Pi * w[6], Bz = kInv4Pi * w[7];
-    u[1] = u[1] + dB * Bx;
-    u[2] = u[2] + dB * By;
-    u[3] = u[3] + dB * Bz;
-    u[4] = u[4] + dB * (Bx * Ux + By * Uy + Bz * Uz);
-    u[5] = u[5] + dB * Ux;
-    u[6] = u[6] + dB * Uy;
-    u[7] = u[7] + dB * Uz;
-  }
+  if (P.use8) source_8wave(w, divB, ieee64::div(dt, RP.dx), u);
   if (GLM) u[8] = psi_damp * u[8];  // PSIPARABOLIC (src/DednerF.ChF:65-87)
   if (P.ce && P.nf >= 2) {
     const double regtr = P.reg_tracer ? B.w[base + (P.nc - 1) * cs] : 0.0;
@@ -314,7 +301,7 @@ __device__ __forceinline__ void update_cells(const DevParams& P, const StageBuff
     if constexpr (sizeof(R) == 4) {
 #pragma unroll
       for (int q = 0; q < MF_MAX_COMP; ++q)
-        if (q < P.ils) u[q] = u[q] - dtinv * fp64::f2d(fsum[q]);
+        if (q < P.ils) u[q] = fma(-dtinv, fp64::f2d(fsum[q]), u[q]);
     }
     double divB = 0.0;
     if (P.use8) {
