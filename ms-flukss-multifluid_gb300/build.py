@@ -48,9 +48,9 @@ def _headers() -> list[str]:
 def _compile(src: str, verbose: bool) -> str:
     obj = os.path.join(BUILD_DIR, os.path.basename(src) + ".o")
     cmd = [_nvcc()] + ARCH + NVCC_FLAGS
-    if "_exact" in os.path.basename(src):
-        # no fused multiply-add: every operation rounds as in
-        # the CPU restatement of the reference
+    if "_exact" in os.path.basename(src) or "_fma" in os.path.basename(src):
+        # no contraction: every operation rounds as in the CPU restatement of
+        # the reference, or (_fma) fuses only where the source says so
         cmd += ["-fmad=false"]
     if src.endswith(".cpp"):
         cmd += ["-x", "cu"]

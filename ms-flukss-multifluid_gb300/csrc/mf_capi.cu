@@ -1523,9 +1523,10 @@ static mf_status enqueue_level_step(mf_level* L, int advance, cudaEvent_t* ev = 
     if (ev) {  // prim, faces, predictor, shift, fluxes, update
       const int k0[4] = {1, 1, 3, 1};
       for (int q = 0; q < 4; ++q) kinds[ne + q] = k0[q];
-      for (int d = 0; d < sd; ++d) kinds[ne + 4 + d] = 2;
-      kinds[ne + 4 + sd] = 3;
-      ne += mf::hancock_launches(sd);
+      const int nh = mf::flux_launches(c->dp, p.precision, false);
+      for (int q = 0; q < nh; ++q) kinds[ne + 4 + q] = 2;
+      kinds[ne + 4 + nh] = 3;
+      ne += mf::hancock_launches(c->dp, p.precision);
     }
     if (ct) {  // the corrector's edges from W(t+dt/2), B from W(t)
       if ((gst = ct_stage(L->b2, H.w2, e2, nullptr, nullptr, (double*)L->U.p, nullptr, nullptr,
@@ -1758,7 +1759,7 @@ mf_status mf_level_create(mf_ctx* c, int npatch, const mf_box* valid, mf_level**
   L->fused = false;
   const int per_stage = mf::stage_launches(sd);
   L->launches = (p.time_approximation == MF_TA_RK2) ? (2 * per_stage + 2 + 1)
-                : (p.time_approximation == MF_TA_HANCOCK) ? (mf::hancock_launches(sd) + 1 + 1)
+                : (p.time_approximation == MF_TA_HANCOCK) ? (mf::hancock_launches(c->dp, p.precision) + 1 + 1)
                                                           : (per_stage + 1 + 1);
   if (L->nfull == 0) L->launches -= 1;
   if (p.time_approximation == MF_TA_RK2 && L->ntwo == 0) L->launches -= 1;

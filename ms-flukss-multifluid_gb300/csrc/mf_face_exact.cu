@@ -6,15 +6,15 @@
 
 namespace mf {
 
-cudaError_t launch_plasma_exact(const DevParams& P, const double* w, void* const f[3],
-                              void* const bn[3], const Batch& b, const StepState* state,
-                              cudaStream_t s) {
-  return launch_plasma_t(P, w, f, bn, b, state, s);
+cudaError_t launch_plasma_exact(const DevParams& P, const double* w, const double* const* fv,
+                               void* const f[3], void* const bn[3], const Batch& b,
+                               const StepState* state, cudaStream_t s) {
+  return launch_plasma_t(P, w, fv, f, bn, b, state, s);
 }
 
-cudaError_t launch_neutral_exact(const DevParams& P, const double* w, void* const f[3],
-                               const Batch& b, cudaStream_t s) {
-  return launch_neutral_t(P, w, f, b, s);
+cudaError_t launch_neutral_exact(const DevParams& P, const double* w, const double* const* fv,
+                                void* const f[3], const Batch& b, cudaStream_t s) {
+  return launch_neutral_t(P, w, fv, f, b, s);
 }
 
 }  // namespace mf

@@ -32,9 +32,14 @@ using namespace MF_PHYS;
 constexpr int kPlasmaThreads = 64, kNeutralThreads = 128;
 
 // The faces of a batch in every direction: the launch's blocks cover those of
-// direction 0, then 1, then 2 (nb blocks each).
+// direction 0, then 1, then 2 (nb blocks each).  w: the primitive state whose
+// cells the face states are limited from; fv: the Hancock corrector's face
+// values instead (low, then high face of every component per cell of the
+// slope box, nc components).
 struct FaceBatch {
   const double* w;
+  const double* fv[3];
+  int nc;
   double* f[3];
   double* bn[3];
   int tot[3], nb[3];
@@ -46,11 +51,15 @@ struct Face {
   int dir, pos;          // direction, index along it
   const double* w;       // component 0 of the cell on the face's high side
   long long cs, st;      // component and stencil strides of w
+  const double* fr;      // Hancock: component 0 of the high cell's low-face value
+  const double* fl;      // and of the low cell's high-face value
+  long long scs;         // their component stride
   double* f;             // component 0 of the face's flux
   double* bn;
   long long fcs;         // component stride of f
 };
 
+template <bool HANCOCK>
 __device__ __forceinline__ bool find_face(const FaceBatch& A, const StageDesc* __restrict__ descs,
                                           int ndesc, Face& F) {
   int blk = blockIdx.x, dir = 0;
@@ -81,6 +90,13 @@ __device__ __forceinline__ bool find_face(const FaceBatch& A, const StageDesc* _
   F.f = A.f[dir] + D.f_off[dir] + fo;
   F.bn = A.bn[dir] + D.bn_off[dir] + fo;
   F.fcs = (long long)n[0] * n[1] * n[2];
+  if (HANCOCK) {
+    F.scs = (long long)D.sn[0] * D.sn[1] * D.sn[2];
+    const long long ss = (dir == 0) ? 1 : (dir == 1) ? (long long)D.sn[0]
+                                                     : (long long)D.sn[0] * D.sn[1];
+    F.fr = A.fv[dir] + D.fv_off[dir] + loc(D.slo, D.sn, i, j, k);
+    F.fl = F.fr + A.nc * F.scs - ss;
+  }
   return true;
 }
 
@@ -104,8 +120,14 @@ __device__ __noinline__ Pair limited(int lim, double a, double b, double c) {
 
 // Face states of component c: the high-face value of the low cell (l) and the
 // low-face value of the high cell (r); flat cells keep their own value.
+template <bool HANCOCK>
 __device__ __forceinline__ void face_pair(const Face& F, int c, int lim, bool flatL, bool flatR,
                                           double& l, double& r) {
+  if (HANCOCK) {
+    l = __ldg(F.fl + c * F.scs);
+    r = __ldg(F.fr + c * F.scs);
+    return;
+  }
   const double* __restrict__ w = F.w + c * F.cs;
   const double wa = __ldg(w - 2 * F.st), wb = __ldg(w - F.st), wc = __ldg(w), wd = __ldg(w + F.st);
   if (lim == MF_LIM_MINMOD) {
@@ -135,24 +157,25 @@ __device__ __forceinline__ void flat_cells(const DevParams& P, const Face& F, bo
   }
 }
 
-// Plasma (and psi) fluxes and Bn of every face, the operations of k_flux.
-template <int RS>
+// Plasma (and psi) fluxes and Bn of every face, the operations of k_flux (or,
+// HANCOCK, of k_hflux: the face values were limited before the predictor).
+template <int RS, bool HANCOCK>
 __global__ void __launch_bounds__(kPlasmaThreads, MF_PLASMA_BLOCKS)
     k_plasma(const __grid_constant__ DevParams P, const __grid_constant__ FaceBatch A,
              const StageDesc* __restrict__ descs, int ndesc, const RunParams* __restrict__ runs,
              const StepState* __restrict__ states) {
   Face F;
-  if (!find_face(A, descs, ndesc, F)) return;
-  bool flatL, flatR;
-  flat_cells(P, F, flatL, flatR);
+  if (!find_face<HANCOCK>(A, descs, ndesc, F)) return;
+  bool flatL = false, flatR = false;
+  if (!HANCOCK) flat_cells(P, F, flatL, flatR);
   double wl[9], wr[9], g[9];
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
     const int c = (v == 0 || v == 4) ? v : (v < 4) ? 1 + axis(F.dir, v - 1) : 5 + axis(F.dir, v - 5);
-    face_pair(F, c, P.lim[c], flatL, flatR, wl[v], wr[v]);
+    face_pair<HANCOCK>(F, c, P.lim[c], flatL, flatR, wl[v], wr[v]);
   }
   wl[8] = wr[8] = 0.0;
-  if (P.glm) face_pair(F, 8, MF_LIM_MINMOD, flatL, flatR, wl[8], wr[8]);
+  if (P.glm) face_pair<HANCOCK>(F, 8, MF_LIM_MINMOD, flatL, flatR, wl[8], wr[8]);
   if (RS == kRusanov)
     rusanov_mhd<double, 0>(P, wl, wr, g);
   else if (RS == kVFRoe)
@@ -187,19 +210,20 @@ __global__ void __launch_bounds__(kPlasmaThreads, MF_PLASMA_BLOCKS)
 }
 
 // Van Leer fluxes of one neutral population (blockIdx.y) of every face.
+template <bool HANCOCK>
 __global__ void __launch_bounds__(kNeutralThreads, MF_NEUTRAL_BLOCKS)
     k_neutral(const __grid_constant__ DevParams P, const __grid_constant__ FaceBatch A,
               const StageDesc* __restrict__ descs, int ndesc) {
   Face F;
-  if (!find_face(A, descs, ndesc, F)) return;
-  bool flatL, flatR;
-  flat_cells(P, F, flatL, flatR);
+  if (!find_face<HANCOCK>(A, descs, ndesc, F)) return;
+  bool flatL = false, flatR = false;
+  if (!HANCOCK) flat_cells(P, F, flatL, flatR);
   const int s = P.irhon + (int)blockIdx.y * 5;
   double nl[5], nr[5], g[5];
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     const int c = s + ((v == 0 || v == 4) ? v : 1 + axis(F.dir, v - 1));
-    face_pair(F, c, MF_LIM_MINMOD, flatL, flatR, nl[v], nr[v]);
+    face_pair<HANCOCK>(F, c, MF_LIM_MINMOD, flatL, flatR, nl[v], nr[v]);
   }
   vanleer_euler<double, 0>(P, nl, nr, g);
 #pragma unroll
@@ -209,11 +233,13 @@ __global__ void __launch_bounds__(kNeutralThreads, MF_NEUTRAL_BLOCKS)
   }
 }
 
-inline FaceBatch face_batch(const DevParams& P, const double* w, void* const f[3],
-                            void* const bn[3], const Batch& b, int nt) {
+inline FaceBatch face_batch(const DevParams& P, const double* w, const double* const* fv,
+                            void* const f[3], void* const bn[3], const Batch& b, int nt) {
   FaceBatch A;
   A.w = w;
+  A.nc = P.nc;
   for (int d = 0; d < 3; ++d) {
+    A.fv[d] = fv ? fv[d] : nullptr;
     A.f[d] = (double*)f[d];
     A.bn[d] = (double*)bn[d];
     A.tot[d] = d < P.sd ? b.tot_f[d] : 0;
@@ -222,30 +248,39 @@ inline FaceBatch face_batch(const DevParams& P, const double* w, void* const f[3
   return A;
 }
 
-inline cudaError_t launch_plasma_t(const DevParams& P, const double* w, void* const f[3],
-                                   void* const bn[3], const Batch& b, const StepState* state,
-                                   cudaStream_t s) {
-  const FaceBatch A = face_batch(P, w, f, bn, b, kPlasmaThreads);
+template <bool HANCOCK>
+cudaError_t launch_plasma_t(const DevParams& P, const FaceBatch& A, const Batch& b,
+                            const StepState* state, cudaStream_t s) {
   const int nb = A.nb[0] + A.nb[1] + A.nb[2];
   if (nb <= 0) return cudaSuccess;
-  if (P.rs == kRusanov)
-    k_plasma<kRusanov><<<nb, kPlasmaThreads, 0, s>>>(P, A, b.desc, b.ndesc, b.runs, state);
-  else if (P.rs == kVFRoe)
-    k_plasma<kVFRoe><<<nb, kPlasmaThreads, 0, s>>>(P, A, b.desc, b.ndesc, b.runs, state);
-  else if (P.rs == kRoe8)
-    k_plasma<kRoe8><<<nb, kPlasmaThreads, 0, s>>>(P, A, b.desc, b.ndesc, b.runs, state);
-  else
-    k_plasma<kRoe7><<<nb, kPlasmaThreads, 0, s>>>(P, A, b.desc, b.ndesc, b.runs, state);
+#define MF_PLASMA(RS) \
+  k_plasma<RS, HANCOCK><<<nb, kPlasmaThreads, 0, s>>>(P, A, b.desc, b.ndesc, b.runs, state)
+  if (P.rs == kRusanov) MF_PLASMA(kRusanov);
+  else if (P.rs == kVFRoe) MF_PLASMA(kVFRoe);
+  else if (P.rs == kRoe8) MF_PLASMA(kRoe8);
+  else MF_PLASMA(kRoe7);
+#undef MF_PLASMA
   return cudaGetLastError();
 }
 
-inline cudaError_t launch_neutral_t(const DevParams& P, const double* w, void* const f[3],
-                                    const Batch& b, cudaStream_t s) {
+inline cudaError_t launch_plasma_t(const DevParams& P, const double* w, const double* const* fv,
+                                   void* const f[3], void* const bn[3], const Batch& b,
+                                   const StepState* state, cudaStream_t s) {
+  const FaceBatch A = face_batch(P, w, fv, f, bn, b, kPlasmaThreads);
+  return fv ? launch_plasma_t<true>(P, A, b, state, s) : launch_plasma_t<false>(P, A, b, state, s);
+}
+
+inline cudaError_t launch_neutral_t(const DevParams& P, const double* w, const double* const* fv,
+                                    void* const f[3], const Batch& b, cudaStream_t s) {
   void* const none[3] = {nullptr, nullptr, nullptr};
-  const FaceBatch A = face_batch(P, w, f, none, b, kNeutralThreads);
+  const FaceBatch A = face_batch(P, w, fv, f, none, b, kNeutralThreads);
   const int nb = A.nb[0] + A.nb[1] + A.nb[2];
   if (nb <= 0 || P.nf < 2) return cudaSuccess;
-  k_neutral<<<dim3(nb, P.nf - 1), kNeutralThreads, 0, s>>>(P, A, b.desc, b.ndesc);
+  const dim3 grid(nb, P.nf - 1);
+  if (fv)
+    k_neutral<true><<<grid, kNeutralThreads, 0, s>>>(P, A, b.desc, b.ndesc);
+  else
+    k_neutral<false><<<grid, kNeutralThreads, 0, s>>>(P, A, b.desc, b.ndesc);
   return cudaGetLastError();
 }
 

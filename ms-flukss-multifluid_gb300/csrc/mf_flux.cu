@@ -1,6 +1,5 @@
-// mf_flux.cu - face-flux kernel with the fast physics (contraction allowed,
-// reciprocals reused): FP32 for the mixed-precision path, FP64 for the fast
-// FP64 path.
+// mf_flux.cu - FP32 face-flux kernels of the mixed-precision path (fast
+// physics: contraction allowed, reciprocals reused), and the line work lists.
 #include <algorithm>
 
 #define MF_PHYS fast
@@ -44,13 +43,8 @@ cudaError_t launch_flux_fast(const DevParams& P, int dir, const double* w, void*
   return cudaGetLastError();
 }
 
-cudaError_t launch_flux_lines_fast(const DevParams& P, int dir, const double* w, void* f,
-                                   void* bn, const Batch& b, const LinePlan& lp,
-                                   const StepState* state, cudaStream_t s) {
-  return launch_lflux_t<double>(P, dir, w, f, bn, b, lp, state, s);
-}
-
 cudaError_t lines_prepare_exact();
+cudaError_t lines_prepare_fma();
 
 cudaError_t lines_prepare() {
   static bool done[64] = {};
@@ -58,7 +52,7 @@ cudaError_t lines_prepare() {
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-  e = lflux_allow_t<double>();
+  e = lines_prepare_fma();
   if (e == cudaSuccess) e = lines_prepare_exact();
   if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
   return e;
@@ -105,23 +99,14 @@ cudaError_t launch_hflux_fast(const DevParams& P, int dir, const double* w, cons
   return launch_hflux_t<R>(P, dir, w, fv, f, bn, b, state, s);
 }
 
-template cudaError_t launch_hflux_fast<double>(const DevParams&, int, const double*,
-                                               const double*, void*, void*, const Batch&,
-                                               const StepState*, cudaStream_t);
 template cudaError_t launch_hflux_fast<float>(const DevParams&, int, const double*,
                                               const double*, void*, void*, const Batch&,
                                               const StepState*, cudaStream_t);
 
-template cudaError_t launch_face_flux_fast<double>(const DevParams&, int, const double*,
-                                                   const double*, double*, int, double,
-                                                   cudaStream_t);
 template cudaError_t launch_face_flux_fast<float>(const DevParams&, int, const double*,
                                                   const double*, double*, int, double,
                                                   cudaStream_t);
 
-template cudaError_t launch_flux_fast<double>(const DevParams&, int, const double*, void*, void*,
-                                              const Batch&, const StepState*, cudaStream_t,
-                                              const float*, int, int);
 template cudaError_t launch_flux_fast<float>(const DevParams&, int, const double*, void*, void*,
                                              const Batch&, const StepState*, cudaStream_t,
                                              const float*, int, int);

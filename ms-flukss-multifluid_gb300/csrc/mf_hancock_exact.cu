@@ -15,10 +15,12 @@
 // The predictor always runs in FP64 with the reference's rounding (this unit
 // is built with -fmad=false); the corrector fluxes and update follow the
 // context's precision mode.
+#define MF_PHYS exact
 #include "mf_kernels.cuh"
 
 #define MF_PHYS exact
 #include "mf_sources_exact.cuh"
+#include "mf_update_kernel.cuh"
 
 namespace mf {
 namespace {
@@ -90,19 +92,18 @@ __global__ void __launch_bounds__(kMaxBlock)
   }
 }
 
-// FLUXESHANCOCK (srcIdeal/PatchIdealMHDF.ChF:235-297) + FLUXESHANCOCK_E
-// (srcIdeal/PatchEulerF.ChF:417-468): physical flux in direction D of one
-// primitive state.  The psi flux is unset in the reference; zero here.
-template <int D, int IRHON>
-__device__ __forceinline__ void point_flux(const DevParams& P, const double* w, double* F) {
+// FLUXESHANCOCK (srcIdeal/PatchIdealMHDF.ChF:235-297): physical plasma flux in
+// direction D of one primitive state.
+template <int D>
+__device__ __forceinline__ void point_flux_plasma(const DevParams& P, const double* w, double* F) {
   constexpr int in = 1 + D, it1 = 1 + (D + 1) % 3, it2 = 1 + (D + 2) % 3;
   constexpr int inB = 5 + D, itB1 = 5 + (D + 1) % 3, itB2 = 5 + (D + 2) % 3;
-  const double rho = fmax(P.smallr, w[0]);
+  const double rho = ieee64::maxnum(P.smallr, w[0]);
   const double u = w[in], v = w[it1], ww = w[it2];
-  double pr = fmax(P.smallp, w[4]);
+  double pr = ieee64::maxnum(P.smallp, w[4]);
   const double bx = w[inB], by = w[itB1], bz = w[itB2];
   const double b = kInv8Pi * (bx * bx + by * by + bz * bz);
-  const double ke = 0.5 * (u * u + v * v + ww * ww);
+  const double ke = ieee64::half(u * u + v * v + ww * ww);
   const double bu = bx * u + by * v + bz * ww;
   double e = pr * P.invhgamma + rho * ke;
   pr = pr + b;
@@ -115,28 +116,38 @@ __device__ __forceinline__ void point_flux(const DevParams& P, const double* w, 
   F[inB] = 0.0;
   F[itB1] = u * by - v * bx;
   F[itB2] = u * bz - ww * bx;
+}
+
+// FLUXESHANCOCK_E (srcIdeal/PatchEulerF.ChF:417-468): one neutral population.
+template <int D>
+__device__ __forceinline__ void point_flux_neutral(const DevParams& P, const double* w, double* F) {
+  constexpr int in = 1 + D, it1 = 1 + (D + 1) % 3, it2 = 1 + (D + 2) % 3;
+  const double r = ieee64::maxnum(P.smallr, w[0]);
+  const double un = w[in], vn = w[it1], wn = w[it2];
+  const double pn = ieee64::maxnum(P.smallp, w[4]);
+  const double k2 = ieee64::half(un * un + vn * vn + wn * wn);
+  const double en = pn * P.invhgamma + r * k2;
+  F[0] = r * un;
+  F[in] = r * un * un + pn;
+  F[it1] = r * un * vn;
+  F[it2] = r * un * wn;
+  F[4] = un * (en + pn);
+}
+
+// Every fluid of one primitive state.  The psi flux is unset in the
+// reference; zero here.
+template <int D, int IRHON>
+__device__ __forceinline__ void point_flux(const DevParams& P, const double* w, double* F) {
+  point_flux_plasma<D>(P, w, F);
   if (IRHON == 9) F[8] = 0.0;
 #pragma unroll
-  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
-    if (f < P.nf) {
-      const int s = IRHON + (f - 1) * 5;
-      const double r = fmax(P.smallr, w[s]);
-      const double un = w[s + 1 + D], vn = w[s + 1 + (D + 1) % 3], wn = w[s + 1 + (D + 2) % 3];
-      const double pn = fmax(P.smallp, w[s + 4]);
-      const double k2 = 0.5 * (un * un + vn * vn + wn * wn);
-      const double en = pn * P.invhgamma + r * k2;
-      F[s] = r * un;
-      F[s + 1 + D] = r * un * un + pn;
-      F[s + 1 + (D + 1) % 3] = r * un * vn;
-      F[s + 1 + (D + 2) % 3] = r * un * wn;
-      F[s + 4] = un * (en + pn);
-    }
-  }
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f)
+    if (f < P.nf) point_flux_neutral<D>(P, w + IRHON + (f - 1) * 5, F + IRHON + (f - 1) * 5);
   // FLUXESHANCOCK_LS (src/LevelSetF.ChF:9-35): surface times the plasma
   // normal velocity
 #pragma unroll
   for (int q = 0; q < MF_MAX_COMP; ++q)
-    if (q >= P.ils && q < P.nc) F[q] = w[q] * w[in];
+    if (q >= P.ils && q < P.nc) F[q] = w[q] * w[1 + D];
 }
 
 // Bn of one face (PatchMHDMF::computeBn, srcIdeal/PatchMHDMF.cpp:509-620)
@@ -146,7 +157,7 @@ __device__ __forceinline__ double face_bn(const DevParams& P, const RunParams& R
                                           double wl, double wr, double cl, double cr) {
   if (P.divb_method == 0) return 0.0;
   if (P.divb_method == 2) return 0.5 * (cl + cr);
-  double bn = 0.5 * (wl + wr);
+  double bn = ieee64::half(wl + wr);
   if (!P.periodic[d]) {
     if (f == RP.dlo[d]) bn = wr;
     if (f == RP.dhi[d] + 1) bn = wl;
@@ -227,22 +238,8 @@ __global__ void __launch_bounds__(kMaxBlock)
   if (P.sd > 2)
     hpredict_dir<2, IRHON>(P, RP, D, H, W, base, cs, scs, c, x, nc, dtinv, dtp, u, divB);
   // addExplicitSources with W(t) and dt/2 (srcIdeal/PatchMHDMF.cpp:1149-1389)
-  double w[MF_MAX_COMP];
-#pragma unroll
-  for (int q = 0; q < MF_MAX_COMP; ++q)
-    if (q < nc) w[q] = W[base + q * cs];
-  if (P.use8) {
-    const double dB = -divB * (dtp / RP.dx);
-    const double Ux = w[1], Uy = w[2], Uz = w[3];
-    const double Bx = kInv4Pi * w[5], By = kInv4Pi * w[6], Bz = kInv4Pi * w[7];
-    u[1] = u[1] + dB * Bx;
-    u[2] = u[2] + dB * By;
-    u[3] = u[3] + dB * Bz;
-    u[4] = u[4] + dB * (Bx * Ux + By * Uy + Bz * Uz);
-    u[5] = u[5] + dB * Ux;
-    u[6] = u[6] + dB * Uy;
-    u[7] = u[7] + dB * Uz;
-  }
+  const WColumn w{W + base, cs};
+  if (P.use8) source_8wave(w, divB, dtp / RP.dx, u);
   if (GLM) u[8] = exp(-dtp * SS.ch * SS.ch / (SS.cp * SS.cp)) * u[8];
   if (P.ce && P.nf >= 2) {
     const double regtr = P.reg_tracer ? W[base + (nc - 1) * cs] : 0.0;
@@ -262,6 +259,129 @@ __global__ void __launch_bounds__(kMaxBlock)
 #pragma unroll
   for (int q = 0; q < MF_MAX_COMP; ++q)
     if (q < nc) H.w2[base + q * cs] = wo[q];
+}
+
+// The predictor with one thread per cell and fluid, as the update kernel
+// (mf_cell_kernel.cuh) and for its reason: a thread with a whole cell took all
+// 255 registers and spilled.  Every option but tracking surfaces.
+template <int D>
+__device__ __forceinline__ void hpredict_fluid(const DevParams& P, const RunParams& RP,
+                                               const StageDesc& Dc, const HancockBuffers& H,
+                                               const double* __restrict__ W, long long base,
+                                               long long cs, long long scs, long long c,
+                                               const int* x, bool plasma, int s, double dtinv,
+                                               double* u, double& divB) {
+  const int nc = P.nc;
+  const double* __restrict__ fv = H.fv[D] + Dc.fv_off[D];
+  double wm[8], wp[8], fm[8], fp[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    if (v < 5 || plasma) {
+      wm[v] = fv[(s + v) * scs + c];
+      wp[v] = fv[(nc + s + v) * scs + c];
+    }
+  }
+  if (plasma) {
+    point_flux_plasma<D>(P, wm, fm);
+    point_flux_plasma<D>(P, wp, fp);
+  } else {
+    point_flux_neutral<D>(P, wm, fm);
+    point_flux_neutral<D>(P, wp, fp);
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (q < 5 || plasma) u[q] = u[q] - dtinv * (fp[q] - fm[q]);
+  if (!plasma || !P.use8) return;
+  const long long ss = dstride(Dc.sn, D);
+  const long long fs = dstride(Dc.fn, D);
+  const double* wbn = W + base + (5 + D) * cs;
+  const double bn_lo = face_bn(P, RP, D, x[D], fv[(nc + 5 + D) * scs + c - ss],
+                               fv[(5 + D) * scs + c], wbn[-fs], wbn[0]);
+  const double bn_hi = face_bn(P, RP, D, x[D] + 1, fv[(nc + 5 + D) * scs + c],
+                               fv[(5 + D) * scs + c + ss], wbn[0], wbn[fs]);
+  divB = divB + bn_hi - bn_lo;
+}
+
+template <int NF>
+__global__ void __launch_bounds__(kCellBlock* NF, 65536 / (128 * kCellBlock * NF))
+    k_hpredict_fluids(const __grid_constant__ DevParams P, const double* __restrict__ U,
+                      const double* __restrict__ W, HancockBuffers H,
+                      const StageDesc* __restrict__ descs, int ndesc, int total,
+                      const RunParams* __restrict__ runs, const StepState* __restrict__ states) {
+  constexpr int NN = NF - 1;
+  __shared__ double terms[NN > 0 ? NN : 1][CeTerms::kShared][kCellBlock];
+  __shared__ int region[kCellBlock];
+  const int role = threadIdx.x / kCellBlock, lane = threadIdx.x % kCellBlock;
+  const bool plasma = NN == 0 || role == 0;
+  const bool ce = NN > 0 && P.ce;
+  const int g = blockIdx.x * kCellBlock + lane;
+  const StageDesc* Dp = nullptr;
+  if (g < total) {
+    Dp = &descs[find_desc(descs, ndesc, kRegV, g)];
+    // (a run-alignment gap holds no cell)
+    if (g - Dp->g0[kRegV] >= Dp->vn[0] * Dp->vn[1] * Dp->vn[2]) Dp = nullptr;
+  }
+  const int s = plasma ? 0 : P.irhon + (role - 1) * 5;
+  long long cs = 0, base = 0;
+  double dtp = 0.0, u[8], psi = 0.0;
+  CeTerms t;
+  if (Dp) {
+    const StageDesc& D = *Dp;
+    const RunParams& RP = runs[D.run];
+    const StepState& SS = states[D.run];
+    int x[3];
+    decode(g - D.g0[kRegV], D.vlo, D.vn, x[0], x[1], x[2]);
+    cs = (long long)D.fn[0] * D.fn[1] * D.fn[2];
+    base = D.u_off + loc(D.flo, D.fn, x[0], x[1], x[2]);
+    const long long scs = (long long)D.sn[0] * D.sn[1] * D.sn[2];
+    const long long c = loc(D.slo, D.sn, x[0], x[1], x[2]);
+    dtp = 0.5 * SS.dt;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < 5 || plasma) u[q] = U[base + (s + q) * cs];
+    // updateHancock -> UPDATECONSHANCOCK (src/PatchMHDAMF.ChF:589-638), one
+    // direction after another; divB from Bn of the face values (COMPUTEDIVB)
+    const double dtinv = dtp * RP.invdx;
+    double divB = 0.0;
+    hpredict_fluid<0>(P, RP, D, H, W, base, cs, scs, c, x, plasma, s, dtinv, u, divB);
+    if (P.sd > 1)
+      hpredict_fluid<1>(P, RP, D, H, W, base, cs, scs, c, x, plasma, s, dtinv, u, divB);
+    if (P.sd > 2)
+      hpredict_fluid<2>(P, RP, D, H, W, base, cs, scs, c, x, plasma, s, dtinv, u, divB);
+    // addExplicitSources with W(t) and dt/2 (srcIdeal/PatchMHDMF.cpp:1149-1389)
+    const WColumn w{W + base, cs};
+    if (plasma) {
+      if (P.use8) source_8wave(w, divB, dtp / RP.dx, u);
+      if (P.glm) psi = exp(-dtp * SS.ch * SS.ch / (SS.cp * SS.cp)) * U[base + 8 * cs];
+      if (ce) region[lane] = region_cell(P, RP.dx, x[0], x[1], x[2], w, 0.0);
+    } else if (ce) {
+      charge_exchange_terms(P, w, s, t);
+#pragma unroll
+      for (int q = 0; q < CeTerms::kShared; ++q) terms[role - 1][q][lane] = t.shared[q];
+    }
+  }
+  if (ce) __syncthreads();
+  if (!Dp) return;
+  if constexpr (NN > 0) {
+    if (ce) {
+      const auto at = [&](int f, int q) { return terms[f][q][lane]; };
+      if (plasma)
+        charge_exchange_plasma<NN>(dtp, u, at);
+      else
+        charge_exchange_neutral<NN>(ce_recipient(NN, region[lane]) == role, role - 1,
+                                    WColumn{W + base, cs}, t, dtp, u, at);
+    }
+  }
+  // W(t + dt/2) (stateToPrim of the predicted state)
+  double wo[8];
+  if (plasma)
+    cons_to_prim_plasma(P, u, wo);
+  else
+    cons_to_prim_euler(P, u, wo);
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if (q < 5 || plasma) H.w2[base + (s + q) * cs] = wo[q];
+  if (plasma && P.glm) H.w2[base + 8 * cs] = psi;
 }
 
 __global__ void __launch_bounds__(kMaxBlock)
@@ -338,7 +458,20 @@ cudaError_t launch_hancock(const DevParams& P, int precision, const StageBuffers
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   mark();
   const int nt2 = a.nt[2];
-  if (a.tot_v > 0) {
+  if (a.tot_v > 0 && P.nls == 0) {
+    const unsigned nb = flat_blocks(a.tot_v, kCellBlock);
+#define MF_PREDICT(NF)                                                                     \
+  k_hpredict_fluids<NF><<<nb, kCellBlock * NF, 0, s>>>(P, B.uin, B.w, H, a.desc, a.ndesc, \
+                                                       a.tot_v, a.runs, state)
+    switch (P.nf) {
+      case 1: MF_PREDICT(1); break;
+      case 2: MF_PREDICT(2); break;
+      case 3: MF_PREDICT(3); break;
+      case 4: MF_PREDICT(4); break;
+      default: MF_PREDICT(5); break;
+    }
+#undef MF_PREDICT
+  } else if (a.tot_v > 0) {
     if (P.glm)
       k_hpredict<1><<<flat_blocks(a.tot_v, nt2), nt2, 0, s>>>(P, B.uin, B.w, H, a.desc, a.ndesc,
                                                               a.tot_v, a.runs, state);
@@ -352,15 +485,30 @@ cudaError_t launch_hancock(const DevParams& P, int precision, const StageBuffers
     k_hshift<<<flat_blocks(a.tot_s, nt), nt, 0, s>>>(P, B.w, H, a.desc, a.ndesc, a.tot_s, a.runs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   mark();
-  for (int d = 0; d < P.sd; ++d) {
-    if (precision == MF_PREC_MIXED)
-      e = launch_hflux_fast<float>(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
-    else if (precision == MF_PREC_FP64_FAST)
-      e = launch_hflux_fast<double>(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
-    else
-      e = launch_hflux_exact(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+  if (flux_split(P, precision)) {
+    const double* const fv[3] = {H.fv[0], H.fv[1], H.fv[2]};
+    const bool fast = precision == MF_PREC_FP64_FAST;
+    e = fast ? launch_plasma_fast(P, B.w, fv, B.f, B.bn, c, state, s)
+             : launch_plasma_exact(P, B.w, fv, B.f, B.bn, c, state, s);
     if (e != cudaSuccess) return e;
     mark();
+    if (P.nf > 1) {
+      e = fast ? launch_neutral_fast(P, B.w, fv, B.f, c, s)
+               : launch_neutral_exact(P, B.w, fv, B.f, c, s);
+      if (e != cudaSuccess) return e;
+      mark();
+    }
+  } else {
+    for (int d = 0; d < P.sd; ++d) {
+      if (precision == MF_PREC_MIXED)
+        e = launch_hflux_fast<float>(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+      else if (precision == MF_PREC_FP64_FAST)
+        e = launch_hflux_fast<double>(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+      else
+        e = launch_hflux_exact(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+      if (e != cudaSuccess) return e;
+      mark();
+    }
   }
   StageBuffers B2 = B;
   B2.w = H.w2;

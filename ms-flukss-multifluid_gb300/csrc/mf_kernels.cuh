@@ -279,16 +279,17 @@ cudaError_t launch_update_exact(const DevParams& P, const StageBuffers& B, const
 inline bool flux_split(const DevParams& P, int precision) {
   return precision != MF_PREC_MIXED && !P.char_rec && !P.helio_bc && P.nls == 0;
 }
-cudaError_t launch_plasma_exact(const DevParams& P, const double* w, void* const f[3],
-                                void* const bn[3], const Batch& b, const StepState* state,
-                                cudaStream_t s);
-cudaError_t launch_neutral_exact(const DevParams& P, const double* w, void* const f[3],
-                                 const Batch& b, cudaStream_t s);
-cudaError_t launch_plasma_fast(const DevParams& P, const double* w, void* const f[3],
-                               void* const bn[3], const Batch& b, const StepState* state,
-                               cudaStream_t s);
-cudaError_t launch_neutral_fast(const DevParams& P, const double* w, void* const f[3],
-                                const Batch& b, cudaStream_t s);
+// fv: null, or the Hancock corrector's face values per direction.
+cudaError_t launch_plasma_exact(const DevParams& P, const double* w, const double* const* fv,
+                                void* const f[3], void* const bn[3], const Batch& b,
+                                const StepState* state, cudaStream_t s);
+cudaError_t launch_neutral_exact(const DevParams& P, const double* w, const double* const* fv,
+                                 void* const f[3], const Batch& b, cudaStream_t s);
+cudaError_t launch_plasma_fast(const DevParams& P, const double* w, const double* const* fv,
+                               void* const f[3], void* const bn[3], const Batch& b,
+                               const StepState* state, cudaStream_t s);
+cudaError_t launch_neutral_fast(const DevParams& P, const double* w, const double* const* fv,
+                                void* const f[3], const Batch& b, cudaStream_t s);
 // The face fluxes and Bn of every direction of a stage from B.w / B.wf, in
 // flux_launches launches, with B.ev's events from *ne on after each.
 cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers& B,
@@ -470,7 +471,9 @@ cudaError_t launch_hancock(const DevParams& P, int precision, const StageBuffers
                            const HancockBuffers& H, const Batch& a, const Batch& c,
                            StepState* state, DtPartial* partials, int* nblocks_v,
                            cudaStream_t s, int corrector_flags = kStageDt);
-inline int hancock_launches(int sd) { return 5 + sd; }
+inline int hancock_launches(const DevParams& P, int precision) {
+  return 5 + flux_launches(P, precision, false);
+}
 
 // Corrector fluxes of the Hancock step from the shifted face values.
 cudaError_t launch_hflux_exact(const DevParams& P, int dir, const double* w, const double* fv,

@@ -8,8 +8,31 @@
 
 #include "mf_device.cuh"
 
+// Each product that a sum takes in is written mad(a, b, c) = a b + c or
+// nmad(a, b, c) = c - a b.  The parity path (namespace exact) rounds the
+// product and the sum; a unit that names another namespace in MF_RIEMANN_NS
+// (the fast FP64 path) gets them fused, in the same places in every kernel.
+// There a difference that is >= 0 exactly can round below 0, and its root
+// takes 0.
+#ifdef MF_RIEMANN_NS
+#define MF_RIEMANN_FUSED 1
+#else
+#define MF_RIEMANN_NS exact
+#define MF_RIEMANN_FUSED 0
+#endif
+
 namespace mf {
-namespace exact {
+namespace MF_RIEMANN_NS {
+
+__device__ __forceinline__ double mad(double a, double b, double c) {
+  return MF_RIEMANN_FUSED ? fma(a, b, c) : a * b + c;
+}
+__device__ __forceinline__ double nmad(double a, double b, double c) {
+  return MF_RIEMANN_FUSED ? fma(-a, b, c) : c - a * b;
+}
+__device__ __forceinline__ double radicand(double x) {
+  return MF_RIEMANN_FUSED ? ieee64::maxnum(0.0, x) : x;
+}
 
 // ---------------------------------------------------------------------------
 // Roe 8-wave / 7-wave MHD flux: RIEMANNF (src/Roe8WaveF.ChF:5-601) and
@@ -44,15 +67,15 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
   const double BXR = wr[inB], BYR = wr[it1B], BZR = wr[it2B];
 
   const double RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
-  const double BxBL = i8pi * (BXL * BXL + BYL * BYL + BZL * BZL);
-  const double RUxUL = half(RUL * UL + RVL * VL + RWL * WL);
+  const double BxBL = i8pi * mad(BZL, BZL, mad(BYL, BYL, BXL * BXL));
+  const double RUxUL = half(mad(RWL, WL, mad(RVL, VL, RUL * UL)));
   const double PL = PGasL + BxBL;
   const double EL = div(PGasL, hgamma) + RUxUL + BxBL;
   const double AL2 = div(gamma * PGasL, RhoL);
 
   const double RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
-  const double BxBR = i8pi * (BXR * BXR + BYR * BYR + BZR * BZR);
-  const double RUxUR = half(RUR * UR + RVR * VR + RWR * WR);
+  const double BxBR = i8pi * mad(BZR, BZR, mad(BYR, BYR, BXR * BXR));
+  const double RUxUR = half(mad(RWR, WR, mad(RVR, VR, RUR * UR)));
   const double PR = PGasR + BxBR;
   const double ER = div(PGasR, hgamma) + RUxUR + BxBR;
   const double AR2 = div(gamma * PGasR, RhoR);
@@ -65,23 +88,23 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
     const double HL = div(EL + PL, RhoL), HR = div(ER + PR, RhoR);
     const double coefRL = div(1.0, 1.0 + root(div(RhoR, RhoL)));
     const double coefRR = 1.0 - coefRL;
-    Rho = RhoR * coefRL + RhoL * coefRR;
-    U = UL * coefRL + UR * coefRR;
-    V = VL * coefRL + VR * coefRR;
-    W = WL * coefRL + WR * coefRR;
-    const double HAV = HL * coefRL + HR * coefRR;
-    BX = BXR * coefRL + BXL * coefRR;
-    BY = BYR * coefRL + BYL * coefRR;
-    BZ = BZR * coefRL + BZL * coefRR;
+    Rho = mad(RhoL, coefRR, RhoR * coefRL);
+    U = mad(UR, coefRR, UL * coefRL);
+    V = mad(VR, coefRR, VL * coefRL);
+    W = mad(WR, coefRR, WL * coefRL);
+    const double HAV = mad(HR, coefRR, HL * coefRL);
+    BX = mad(BXL, coefRR, BXR * coefRL);
+    BY = mad(BYL, coefRR, BYR * coefRL);
+    BZ = mad(BZL, coefRR, BZR * coefRL);
     const double BXAV = half(BXL + BXR);
     BX2 = BXAV * BXAV;
-    const double BY2 = BY * BY, BZ2 = BZ * BZ;
-    BYZ2 = BY2 + BZ2;
+    BYZ2 = mad(BZ, BZ, BY * BY);
     BxBH = i8pi * (BX2 + BYZ2);
-    kk = half(U * U + V * V + W * W);
+    kk = half(mad(W, W, mad(V, V, U * U)));
     const double DBX = BXR - BXL, DBY = BYR - BYL, DBZ = BZR - BZL;
-    const double X = div(i8pi * (DBX * DBX + DBY * DBY + DBZ * DBZ) * coefRL * coefRL, RhoL);
-    cc = hgamma * (HAV - kk - div(i4pi * (BX * BXAV + BYZ2), Rho)) + (2.0 - gamma) * X;
+    const double X =
+        div(i8pi * mad(DBZ, DBZ, mad(DBY, DBY, DBX * DBX)) * coefRL * coefRL, RhoL);
+    cc = mad(2.0 - gamma, X, hgamma * (HAV - kk - div(i4pi * mad(BX, BXAV, BYZ2), Rho)));
   } else {
     Rho = half(RhoL + RhoR);
     U = half(UL + UR);
@@ -92,10 +115,9 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
     BZ = half(BZL + BZR);
     const double Pav = half(PL + PR);
     BX2 = BX * BX;
-    const double BY2 = BY * BY, BZ2 = BZ * BZ;
-    BYZ2 = BY2 + BZ2;
+    BYZ2 = mad(BZ, BZ, BY * BY);
     BxBH = i8pi * (BX2 + BYZ2);
-    kk = half(U * U + V * V + W * W);
+    kk = half(mad(W, W, mad(V, V, U * U)));
     const double PGas = Pav - BxBH;
     cc = div(gamma * PGas, Rho);
   }
@@ -121,7 +143,7 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
     hyy = div(BY, hyz);
     hzz = div(BZ, hyz);
     const double szb = cc + div(scale<1>(BxBH), Rho);
-    const double h = root(szb * szb - scale<2>(cc) * bb);
+    const double h = root(radicand(nmad(scale<2>(cc), bb, szb * szb)));
     aas = half(szb - h);
     const bool gone = le(aas, 0.0), capped = le(cc, aas);
     as = root(gone | capped ? 0.0 : aas);
@@ -141,7 +163,7 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
   auto fix = [&](double e) -> double {
     const double z = absval(e);
     if (le(del, z)) return z;
-    return div(half(z * z + dell2), del);
+    return div(half(mad(z, z, dell2)), del);
   };
   const double A1 = fix(U);
   const double A2 = A1;
@@ -161,19 +183,21 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
   const uint32_t sih = le(0.0, BX) ? 0u : 0x80000000u;
 
   const double fl1 = RUL;
-  const double fl2 = UL * RUL - BXL * BXL * i4pi + PL;
-  const double fl3 = UL * RVL - BXL * BYL * i4pi;
-  const double fl4 = UL * RWL - BXL * BZL * i4pi;
-  const double fl5 = UL * (EL + PL) - BXL * (UL * BXL + VL * BYL + WL * BZL) * i4pi;
-  const double fl7 = UL * BYL - BXL * VL;
-  const double fl8 = UL * BZL - BXL * WL;
+  const double fl2 = nmad(BXL * BXL, i4pi, UL * RUL) + PL;
+  const double fl3 = nmad(BXL * BYL, i4pi, UL * RVL);
+  const double fl4 = nmad(BXL * BZL, i4pi, UL * RWL);
+  const double fl5 =
+      nmad(BXL * mad(WL, BZL, mad(VL, BYL, UL * BXL)), i4pi, UL * (EL + PL));
+  const double fl7 = nmad(BXL, VL, UL * BYL);
+  const double fl8 = nmad(BXL, WL, UL * BZL);
   const double fr1 = RUR;
-  const double fr2 = UR * RUR - BXR * BXR * i4pi + PR;
-  const double fr3 = UR * RVR - BXR * BYR * i4pi;
-  const double fr4 = UR * RWR - BXR * BZR * i4pi;
-  const double fr5 = UR * (ER + PR) - BXR * (UR * BXR + VR * BYR + WR * BZR) * i4pi;
-  const double fr7 = UR * BYR - BXR * VR;
-  const double fr8 = UR * BZR - BXR * WR;
+  const double fr2 = nmad(BXR * BXR, i4pi, UR * RUR) + PR;
+  const double fr3 = nmad(BXR * BYR, i4pi, UR * RVR);
+  const double fr4 = nmad(BXR * BZR, i4pi, UR * RWR);
+  const double fr5 =
+      nmad(BXR * mad(WR, BZR, mad(VR, BYR, UR * BXR)), i4pi, UR * (ER + PR));
+  const double fr7 = nmad(BXR, VR, UR * BYR);
+  const double fr8 = nmad(BXR, WR, UR * BZR);
 
   const double du1 = RhoL - RhoR;
   double du2 = RUL - RUR;
@@ -183,14 +207,12 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
   const double du6 = BXL - BXR;
   const double du7 = BYL - BYR;
   const double du8 = BZL - BZR;
-  if (SEVEN)
-    du5 = -hgamma * (-kk * du1 + U * du2 + V * du3 + W * du4 - du5 + (BY * du7 + BZ * du8) * i4pi);
-  else
-    du5 = -hgamma *
-          (-kk * du1 + U * du2 + V * du3 + W * du4 - du5 + (BX * du6 + BY * du7 + BZ * du8) * i4pi);
-  du2 = div(-U * du1 + du2, Rho);
-  du3 = div(-V * du1 + du3, Rho);
-  du4 = div(-W * du1 + du4, Rho);
+  const double bdb = mad(BZ, du8, SEVEN ? BY * du7 : mad(BY, du7, BX * du6));
+  du5 = -hgamma *
+        mad(bdb, i4pi, mad(W, du4, mad(V, du3, mad(U, du2, -kk * du1))) - du5);
+  du2 = div(nmad(U, du1, du2), Rho);
+  du3 = div(nmad(V, du1, du3), Rho);
+  du4 = div(nmad(W, du1, du4), Rho);
 
   const double sqPiRho = root(kPi * Rho);
   const double sq2PiRho = root(k2Pi * Rho);
@@ -201,51 +223,48 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
   const double ccr = cc * Rho, csq = c * sqPiRho;
   const double h7 = half(du7), h8 = half(du8);
 
-  const double lu1 = A1 * (du1 + flip(div(1.0, cc), 0x80000000u) * du5);
+  const double lu1 = A1 * nmad(div(1.0, cc), du5, du1);
   const double lu2 = A2 * du6;
   const double s33 = hzz * sq2, s34 = hyy * sq2;
-  const double e34 = s34 * du4 - s33 * du3;
-  const double e37 = flip(div(hzz, sq2PiRho) * h7, sih), e38 = flip(div(hyy, sq2PiRho) * h8, sih);
-  const double lu3 = A3 * (e34 + e37 - e38);
-  const double lu4 = A4 * (e34 - e37 + e38);
+  const double e34 = nmad(s33, du3, s34 * du4);
+  const double d37 = flip(div(hzz, sq2PiRho), sih), d38 = flip(div(hyy, sq2PiRho), sih);
+  const double lu3 = A3 * nmad(d38, h8, mad(d37, h7, e34));
+  const double lu4 = A4 * mad(d38, h8, nmad(d37, h7, e34));
   // twice the amplitudes of the fast and slow waves' common parts
-  const double f234 = div(p1, cc) * du2 - flip(div(q1, cc), sih) * du3 - flip(div(q2, cc), sih) * du4;
-  const double f5 = div(alf, ccr) * du5;
-  const double f7 = div(als * hyy, csq) * h7, f8 = div(als * hzz, csq) * h8;
-  const double lu5 = half(A5 * (f234 + f5 + f7 + f8));
-  const double lu6 = half(A6 * (f5 - f234 + f7 + f8));
-  const double g234 = div(p2, cc) * du2 + flip(div(q3, cc), sih) * du3 + flip(div(q4, cc), sih) * du4;
-  const double g5 = div(als, ccr) * du5;
-  const double g7 = div(alf * hyy, csq) * h7, g8 = div(alf * hzz, csq) * h8;
-  const double lu7 = half(A7 * (g234 + g5 - g7 - g8));
-  const double lu8 = half(A8 * (g5 - g234 - g7 - g8));
+  const double f234 = nmad(flip(div(q2, cc), sih), du4,
+                           nmad(flip(div(q1, cc), sih), du3, div(p1, cc) * du2));
+  const double x5 = div(alf, ccr), x7 = div(als * hyy, csq), x8 = div(als * hzz, csq);
+  const double lu5 = half(A5 * mad(x8, h8, mad(x7, h7, mad(x5, du5, f234))));
+  const double lu6 = half(A6 * mad(x8, h8, mad(x7, h7, mad(x5, du5, -f234))));
+  const double g234 = mad(flip(div(q4, cc), sih), du4,
+                          mad(flip(div(q3, cc), sih), du3, div(p2, cc) * du2));
+  const double y5 = div(als, ccr), y7 = div(alf * hyy, csq), y8 = div(alf * hzz, csq);
+  const double lu7 = half(A7 * nmad(y8, h8, nmad(y7, h7, mad(y5, du5, g234))));
+  const double lu8 = half(A8 * nmad(y8, h8, nmad(y7, h7, mad(y5, du5, -g234))));
 
   // right eigenvectors (non-zero entries only)
   const double sp15 = Rho * alf, sp17 = Rho * als;
-  double ra1 = lu1 + sp15 * lu5 + sp15 * lu6 + sp17 * lu7 + sp17 * lu8;
-  double ra2 = p1 * lu5 - p1 * lu6 + p2 * lu7 - p2 * lu8;
-  double ra3 = -(s33 * lu3) - s33 * lu4 - flip(q1 * lu5, sih) + flip(q1 * lu6, sih) +
-               flip(q3 * lu7, sih) - flip(q3 * lu8, sih);
-  double ra4 = s34 * lu3 + s34 * lu4 - flip(q2 * lu5, sih) + flip(q2 * lu6, sih) +
-               flip(q4 * lu7, sih) - flip(q4 * lu8, sih);
+  double ra1 = mad(sp17, lu8, mad(sp17, lu7, mad(sp15, lu6, mad(sp15, lu5, lu1))));
+  double ra2 = nmad(p2, lu8, mad(p2, lu7, nmad(p1, lu6, p1 * lu5)));
+  const double r1 = flip(q1, sih), r2 = flip(q2, sih), r3 = flip(q3, sih), r4 = flip(q4, sih);
+  double ra3 = nmad(r3, lu8, mad(r3, lu7, mad(r1, lu6, nmad(r1, lu5, nmad(s33, lu4, -(s33 * lu3))))));
+  double ra4 = nmad(r4, lu8, mad(r4, lu7, mad(r2, lu6, nmad(r2, lu5, mad(s34, lu4, s34 * lu3)))));
   const double sp55 = sp15 * cc, sp57 = sp17 * cc;
-  double ra5 = sp55 * lu5 + sp55 * lu6 + sp57 * lu7 + sp57 * lu8;
+  double ra5 = mad(sp57, lu8, mad(sp57, lu7, mad(sp55, lu6, sp55 * lu5)));
   const double ra6 = lu2;
   const double sp73 = flip(hzz * sq2PiRho, sih), sp84 = flip(hyy * sq2PiRho, sih);
   const double t5 = scale<1>(als * sqPiRho * c), t7 = scale<1>(alf * sqPiRho * c);
   const double sp75 = t5 * hyy, sp77 = t7 * hyy, sp85 = t5 * hzz, sp87 = t7 * hzz;
-  const double ra7 = sp73 * lu3 - sp73 * lu4 + sp75 * lu5 + sp75 * lu6 - sp77 * lu7 - sp77 * lu8;
-  const double ra8 = sp84 * lu4 - sp84 * lu3 + sp85 * lu5 + sp85 * lu6 - sp87 * lu7 - sp87 * lu8;
+  const double ra7 =
+      nmad(sp77, lu8, nmad(sp77, lu7, mad(sp75, lu6, mad(sp75, lu5, nmad(sp73, lu4, sp73 * lu3)))));
+  const double ra8 =
+      nmad(sp87, lu8, nmad(sp87, lu7, mad(sp85, lu6, mad(sp85, lu5, nmad(sp84, lu3, sp84 * lu4)))));
 
-  if (SEVEN)
-    ra5 = ra1 * kk + Rho * (U * ra2 + V * ra3 + W * ra4) + div(ra5, hgamma) +
-          i4pi * (BY * ra7 + BZ * ra8);
-  else
-    ra5 = ra1 * kk + Rho * (U * ra2 + V * ra3 + W * ra4) + div(ra5, hgamma) +
-          i4pi * (BX * ra6 + BY * ra7 + BZ * ra8);
-  ra2 = U * ra1 + Rho * ra2;
-  ra3 = V * ra1 + Rho * ra3;
-  ra4 = W * ra1 + Rho * ra4;
+  const double bra = mad(BZ, ra8, SEVEN ? BY * ra7 : mad(BY, ra7, BX * ra6));
+  ra5 = mad(i4pi, bra, mad(Rho, mad(W, ra4, mad(V, ra3, U * ra2)), ra1 * kk) + div(ra5, hgamma));
+  ra2 = mad(Rho, ra2, U * ra1);
+  ra3 = mad(Rho, ra3, V * ra1);
+  ra4 = mad(Rho, ra4, W * ra1);
 
   g[0] = half(fl1 + fr1 + ra1);
   g[in] = half(fl2 + fr2 + ra2);
@@ -314,7 +333,7 @@ __device__ __forceinline__ void rusanov_mhd(const DevParams& P, const R* wl, con
   }
   R bb = i4pi * BX2 / Rho;
   R szb = A2 + (BxBH + BxBH) / Rho;
-  R h = sqrt_r<R>(szb * szb - R(4) * A2 * bb);
+  R h = sqrt_r<R>(radicand(szb * szb - R(4) * A2 * bb));
   R aaf = R(0.5) * (szb + h);
   R af = sqrt_r<R>(aaf);
   R em = rabs<R>(U) + af;
@@ -336,12 +355,12 @@ __device__ __forceinline__ void dedner_2x2(R ch, R bxl, R psil, R bxr, R psir, R
   const R ch2 = ch * ch;
   const R hc = div(0.5, ch);
   const R du1 = half(bxl - bxr), du2 = psil - psir;
-  const R lu1 = ch * (du1 - hc * du2);
-  const R lu2 = ch * (du1 + hc * du2);
+  const R lu1 = ch * nmad(hc, du2, du1);
+  const R lu2 = ch * mad(hc, du2, du1);
   const R ra1 = lu1 + lu2;
-  const R ra2 = ch * lu2 - ch * lu1;
+  const R ra2 = nmad(ch, lu1, ch * lu2);
   fbn = half(psil + psir + ra1);
-  fpsi = half(ch2 * bxl + ch2 * bxr + ra2);
+  fpsi = half(mad(ch2, bxr, ch2 * bxl) + ra2);
 }
 
 // VANLEERF (src/VanLeerRSF.ChF:4-130): wl/wr = rho,u,v,w,p of one Euler fluid.
@@ -355,14 +374,14 @@ __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, c
   const R PGasL = maxnum(P.smallp, wl[4]), RhoL = maxnum(P.smallr, wl[0]);
   const R UL = wl[in], VL = wl[it1], WL = wl[it2];
   const R RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
-  const R RUxUL = half(RUL * UL + RVL * VL + RWL * WL);
+  const R RUxUL = half(mad(RWL, WL, mad(RVL, VL, RUL * UL)));
   const R EL = div(PGasL, hgamma) + RUxUL;
   const R AL = root(div(gamma * PGasL, RhoL));
   if (le(UL, -AL)) {
     fr1 = fr2 = fr3 = fr4 = fr5 = R(0);
   } else if (le(AL, UL)) {
     fr1 = RhoL * UL;
-    fr2 = fr1 * UL + PGasL;
+    fr2 = mad(fr1, UL, PGasL);
     fr3 = fr1 * VL;
     fr4 = fr1 * WL;
     fr5 = UL * (EL + PGasL);
@@ -379,14 +398,14 @@ __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, c
   const R PGasR = maxnum(P.smallp, wr[4]), RhoR = maxnum(P.smallr, wr[0]);
   const R UR = wr[in], VR = wr[it1], WR = wr[it2];
   const R RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
-  const R RUxUR = half(RUR * UR + RVR * VR + RWR * WR);
+  const R RUxUR = half(mad(RWR, WR, mad(RVR, VR, RUR * UR)));
   const R ER = div(PGasR, hgamma) + RUxUR;
   const R AR = root(div(gamma * PGasR, RhoR));
   if (le(AR, UR)) {
     fl1 = fl2 = fl3 = fl4 = fl5 = R(0);
   } else if (le(UR, -AR)) {
     fl1 = RhoR * UR;
-    fl2 = fl1 * UR + PGasR;
+    fl2 = mad(fl1, UR, PGasR);
     fl3 = fl1 * VR;
     fl4 = fl1 * WR;
     fl5 = UR * (ER + PGasR);
@@ -408,5 +427,5 @@ __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, c
 }
 
 
-}  // namespace exact
+}  // namespace MF_RIEMANN_NS
 }  // namespace mf

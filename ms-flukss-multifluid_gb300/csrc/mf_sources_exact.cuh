@@ -163,56 +163,65 @@ __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const 
 }
 
 // S = -dt H of the plasma (momentum and energy; the magnetic field's and
-// psi's S is zero).  at(f, q): CeTerms::shared[q] of population f (from 0);
-// NN populations, or nN at run time with NN = 0.
-template <int NN, typename T = double, typename AT>
-__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at,
-                                                       int nN = NN) {
+// psi's S is zero); h: h2..h5.
+__device__ __forceinline__ void charge_exchange_source(double dt, double* u, const double* h) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    double h = 0.0;
-#pragma unroll
-    for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
-      if (f < (NN > 0 ? NN : nN)) h = h + at(f, q);
-    u[1 + q] = u[1 + q] + (-dt * h);
-  }
+  for (int q = 0; q < 4; ++q) u[1 + q] = u[1 + q] + (-dt * h[q]);
 }
 
-// S = -dt H of population f (from 0) with terms c; rec: it receives the
-// newly created neutrals.
+// S = -dt H of a population with terms c; rec: it receives the newly created
+// neutrals, density H1 and the plasma's totals plu (PPLUX, PPLUY, PPLUZ, ENPLU).
+__device__ __forceinline__ void charge_exchange_source(bool rec, double H1, const double* plu,
+                                                       const CeTerms& c, double dt, double* un) {
+  un[0] = un[0] + (-dt * (rec ? H1 : c.shared[4]));
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    un[1 + q] = un[1 + q] + (-dt * (rec ? plu[q] + c.pmi[q] : c.pmi[q]));
+  un[4] = un[4] + (-dt * (rec ? plu[3] + c.enmi : c.enmi));
+}
+
+// H1 of the recipient f (from 0) of nN populations; lost(q): ARR UD
+// (-DENPLU) of population q.
+template <typename L>
+__device__ __forceinline__ double new_neutrals(int nN, int f, const L& lost) {
+  double sum = 0.0;
+  bool first = true;
+#pragma unroll
+  for (int q = 0; q < MF_MAX_FLUIDS - 1; ++q) {
+    if (q < nN && (nN > 3 || q != f)) {
+      sum = first ? -lost(q) : sum - lost(q);
+      first = false;
+    }
+  }
+  return (nN > 3) ? sum + lost(f) : sum;
+}
+
+// The same for a thread per fluid; at(f, q): CeTerms::shared[q] of population f.
+template <int NN, typename T = double, typename AT>
+__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at) {
+  double h[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    h[q] = 0.0;
+#pragma unroll
+    for (int f = 0; f < NN; ++f) h[q] = h[q] + at(f, q);
+  }
+  charge_exchange_source(dt, u, h);
+}
 template <int NN, typename T = double, typename WA, typename AT>
 __device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const WA&,
                                                         const CeTerms& c, double dt, double* un,
-                                                        const AT& at, int nN_ = NN) {
-  const int nN = NN > 0 ? NN : nN_;
-  double H1 = c.shared[4], H2 = c.pmi[0], H3 = c.pmi[1], H4 = c.pmi[2], H5 = c.enmi;
+                                                        const AT& at) {
+  double H1 = 0.0, plu[4] = {0.0, 0.0, 0.0, 0.0};
   if (rec) {
-    double X = 0.0, Y = 0.0, Z = 0.0, E = 0.0, sum = 0.0;
-    bool first = true;
 #pragma unroll
-    for (int q = 0; q < MF_MAX_FLUIDS - 1; ++q) {
-      if (q < nN) {
-        X = X - at(q, 5);
-        Y = Y - at(q, 6);
-        Z = Z - at(q, 7);
-        E = E - at(q, 8);
-        if (nN > 3 || q != f) {
-          sum = first ? -at(q, 4) : sum - at(q, 4);
-          first = false;
-        }
-      }
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int e = 0; e < NN; ++e) plu[q] = plu[q] - at(e, 5 + q);
     }
-    H1 = (nN > 3) ? sum + c.shared[4] : sum;
-    H2 = X + H2;
-    H3 = Y + H3;
-    H4 = Z + H4;
-    H5 = E + H5;
+    H1 = new_neutrals(NN, f, [&](int e) { return at(e, 4); });
   }
-  un[0] = un[0] + (-dt * H1);
-  un[1] = un[1] + (-dt * H2);
-  un[2] = un[2] + (-dt * H3);
-  un[3] = un[3] + (-dt * H4);
-  un[4] = un[4] + (-dt * H5);
+  charge_exchange_source(rec, H1, plu, c, dt, un);
 }
 
 // All populations of one cell by one thread.  T names the arithmetic type for
@@ -224,15 +233,27 @@ __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA
   static_assert(sizeof(T) == sizeof(double), "FP64 physics");
   const int nN = NN > 0 ? NN : P.nf - 1;
   CeTerms c[MF_MAX_FLUIDS - 1];
+  double h[4] = {0.0, 0.0, 0.0, 0.0}, plu[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
-    if (f < nN) charge_exchange_terms(P, w, IRHON + f * 5, c[f]);
-  auto at = [&](int f, int q) { return c[f].shared[q]; };
-  charge_exchange_plasma<NN>(dt, u, at, nN);
+  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f) {
+    if (f < nN) {
+      charge_exchange_terms(P, w, IRHON + f * 5, c[f]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        h[q] = h[q] + c[f].shared[q];
+        plu[q] = plu[q] - c[f].shared[5 + q];
+      }
+    }
+  }
+  charge_exchange_source(dt, u, h);
   const int rk = ce_recipient(nN, reg);
 #pragma unroll
-  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
-    if (f < nN) charge_exchange_neutral<NN>(f + 1 == rk, f, w, c[f], dt, u + IRHON + f * 5, at, nN);
+  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f) {
+    if (f < nN) {
+      const double H1 = new_neutrals(nN, f, [&](int e) { return c[e].shared[4]; });
+      charge_exchange_source(f + 1 == rk, H1, plu, c[f], dt, u + IRHON + f * 5);
+    }
+  }
 }
 
 // SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES

@@ -13,10 +13,11 @@ cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers&
   };
   if (!B.lines && flux_split(P, precision)) {
     const bool fast = precision == MF_PREC_FP64_FAST;
-    e = fast ? launch_plasma_fast(P, B.w, B.f, B.bn, b, state, s)
-             : launch_plasma_exact(P, B.w, B.f, B.bn, b, state, s);
+    e = fast ? launch_plasma_fast(P, B.w, nullptr, B.f, B.bn, b, state, s)
+             : launch_plasma_exact(P, B.w, nullptr, B.f, B.bn, b, state, s);
     if (done() != cudaSuccess || P.nf < 2) return e;
-    e = fast ? launch_neutral_fast(P, B.w, B.f, b, s) : launch_neutral_exact(P, B.w, B.f, b, s);
+    e = fast ? launch_neutral_fast(P, B.w, nullptr, B.f, b, s)
+             : launch_neutral_exact(P, B.w, nullptr, B.f, b, s);
     return done();
   }
   for (int d = 0; d < P.sd; ++d) {
