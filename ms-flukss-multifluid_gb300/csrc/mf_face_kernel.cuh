@@ -1,35 +1,32 @@
 // mf_face_kernel.cuh - face fluxes of the FP64 paths, plasma and neutral
 // populations in kernels of their own, all directions in one launch.
-// Included by mf_face.cu (fast physics) and mf_face_exact.cu (parity
-// physics); MF_PHYS names the physics namespace of the including unit.
+// Included by mf_face_exact.cu (parity path) and mf_face_fma.cu (fast FP64
+// path); MF_PHYS names the physics namespace of the including unit.
 //
 // Bound by the FP64 pipe while enough warps are resident, else by the
 // latency of each warp's chain of FP64 and integer instructions (with both
 // parts in one kernel, 200 registers, 2 warps per scheduler: pipe 53 % busy).
 // The parts share nothing but the face, so the neutral populations run one
-// per thread with about half the registers, and the plasma solver alone fits
-// MF_PLASMA_BLOCKS blocks of 64 per SM.  The state is loaded in the face's
+// per thread with a third of the registers, and the plasma solver alone fits
+// six blocks of 64 per SM.  The state is loaded in the face's
 // frame (normal, then the two transverse components), which makes the code
 // the same for the three directions: one kernel instead of three, a third of
 // the instruction cache.  Fluxes of a 64^3 heliosphere step: 3.68 -> 2.33 ms
-// (pipe 75 % busy); 5 to 8 blocks of the plasma kernel and 3 to 8 of the
-// neutral one per SM measured the same within 2 %.
+// (pipe 75 % busy); 5 to 8 blocks of the plasma kernel per SM measured the
+// same within 2 %.  The neutral kernel takes 8 blocks (64 registers): its
+// products run on the integer pipes (vanleer_euler), whose latency more warps
+// hide (128^3, three populations: 6.04 ms a step with the products on the
+// FP64 pipe and 4 blocks, 5.67 with both changed).
 #pragma once
 
 #include "mf_kernels.cuh"
-
-#ifndef MF_PLASMA_BLOCKS
-#define MF_PLASMA_BLOCKS 6
-#endif
-#ifndef MF_NEUTRAL_BLOCKS
-#define MF_NEUTRAL_BLOCKS 4
-#endif
 
 namespace mf {
 namespace {
 using namespace MF_PHYS;
 
 constexpr int kPlasmaThreads = 64, kNeutralThreads = 128;
+constexpr int kPlasmaBlocks = 6, kNeutralBlocks = 8;  // per SM
 
 // The faces of a batch in every direction: the launch's blocks cover those of
 // direction 0, then 1, then 2 (nb blocks each).  w: the primitive state whose
@@ -160,7 +157,7 @@ __device__ __forceinline__ void flat_cells(const DevParams& P, const Face& F, bo
 // Plasma (and psi) fluxes and Bn of every face, the operations of k_flux (or,
 // HANCOCK, of k_hflux: the face values were limited before the predictor).
 template <int RS, bool HANCOCK>
-__global__ void __launch_bounds__(kPlasmaThreads, MF_PLASMA_BLOCKS)
+__global__ void __launch_bounds__(kPlasmaThreads, kPlasmaBlocks)
     k_plasma(const __grid_constant__ DevParams P, const __grid_constant__ FaceBatch A,
              const StageDesc* __restrict__ descs, int ndesc, const RunParams* __restrict__ runs,
              const StepState* __restrict__ states) {
@@ -211,7 +208,7 @@ __global__ void __launch_bounds__(kPlasmaThreads, MF_PLASMA_BLOCKS)
 
 // Van Leer fluxes of one neutral population (blockIdx.y) of every face.
 template <bool HANCOCK>
-__global__ void __launch_bounds__(kNeutralThreads, MF_NEUTRAL_BLOCKS)
+__global__ void __launch_bounds__(kNeutralThreads, kNeutralBlocks)
     k_neutral(const __grid_constant__ DevParams P, const __grid_constant__ FaceBatch A,
               const StageDesc* __restrict__ descs, int ndesc) {
   Face F;

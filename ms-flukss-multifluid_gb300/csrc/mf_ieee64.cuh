@@ -116,6 +116,38 @@ __device__ __forceinline__ double root(double x) {
   return zero ? x : pack((uint32_t)(s >> 32) + ex, (uint32_t)s);
 }
 
+// a b rounded to nearest even: the 106-bit product of the significands in four
+// 32-bit products, its top 64 bits shifted by one where the product of two
+// numbers in [1, 2) stays below 2.  About 40 integer instructions; a zero
+// factor is handled here, operands or results outside the normal range take the
+// FP64 instruction.  Worth it beside FP64 arithmetic only: alone it takes as
+// long as the instruction (73 clocks against 77 per warp and scheduler).
+__device__ __forceinline__ double mul(double a, double b) {
+  const uint32_t ha = hi_of(a), hb = hi_of(b), la = lo_of(a), lb = lo_of(b);
+  const uint32_t ea = ha & 0x7ff00000u, eb = hb & 0x7ff00000u;
+  const bool zero = (((ha << 1) | la) == 0u) | (((hb << 1) | lb) == 0u);
+  const bool na = ea - 0x00100000u < 0x7fe00000u, nb = eb - 0x00100000u < 0x7fe00000u;
+  // exponent fields' sum in (1024, 3069): a normal result either way of the shift
+  const bool in = na & nb & (((ea >> 1) + (eb >> 1)) - 0x20000000u < 0x3fe00000u);
+  if (!(in | (zero & (ea != 0x7ff00000u) & (eb != 0x7ff00000u)))) return a * b;
+  const uint32_t Ah = __funnelshift_l(la, ha, 11) | 0x80000000u, Al = la << 11;
+  const uint32_t Bh = (hb & 0xfffffu) | 0x100000u;
+  const uint64_t t0 = (uint64_t)Al * lb;
+  const uint64_t t1 = (uint64_t)Ah * lb + (uint32_t)(t0 >> 32);
+  const uint64_t t2 = (uint64_t)Al * Bh + (uint32_t)t1;
+  const uint64_t H = (uint64_t)Ah * Bh + (uint32_t)(t1 >> 32) + (uint32_t)(t2 >> 32);
+  const uint32_t up = (uint32_t)(H >> 52);  // 1: the product is >= 2
+  const uint32_t hh = __funnelshift_l((uint32_t)H, (uint32_t)(H >> 32), 1 - up);
+  const uint32_t hl = __funnelshift_l((uint32_t)t2, (uint32_t)H, 1 - up);
+  const uint32_t rest = __funnelshift_l((uint32_t)t0, (uint32_t)t2, 1 - up);
+  // round up above half, and at half where the last bit is odd
+  const uint32_t sticky = (((uint32_t)t0 << (1 - up)) != 0u) | (hl & 1u);
+  const uint64_t q = join(hh, hl) + ((rest | sticky) > 0x80000000u ? 1u : 0u);
+  const uint32_t ex = ea + eb - 0x40000000u + (up << 20);
+  const uint32_t sg = (ha ^ hb) & 0x80000000u;
+  return zero ? pack(sg, 0u) : pack(((uint32_t)(q >> 32) + ex) | sg, (uint32_t)q);
+}
+
 // Sign-magnitude bits as an ordered integer (-0 and +0 equal).
 __device__ __forceinline__ int64_t key(double x) {
   const int64_t s = (int64_t)((int32_t)hi_of(x) >> 31);

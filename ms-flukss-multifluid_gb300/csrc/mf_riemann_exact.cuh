@@ -364,7 +364,11 @@ __device__ __forceinline__ void dedner_2x2(R ch, R bxl, R psil, R bxr, R psir, R
 }
 
 // VANLEERF (src/VanLeerRSF.ChF:4-130): wl/wr = rho,u,v,w,p of one Euler fluid.
-// Divisions, roots, comparisons and powers of two as in roe_mhd.
+// Divisions, roots, comparisons and powers of two as in roe_mhd, and here the
+// products that no sum takes in: with the warps that fit, the integer pipes
+// have room for them (fluxes of three populations, 128^3: 6.04 -> 5.67 ms a
+// step; in roe_mhd, whose chain is longer and warps are fewer, they cost as
+// much as they save: 12.2 -> 12.1 ms).
 template <typename R, int DIR>
 __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, const R* wr, R* g) {
   using namespace ieee64;
@@ -373,7 +377,7 @@ __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, c
   R fl1, fl2, fl3, fl4, fl5, fr1, fr2, fr3, fr4, fr5;
   const R PGasL = maxnum(P.smallp, wl[4]), RhoL = maxnum(P.smallr, wl[0]);
   const R UL = wl[in], VL = wl[it1], WL = wl[it2];
-  const R RUL = RhoL * UL, RVL = RhoL * VL, RWL = RhoL * WL;
+  const R RUL = mul(RhoL, UL), RVL = mul(RhoL, VL), RWL = mul(RhoL, WL);
   const R RUxUL = half(mad(RWL, WL, mad(RVL, VL, RUL * UL)));
   const R EL = div(PGasL, hgamma) + RUxUL;
   const R AL = root(div(gamma * PGasL, RhoL));
@@ -382,22 +386,22 @@ __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, c
   } else if (le(AL, UL)) {
     fr1 = RhoL * UL;
     fr2 = mad(fr1, UL, PGasL);
-    fr3 = fr1 * VL;
-    fr4 = fr1 * WL;
+    fr3 = mul(fr1, VL);
+    fr4 = mul(fr1, WL);
     fr5 = UL * (EL + PGasL);
   } else {
     const R UA = div(scale<1>(AL) - UL, gamma);
     const R H = div(EL + PGasL, RhoL);
     const R HU = UL + AL;
-    fr1 = scale<-2>(div(RhoL * HU * HU, AL));
+    fr1 = scale<-2>(div(mul(mul(RhoL, HU), HU), AL));
     fr2 = fr1 * (UL + UA);
-    fr3 = fr1 * VL;
-    fr4 = fr1 * WL;
-    fr5 = fr1 * H;
+    fr3 = mul(fr1, VL);
+    fr4 = mul(fr1, WL);
+    fr5 = mul(fr1, H);
   }
   const R PGasR = maxnum(P.smallp, wr[4]), RhoR = maxnum(P.smallr, wr[0]);
   const R UR = wr[in], VR = wr[it1], WR = wr[it2];
-  const R RUR = RhoR * UR, RVR = RhoR * VR, RWR = RhoR * WR;
+  const R RUR = mul(RhoR, UR), RVR = mul(RhoR, VR), RWR = mul(RhoR, WR);
   const R RUxUR = half(mad(RWR, WR, mad(RVR, VR, RUR * UR)));
   const R ER = div(PGasR, hgamma) + RUxUR;
   const R AR = root(div(gamma * PGasR, RhoR));
@@ -406,18 +410,18 @@ __device__ __forceinline__ void vanleer_euler(const DevParams& P, const R* wl, c
   } else if (le(UR, -AR)) {
     fl1 = RhoR * UR;
     fl2 = mad(fl1, UR, PGasR);
-    fl3 = fl1 * VR;
-    fl4 = fl1 * WR;
+    fl3 = mul(fl1, VR);
+    fl4 = mul(fl1, WR);
     fl5 = UR * (ER + PGasR);
   } else {
     const R UA = div(-UR - scale<1>(AR), gamma);
     const R H = div(ER + PGasR, RhoR);
     const R HU = UR - AR;
-    fl1 = -scale<-2>(div(RhoR * HU * HU, AR));
+    fl1 = -scale<-2>(div(mul(mul(RhoR, HU), HU), AR));
     fl2 = fl1 * (UR + UA);
-    fl3 = fl1 * VR;
-    fl4 = fl1 * WR;
-    fl5 = fl1 * H;
+    fl3 = mul(fl1, VR);
+    fl4 = mul(fl1, WR);
+    fl5 = mul(fl1, H);
   }
   g[0] = fl1 + fr1;
   g[in] = fl2 + fr2;

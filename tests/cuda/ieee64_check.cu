@@ -26,8 +26,9 @@ __device__ double ref_minmod(double a, double b) {
   return s * fmax(0.0, fmin(fabs(a), s * b));
 }
 
-// out: div, root, comparisons, max/min, scale, minmod
+// out: div, root, comparisons, max/min, scale, minmod, mul
 __device__ void one(double a, double b, unsigned* out) {
+  if (!same(mul(a, b), __dmul_rn(a, b))) atomicAdd(&out[6], 1u);
   if (!same(div(a, b), __ddiv_rn(a, b))) atomicAdd(&out[0], 1u);
   if (!same(root(b), __dsqrt_rn(b))) atomicAdd(&out[1], 1u);
   if (lt(a, b) != (a < b) || le(a, b) != (a <= b)) atomicAdd(&out[2], 1u);
@@ -54,6 +55,9 @@ __global__ void k_check(unsigned* out) {
     if (m == 3) a = nextafter(a * b, (s & 1) ? 1e308 : -1e308);  // quotient next to a number
     if (m == 5) a = b;
     if (m == 6) a = nextafter(b, (s & 1) ? 1e308 : 0.0);
+    // products near the rounding's half-way points: few significant bits
+    if (m == 7) one(bits(__double_as_longlong(a) & 0xfffffffff8000000ull),
+                    bits((__double_as_longlong(b) & 0xfffffffffc000000ull) | ((s >> 40) & 3)), out);
     one(a, b, out);
     const double q = b * b;  // root next to a number
     if (!same(root(nextafter(q, (s & 1) ? 1e308 : 0.0)), __dsqrt_rn(nextafter(q, (s & 1) ? 1e308 : 0.0))) ||
@@ -75,13 +79,13 @@ __global__ void k_special(unsigned* out) {
 }
 
 int main() {
-  unsigned *d, h[6];
+  unsigned *d, h[7];
   if (cudaMalloc(&d, sizeof(h)) != cudaSuccess) return 2;
   cudaMemset(d, 0, sizeof(h));
   k_check<<<(1 << 23) / 256, 256>>>(d);
   k_special<<<1, 1>>>(d);
   const cudaError_t e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
-  printf("div %u\nroot %u\ncompare %u\nmaxmin %u\nscale %u\nminmod %u\nstatus %s\n", h[0], h[1], h[2],
-         h[3], h[4], h[5], cudaGetErrorString(e));
+  printf("div %u\nroot %u\ncompare %u\nmaxmin %u\nscale %u\nminmod %u\nmul %u\nstatus %s\n", h[0],
+         h[1], h[2], h[3], h[4], h[5], h[6], cudaGetErrorString(e));
   return e == cudaSuccess ? 0 : 1;
 }

@@ -1,5 +1,5 @@
 """The integer-pipe forms of csrc/mf_ieee64.cuh against the FP64 instructions
-on the GPU, bit for bit: division, square root, comparisons, maximum and
+on the GPU, bit for bit: division, square root, product, comparisons, maximum and
 minimum, scaling by powers of two and minmod."""
 import os
 import shutil
@@ -9,7 +9,7 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(HERE), "ms-flukss-multifluid_gb300", "csrc")
-NAMES = ("div", "root", "compare", "maxmin", "scale", "minmod")
+NAMES = ("div", "root", "compare", "maxmin", "scale", "minmod", "mul")
 
 
 @pytest.fixture(scope="module")
