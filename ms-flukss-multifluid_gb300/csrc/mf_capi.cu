@@ -1294,11 +1294,13 @@ mf_status build_level_plan(const mf_params& p, int ng, int nc, int npatch, const
           D.wlo[d] = valid[i].lo[d];
           D.wn[d] = valid[i].hi[d] - valid[i].lo[d] + 1;
         }
-        // far-field ghosts of valid.grow(2): slabs peeled off the box one
-        // non-periodic direction at a time
-        mf_box rest = box_grow(valid[i], 2, sd);
+        // far-field ghosts of valid.grow(2), on its faces: the stencils reach
+        // out of the valid box in one direction at a time
         for (int d = 0; d < sd; ++d) {
           if (p.periodic[d]) continue;
+          mf_box rest = valid[i];
+          rest.lo[d] -= 2;
+          rest.hi[d] += 2;
           for (int side = 0; side < 2; ++side) {
             mf_box slab = rest;
             if (side == 0)
@@ -1318,8 +1320,29 @@ mf_status build_level_plan(const mf_params& p, int ng, int nc, int npatch, const
             R.run = 0;
             L.far.push_back(R);
           }
-          rest.lo[d] = std::max(rest.lo[d], p.domain_lo[d]);
-          rest.hi[d] = std::min(rest.hi[d], p.domain_hi[d]);
+        }
+      }
+      // the sibling copies likewise: the parts of each region on the faces
+      for (const CopyReg& R : L.two) {
+        const int i = by_off[R.dst_off];
+        mf_box b;
+        for (int e = 0; e < 3; ++e) {
+          b.lo[e] = L.fab[i].lo[e] + R.d0[e];
+          b.hi[e] = b.lo[e] + R.ext[e] - 1;
+        }
+        for (int d = 0; d < sd; ++d) {
+          mf_box arm = valid[i];
+          arm.lo[d] -= 2;
+          arm.hi[d] += 2;
+          const mf_box c = box_isect(b, arm);
+          if (box_empty(c)) continue;
+          CopyReg F = R;
+          for (int e = 0; e < 3; ++e) {
+            F.s0[e] += c.lo[e] - b.lo[e];
+            F.d0[e] += c.lo[e] - b.lo[e];
+            F.ext[e] = c.hi[e] - c.lo[e] + 1;
+          }
+          L.two_faces.push_back(F);
         }
       }
     }
@@ -1651,7 +1674,7 @@ mf_status mf_level_create(mf_ctx* c, int npatch, const mf_box* valid, mf_level**
   mf::batch_default_threads(L->b2);
   mf::batch_default_threads(L->bp);
   const std::vector<CopyReg>& full = plan.full;
-  const std::vector<CopyReg>& two = plan.two;
+  const std::vector<CopyReg>& two = plan.lean ? plan.two_faces : plan.two;
   L->nfull = (int)full.size();
   L->ntwo = (int)two.size();
   L->nparts = mf::dt_partials(L->b2);
@@ -1746,6 +1769,9 @@ mf_status mf_level_create(mf_ctx* c, int npatch, const mf_box* valid, mf_level**
     L->lp.nregs = L->ntwo;
     L->lp.far = (const mf::FarReg*)L->far.p;
     L->lp.nfar = (int)plan.far.size();
+    L->lp.far_cells = 0;
+    for (const mf::FarReg& R : plan.far)
+      L->lp.far_cells = std::max(L->lp.far_cells, R.ext[0] * R.ext[1] * R.ext[2]);
     // the FP64 primitive ghosts are read by the FP64 flux kernels, the
     // characteristic projections, central Bn and the tracking surfaces'
     // floor; the FP32 flux kernels read only the FP32 copy

@@ -51,7 +51,6 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     lin = g - Dp->g0[kRegV];
     if (lin >= Dp->vn[0] * Dp->vn[1] * Dp->vn[2]) Dp = nullptr;  // run-alignment gap
   }
-  const double psi_damp = (plasma && P.glm) ? warp_psi_damping(Dp, states, dt_scale) : 1.0;
   const int s = plasma ? 0 : P.irhon + (role - 1) * 5;  // first component of the thread's fluid
   int i = 0, j = 0, k = 0;
   long long cs = 0, base = 0;
@@ -112,7 +111,7 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
         source_8wave(w, divB, ieee64::div(dt, RP.dx), u);
         if ((flags & kStageDt) && B.divb) B.divb[loc(B.divb_lo, B.divb_n, i, j, k)] = divB;
       }
-      if (P.glm) u[8] = psi_damp * u[8];  // PSIPARABOLIC (src/DednerF.ChF:65-87)
+      if (P.glm) u[8] = states[D.run].damp * u[8];  // PSIPARABOLIC (src/DednerF.ChF:65-87)
       if (ce) region[lane] = region_cell(P, RP.dx, i, j, k, w, 0.0);
     } else if (ce) {
       charge_exchange_terms<T>(P, w, s, t);

@@ -67,6 +67,7 @@ struct StepState {
   int min_idx;      // result: Fortran-order index inside the valid box
   unsigned flags;   // error bits (kFlag*)
   int pad;
+  double damp;      // the current stage's factor of PSIPARABOLIC (written by the prim kernel)
 };
 
 // Problem time of a stage's post-processing: HeliosphericProblem::postprocessing

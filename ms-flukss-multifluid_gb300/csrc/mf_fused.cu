@@ -290,8 +290,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2)
   // the update of the thread's cell
   double dtc = DBL_MAX;
   int myidx = INT_MAX;
-  const StageDesc* Dp = (t < ncell) ? &D : nullptr;
-  const double psi_damp = GLM ? warp_psi_damping(Dp, states, dt_scale) : 1.0;
+  const double psi_damp = GLM ? ss->damp : 1.0;
   if (t < ncell) {
     const int ci = t % T.n[0], cj = (t / T.n[0]) % T.n[1], ck = t / (T.n[0] * T.n[1]);
     const int i = T.lo[0] + ci, j = T.lo[1] + cj, k = T.lo[2] + ck;

@@ -449,7 +449,7 @@ cudaError_t launch_hancock(const DevParams& P, int precision, const StageBuffers
   auto mark = [&]() {
     if (B.ev) cudaEventRecord(B.ev[ne++], s);
   };
-  cudaError_t e = launch_prim(P, B.uin, B.w, a, s);
+  cudaError_t e = launch_prim(P, B.uin, B.w, a, s, nullptr, state, 1.0);
   if (e != cudaSuccess) return e;
   mark();
   const int nt = a.nt[0];

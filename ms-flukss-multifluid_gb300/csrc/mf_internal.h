@@ -52,9 +52,10 @@ struct LevelPlan {
   // sibling's valid cell (or its periodic image) or lies outside the domain,
   // and stage 1 runs on the valid box; the primitive state is then computed
   // on the valid cells (dp: descs whose W box is the valid box), copied into
-  // the ghosts (two) and completed by the far-field fill (far).
+  // the ghosts (two_faces) and completed by the far-field fill (far).
   bool lean = false;
   std::vector<StageDesc> dp;
+  std::vector<CopyReg> two_faces;  // two without the edges and corners, which no stencil reads
   std::vector<FarReg> far;
 };
 

@@ -28,9 +28,17 @@ enum RegionKind : int { kRegW = 0, kRegF = 1, kRegV = 4, kRegS = 5 };
 // Patch whose items contain flattened index g (0 <= g < launch total): the
 // largest d with descs[d].g0[kind] <= g.  Patches with no items share their
 // start with the next one and are skipped by taking the largest such d.
+// Levels of equal patches are the common case, so the patch is guessed from
+// the mean items per patch first (the search of 512 patches takes nine
+// dependent loads and as many branches per thread).
 __device__ __forceinline__ int find_desc(const StageDesc* __restrict__ descs, int ndesc, int kind,
                                          int g) {
+  if (ndesc == 1) return 0;
   int lo = 0, hi = ndesc - 1;
+  const int last = __ldg(&descs[hi].g0[kind]);
+  const int at = min(hi, (int)__fdividef((float)g * (float)hi, (float)last));
+  if (g < last && at < hi && __ldg(&descs[at].g0[kind]) <= g && __ldg(&descs[at + 1].g0[kind]) > g)
+    return at;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (__ldg(&descs[mid].g0[kind]) <= g)
@@ -176,7 +184,7 @@ struct LeanPrim {
   const CopyReg* regs;       // sibling copies into the 2 ghost layers
   int nregs;
   const FarReg* far;         // far-field ghost boxes
-  int nfar;
+  int nfar, far_cells;       // their number, and the cells of the largest
   int exchange_w;            // copy the FP64 W (else only the FP32 copy)
 };
 
@@ -261,10 +269,12 @@ cudaError_t launch_flux_update_overlap(const DevParams& P, const StageBuffers& B
                                        StepState* state, DtPartial* partials, int* nblocks_v,
                                        cudaStream_t s);
 
-// wf (nullable): also the FP32 copy of w (round to nearest, as the FP32 flux
+// state (nullable): also each run's GLM damping factor of a stage of dt_scale
+// time steps; wf (nullable): also the FP32 copy of w (round to nearest, as the FP32 flux
 // kernels would convert each value)
 cudaError_t launch_prim(const DevParams& P, const double* uin, double* w, const Batch& b,
-                        cudaStream_t s, float* wf = nullptr);
+                        cudaStream_t s, float* wf = nullptr, StepState* state = nullptr,
+                        double dt_scale = 1.0);
 
 // FP64 parity path (reference evaluation order, no contraction)
 cudaError_t launch_flux_exact(const DevParams& P, int dir, const double* w, void* f, void* bn,
@@ -381,10 +391,11 @@ cudaError_t launch_finalize(const DevParams& P, const DtPartial* partials, const
 cudaError_t launch_exchange(double* u, const CopyReg* regs, int nreg, int nc, cudaStream_t s);
 cudaError_t launch_exchange_f(float* u, const CopyReg* regs, int nreg, int nc, cudaStream_t s);
 // Far-field ghosts of the primitive state (HELIOGS, as the primitive kernel
-// fills them) on the boxes far (W and, when set, its FP32 copy wf).
+// fills them) on the boxes far, of at most `most` cells (W where
+// write_w, and its FP32 copy wf where set).
 cudaError_t launch_farfield(const DevParams& P, const double* u, double* w, float* wf,
-                            const FarReg* far, int nfar, const RunParams* runs, int have_w,
-                            cudaStream_t s);
+                            const FarReg* far, int nfar, int most, const RunParams* runs,
+                            int write_w, cudaStream_t s);
 // Kernel launches of the primitive part of a stage (1 without lean).
 inline int prim_launches(const LeanPrim* lp, int mixed) {
   if (!lp) return 1;

@@ -13,161 +13,144 @@
 
 namespace mf {
 namespace {
-template <int GLM>
-__global__ void __launch_bounds__(kMaxBlock)
-    k_prim(const __grid_constant__ DevParams P, const double* __restrict__ U, double* __restrict__ W,
-           float* __restrict__ Wf, const StageDesc* __restrict__ descs, int ndesc, int total,
-           const RunParams* __restrict__ runs) {
-  constexpr int IRHON = 8 + GLM;
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= total) return;
-  const StageDesc& D = descs[find_desc(descs, ndesc, kRegW, g)];
-  const int lin = g - D.g0[kRegW];
-  const RunParams& R = runs[D.run];
-  int i, j, k;
-  decode(lin, D.wlo, D.wn, i, j, k);
-  const long long cs = (long long)D.fn[0] * D.fn[1] * D.fn[2];
-  const long long base = D.u_off + loc(D.flo, D.fn, i, j, k);
-  int od = -1;
-  if (P.bc_kind == MF_BC_FARFIELD) {
-    const int x[3] = {i, j, k};
-    for (int d = 0; d < P.sd; ++d)
-      if (!P.periodic[d] && (x[d] < R.dlo[d] || x[d] > R.dhi[d])) od = d;
+// Store N primitive components of a cell to W and to its FP32 copy (each
+// where not null).
+template <int N>
+__device__ __forceinline__ void store_prim(double* __restrict__ W, float* __restrict__ Wf,
+                                           long long o, long long cs, const double* w) {
+  if (W) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) W[o + q * cs] = w[q];
   }
-  double w[MF_MAX_COMP];
-  if (od < 0) {
-    double u[MF_MAX_COMP];
-#pragma unroll
-    for (int q = 0; q < MF_MAX_COMP; ++q)
-      if (q < P.ils) u[q] = U[base + q * cs];
-    cons_to_prim_plasma(P, u, w);
-    if (GLM) w[8] = u[8];
-#pragma unroll
-    for (int f = 1; f < MF_MAX_FLUIDS; ++f)
-      if (f < P.nf) cons_to_prim_euler(P, u + IRHON + (f - 1) * 5, w + IRHON + (f - 1) * 5);
-  } else {
-    // far-field ghost (HELIOGS, swlism/HeliosphericF.ChF:978-1140): plasma and
-    // neutral fluid 1 from the boundary state, the other neutral fluids copy the
-    // primitive state of the nearest domain cell along the boundary normal.
-#pragma unroll
-    for (int q = 0; q < 8; ++q) w[q] = R.bc_plasma[q];
-    if (GLM) w[8] = 0.0;
-    if (P.nf > 1) {
-#pragma unroll
-      for (int q = 0; q < 5; ++q) w[IRHON + q] = R.bc_n1[q];
-    }
-    int x[3] = {i, j, k};
-    x[od] = (x[od] < R.dlo[od]) ? R.dlo[od] : R.dhi[od];
-    const long long eb = D.u_off + loc(D.flo, D.fn, x[0], x[1], x[2]);
-#pragma unroll
-    for (int f = 2; f < MF_MAX_FLUIDS; ++f) {
-      if (f < P.nf) {
-        double u5[5];
-#pragma unroll
-        for (int q = 0; q < 5; ++q) u5[q] = U[eb + (IRHON + (f - 1) * 5 + q) * cs];
-        cons_to_prim_euler(P, u5, w + IRHON + (f - 1) * 5);
-      }
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < MF_MAX_COMP; ++q)
-    if (q < P.ils) W[base + q * cs] = w[q];
-  // tracking surfaces: copied (EqSysMHDMF::stateToPrim, srcIdeal/EqSysMHDMF.cpp:
-  // 207-210); on far-field ghosts the region tracer holds +1 (HELIOGS
-  // :996-1000) and the other surfaces, which HELIOGS leaves unassigned, keep
-  // U's ghost value
-  for (int q = P.ils; q < P.nc; ++q)
-    W[base + q * cs] = (od >= 0 && P.reg_tracer && q == P.nc - 1) ? 1.0 : U[base + q * cs];
   if (Wf) {  // the FP32 copy the mixed-precision flux kernels read
 #pragma unroll
-    for (int q = 0; q < MF_MAX_COMP; ++q)
-      if (q < P.ils) Wf[base + q * cs] = fp64::d2f(w[q]);
-    for (int q = P.ils; q < P.nc; ++q) Wf[base + q * cs] = fp64::d2f(W[base + q * cs]);
+    for (int q = 0; q < N; ++q) Wf[o + q * cs] = fp64::d2f(w[q]);
   }
 }
 
-// Far-field ghosts of the primitive state, exactly as k_prim's far-field
-// branch fills them (HELIOGS, swlism/HeliosphericF.ChF:978-1140), for the
-// levels whose valid-cell primitives and ghost copies come first: plasma and
-// neutral fluid 1 from the boundary state, the other neutral fluids from the
-// primitive state of the nearest cell along the boundary normal.  That cell,
-// when it lies in the domain, is a valid cell of the patch or a ghost cell
-// filled by the copy before this launch (its FP64 state when that copy ran,
-// else the FP32 copy, the only one read downstream); outside the domain (a
-// corner) its conserved state never changes and is converted here.
-template <int GLM>
-__global__ void __launch_bounds__(256)
-    k_farfield(const __grid_constant__ DevParams P, const double* __restrict__ U, double* __restrict__ W,
-               float* __restrict__ Wf, const FarReg* __restrict__ regs,
-               const RunParams* __restrict__ runs, int have_w) {
-  constexpr int IRHON = 8 + GLM;
-  const FarReg F = regs[blockIdx.x];
-  const RunParams& R = runs[F.run];
-  const int n = F.ext[0] * F.ext[1] * F.ext[2];
-  const long long cs = (long long)F.fn[0] * F.fn[1] * F.fn[2];
-  for (int t = threadIdx.x; t < n; t += blockDim.x) {
-    int i, j, k;
-    decode(t, F.lo, F.ext, i, j, k);
-    const long long base = F.off + loc(F.flo, F.fn, i, j, k);
-    int x[3] = {i, j, k};
-    int od = -1;
+// Far-field ghost state of the plasma (HELIOGS, swlism/HeliosphericF.ChF:
+// 978-1140), psi 0 and the tracking surfaces: the region tracer +1 (:996-1000),
+// the others, which HELIOGS leaves unassigned, keep U's ghost value.
+__device__ __forceinline__ void far_plasma(const DevParams& P, const RunParams& R,
+                                           const double* __restrict__ U, double* __restrict__ W,
+                                           float* __restrict__ Wf, long long base, long long cs) {
+  double w[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) w[q] = R.bc_plasma[q];
+  store_prim<8>(W, Wf, base, cs, w);
+  const double zero = 0.0;
+  if (P.glm) store_prim<1>(W, Wf, base + 8 * cs, cs, &zero);
+  for (int q = P.ils; q < P.nc; ++q) {
+    const double v = (P.reg_tracer && q == P.nc - 1) ? 1.0 : U[base + q * cs];
+    store_prim<1>(W, Wf, base + q * cs, cs, &v);
+  }
+}
+
+// One thread per cell and fluid (blockIdx.y: 0 the plasma, psi and the
+// tracking surfaces, else a neutral population): the kernel moves data, and a
+// thread with a whole cell held 100 registers, too few warps to keep loads in
+// flight.
+__global__ void __launch_bounds__(kMaxBlock)
+    k_prim(const __grid_constant__ DevParams P, const double* __restrict__ U, double* __restrict__ W,
+           float* __restrict__ Wf, const StageDesc* __restrict__ descs, int ndesc, int total,
+           const RunParams* __restrict__ runs, StepState* __restrict__ states, double dt_scale) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= total) return;
+  const int f = blockIdx.y;
+  const StageDesc& D = descs[find_desc(descs, ndesc, kRegW, g)];
+  const int lin = g - D.g0[kRegW];
+  const RunParams& R = runs[D.run];
+  int x[3];
+  decode(lin, D.wlo, D.wn, x[0], x[1], x[2]);
+  const long long cs = (long long)D.fn[0] * D.fn[1] * D.fn[2];
+  const long long base = D.u_off + loc(D.flo, D.fn, x[0], x[1], x[2]);
+  int od = -1;
+  if (P.bc_kind == MF_BC_FARFIELD) {
     for (int d = 0; d < P.sd; ++d)
       if (!P.periodic[d] && (x[d] < R.dlo[d] || x[d] > R.dhi[d])) od = d;
-    if (od < 0) continue;  // (the regions hold far-field cells only)
-    double w[MF_MAX_COMP];
-    float wf[MF_MAX_COMP];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) w[q] = R.bc_plasma[q];
-    if (GLM) w[8] = 0.0;
-    if (P.nf > 1) {
-#pragma unroll
-      for (int q = 0; q < 5; ++q) w[IRHON + q] = R.bc_n1[q];
-    }
-#pragma unroll
-    for (int q = 0; q < MF_MAX_COMP; ++q) wf[q] = fp64::d2f(w[q]);
-    x[od] = (x[od] < R.dlo[od]) ? R.dlo[od] : R.dhi[od];
-    bool inside = true;
-    for (int d = 0; d < P.sd; ++d)
-      if (!P.periodic[d] && (x[d] < R.dlo[d] || x[d] > R.dhi[d])) inside = false;
-    const long long eb = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]);
-#pragma unroll
-    for (int f = 2; f < MF_MAX_FLUIDS; ++f) {
-      if (f < P.nf) {
-        const int s0 = IRHON + (f - 1) * 5;
-        if (!inside) {
-          double u5[5];
-#pragma unroll
-          for (int q = 0; q < 5; ++q) u5[q] = U[eb + (s0 + q) * cs];
-          cons_to_prim_euler(P, u5, w + s0);
-#pragma unroll
-          for (int q = 0; q < 5; ++q) wf[s0 + q] = fp64::d2f(w[s0 + q]);
-        } else if (have_w) {
-#pragma unroll
-          for (int q = 0; q < 5; ++q) {
-            w[s0 + q] = W[eb + (s0 + q) * cs];
-            wf[s0 + q] = fp64::d2f(w[s0 + q]);
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 5; ++q) {
-            wf[s0 + q] = Wf[eb + (s0 + q) * cs];
-            w[s0 + q] = (double)wf[s0 + q];
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int q = 0; q < MF_MAX_COMP; ++q)
-      if (q < P.ils) {
-        W[base + q * cs] = w[q];
-        if (Wf) Wf[base + q * cs] = wf[q];
-      }
-    for (int q = P.ils; q < P.nc; ++q) {
-      const double v = (P.reg_tracer && q == P.nc - 1) ? 1.0 : U[base + q * cs];
-      W[base + q * cs] = v;
-      if (Wf) Wf[base + q * cs] = fp64::d2f(v);
-    }
   }
+  if (f == 0) {
+    // GLM damping factor exp(-dt Ch^2 / Cp^2) of PSIPARABOLIC (src/DednerF.ChF:
+    // 65-87) of the stage, once per patch (all of a run write the same value)
+    // instead of in every warp of the update
+    if (P.glm && states && lin == 0) {
+      StepState& S = states[D.run];
+      const double dt = S.dt * dt_scale;
+      S.damp = exp(-dt * S.ch * S.ch / (S.cp * S.cp));
+    }
+    if (od >= 0) {
+      far_plasma(P, R, U, W, Wf, base, cs);
+      return;
+    }
+    double u[8], w[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) u[q] = U[base + q * cs];
+    cons_to_prim_plasma(P, u, w);
+    store_prim<8>(W, Wf, base, cs, w);
+    // psi and the tracking surfaces: copied (EqSysMHDMF::stateToPrim,
+    // srcIdeal/EqSysMHDMF.cpp:198-201, 207-210)
+    if (P.glm) store_prim<1>(W, Wf, base + 8 * cs, cs, U + base + 8 * cs);
+    for (int q = P.ils; q < P.nc; ++q)
+      store_prim<1>(W, Wf, base + q * cs, cs, U + base + q * cs);
+    return;
+  }
+  // far-field ghost: neutral fluid 1 from the boundary state, the others the
+  // primitive state of the nearest domain cell along the boundary normal
+  const int s = P.irhon + (f - 1) * 5;
+  double u[5], w[5];
+  if (od >= 0 && f == 1) {
+#pragma unroll
+    for (int q = 0; q < 5; ++q) w[q] = R.bc_n1[q];
+  } else {
+    long long from = base;
+    if (od >= 0) {
+      x[od] = (x[od] < R.dlo[od]) ? R.dlo[od] : R.dhi[od];
+      from = D.u_off + loc(D.flo, D.fn, x[0], x[1], x[2]);
+    }
+#pragma unroll
+    for (int q = 0; q < 5; ++q) u[q] = U[from + (s + q) * cs];
+    cons_to_prim_euler(P, u, w);
+  }
+  store_prim<5>(W, Wf, base + s * cs, cs, w);
+}
+
+// Far-field ghosts of the primitive state, exactly as k_prim's far-field
+// branch fills them, for the levels whose valid-cell primitives and ghost
+// copies come first: plasma and neutral fluid 1 from the boundary state, the
+// other neutral fluids from the primitive state of the nearest cell along the
+// boundary normal, a valid cell of the patch.  One block per box, fluid and
+// 256 cells.
+__global__ void __launch_bounds__(256)
+    k_farfield(const __grid_constant__ DevParams P, const double* __restrict__ U, double* W,
+               float* __restrict__ Wf, const FarReg* __restrict__ regs,
+               const RunParams* __restrict__ runs, int write_w) {
+  const FarReg& F = regs[blockIdx.x];
+  const RunParams& R = runs[F.run];
+  const int f = blockIdx.y;
+  const int t = blockIdx.z * blockDim.x + threadIdx.x;
+  if (t >= F.ext[0] * F.ext[1] * F.ext[2]) return;
+  const long long cs = (long long)F.fn[0] * F.fn[1] * F.fn[2];
+  int x[3];
+  decode(t, F.lo, F.ext, x[0], x[1], x[2]);
+  const long long base = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]);
+  double* Ww = write_w ? W : nullptr;  // (else only the FP32 ghosts are read)
+  if (f == 0) {
+    far_plasma(P, R, U, Ww, Wf, base, cs);
+    return;
+  }
+  const int s = P.irhon + (f - 1) * 5;
+  double w[5];
+  if (f == 1) {
+#pragma unroll
+    for (int q = 0; q < 5; ++q) w[q] = R.bc_n1[q];
+  } else {
+    for (int d = 0; d < P.sd; ++d)
+      if (!P.periodic[d]) x[d] = min(max(x[d], R.dlo[d]), R.dhi[d]);
+    const long long from = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]) + s * cs;
+#pragma unroll
+    for (int q = 0; q < 5; ++q) w[q] = W[from + q * cs];
+  }
+  store_prim<5>(Ww, Wf, base + s * cs, cs, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -175,25 +158,20 @@ __global__ void __launch_bounds__(256)
 }  // namespace
 
 cudaError_t launch_farfield(const DevParams& P, const double* u, double* w, float* wf,
-                            const FarReg* far, int nfar, const RunParams* runs, int have_w,
-                            cudaStream_t s) {
+                            const FarReg* far, int nfar, int most, const RunParams* runs,
+                            int write_w, cudaStream_t s) {
   if (nfar <= 0) return cudaSuccess;
-  if (P.glm)
-    k_farfield<1><<<nfar, 256, 0, s>>>(P, u, w, wf, far, runs, have_w);
-  else
-    k_farfield<0><<<nfar, 256, 0, s>>>(P, u, w, wf, far, runs, have_w);
+  const dim3 grid(nfar, P.nf, (most + 255) / 256);
+  k_farfield<<<grid, 256, 0, s>>>(P, u, w, wf, far, runs, write_w);
   return cudaGetLastError();
 }
 
 cudaError_t launch_prim(const DevParams& P, const double* uin, double* w, const Batch& b,
-                        cudaStream_t s, float* wf) {
+                        cudaStream_t s, float* wf, StepState* state, double dt_scale) {
   if (b.tot_w <= 0) return cudaSuccess;
   const int nt = b.nt[0];
-  const unsigned gw = flat_blocks(b.tot_w, nt);
-  if (P.glm)
-    k_prim<1><<<gw, nt, 0, s>>>(P, uin, w, wf, b.desc, b.ndesc, b.tot_w, b.runs);
-  else
-    k_prim<0><<<gw, nt, 0, s>>>(P, uin, w, wf, b.desc, b.ndesc, b.tot_w, b.runs);
+  const dim3 grid(flat_blocks(b.tot_w, nt), P.nf);
+  k_prim<<<grid, nt, 0, s>>>(P, uin, w, wf, b.desc, b.ndesc, b.tot_w, b.runs, state, dt_scale);
   return cudaGetLastError();
 }
 

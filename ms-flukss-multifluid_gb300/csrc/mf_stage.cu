@@ -44,7 +44,7 @@ cudaError_t launch_stage(const DevParams& P, int precision, const StageBuffers& 
     // primitive state of the valid cells, the siblings' copies into the
     // ghost layers, then the far-field ghosts (which read the copies)
     const LeanPrim& L = *B.lean;
-    e = launch_prim(P, B.uin, B.w, *L.prim, s, wf);
+    e = launch_prim(P, B.uin, B.w, *L.prim, s, wf, state, dt_scale);
     if (e != cudaSuccess) return e;
     if (B.ev) cudaEventRecord(B.ev[ne++], s);
     if (L.nregs && L.exchange_w) {
@@ -58,12 +58,12 @@ cudaError_t launch_stage(const DevParams& P, int precision, const StageBuffers& 
       if (B.ev) cudaEventRecord(B.ev[ne++], s);
     }
     if (L.nfar) {
-      e = launch_farfield(P, B.uin, B.w, wf, L.far, L.nfar, b.runs, L.exchange_w, s);
+      e = launch_farfield(P, B.uin, B.w, wf, L.far, L.nfar, L.far_cells, b.runs, L.exchange_w, s);
       if (e != cudaSuccess) return e;
       if (B.ev) cudaEventRecord(B.ev[ne++], s);
     }
   } else {
-    e = launch_prim(P, B.uin, B.w, b, s, wf);
+    e = launch_prim(P, B.uin, B.w, b, s, wf, state, dt_scale);
     if (e != cudaSuccess) return e;
     if (B.ev) cudaEventRecord(B.ev[ne++], s);
   }

@@ -54,7 +54,8 @@ __device__ __forceinline__ bool part_less(const DtPartial& a, const DtPartial& b
 // One block per run: the minimum over the run's block partials, the run's
 // time after the step, then (advance) its next dt and GLM speeds
 // (AMRLevelIdealMHD::advance, srcIdeal/AMRLevelIdealMHD.cpp:1531-1548, 1588).
-__global__ void __launch_bounds__(256)
+constexpr int kFinalThreads = 1024;
+__global__ void __launch_bounds__(kFinalThreads)
     k_finalize(const __grid_constant__ DevParams P, const DtPartial* __restrict__ parts,
                const RunParams* __restrict__ runs, int nt, StepState* __restrict__ states,
                int advance, int nparts) {
@@ -66,20 +67,34 @@ __global__ void __launch_bounds__(256)
   best.dt = DBL_MAX;
   best.desc = INT_MAX;
   best.idx = INT_MAX;
-  for (int q = p0 + threadIdx.x; q < p1; q += blockDim.x) {
-    DtPartial c = parts[q];
-    if (part_less(c, best)) best = c;
+  // one block reads all of a run's partials: latency, so four loads in flight
+  for (int q = p0 + threadIdx.x; q < p1; q += 4 * kFinalThreads) {
+    DtPartial c[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (q + j * kFinalThreads < p1) c[j] = parts[q + j * kFinalThreads];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (q + j * kFinalThreads < p1 && part_less(c[j], best)) best = c[j];
   }
-  __shared__ DtPartial sb[256];
-  sb[threadIdx.x] = best;
+  auto take_min = [&best]() {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      DtPartial c;
+      c.dt = __shfl_down_sync(0xffffffffu, best.dt, off);
+      c.desc = __shfl_down_sync(0xffffffffu, best.desc, off);
+      c.idx = __shfl_down_sync(0xffffffffu, best.idx, off);
+      if (part_less(c, best)) best = c;
+    }
+  };
+  __shared__ DtPartial sb[kFinalThreads / 32];
+  take_min();
+  if ((threadIdx.x & 31) == 0) sb[threadIdx.x >> 5] = best;
   __syncthreads();
-  for (int s = 128; s > 0; s >>= 1) {
-    if (threadIdx.x < s && part_less(sb[threadIdx.x + s], sb[threadIdx.x]))
-      sb[threadIdx.x] = sb[threadIdx.x + s];
-    __syncthreads();
-  }
+  if (threadIdx.x >= 32) return;
+  best = sb[threadIdx.x];
+  take_min();
   if (threadIdx.x == 0) {
-    best = sb[0];
     ss->dt_min = best.dt;
     ss->min_desc = (best.desc == INT_MAX) ? INT_MAX : best.desc - R.d0;
     ss->min_idx = best.idx;
@@ -111,47 +126,47 @@ template <> struct Vec<float, 4> { using type = float4; };
 template <> struct Vec<double, 2> { using type = double2; };
 template <typename T> struct Vec<T, 1> { using type = T; };
 
-// The copy of one region's components in vectors of V elements along x (V
-// divides the region's x extent, and every row starts on a multiple of V).
-// Flat over the (component, vector) items so that small regions still occupy
-// the block; 32-bit index arithmetic (a region is part of one patch's ghost
-// layers: 2^31 elements would take a patch whose fab alone exceeds HBM); four
-// loads in flight per thread before their stores.
+// The copy of one region's components (every gridDim.y-th) in vectors of V
+// elements along x (V divides the region's x extent, and every row starts on a
+// multiple of V).  A thread finds its vector's place once and then steps
+// through the components, eight loads in flight before their stores; in a
+// region of fewer vectors than the block's threads, groups of threads take
+// different components.
 template <typename T, int V>
 __device__ __forceinline__ void copy_region(T* __restrict__ U, const CopyReg& R, int nc,
                                             long long scs, long long dcs) {
   using VT = typename Vec<T, V>::type;
+  constexpr int kFlight = 8;
   const int rowv = R.ext[0] / V;
   const int n = rowv * R.ext[1] * R.ext[2];
-  const int tot = n * nc;
-  const int step = blockDim.x;
-  for (int t0 = threadIdx.x; t0 < tot; t0 += 4 * step) {
-    VT v[4];
-    long long dof[4];
+  const int nt = blockDim.x, groups = n < nt ? nt / n : 1;
+  const int grp = groups > 1 ? (int)threadIdx.x / n : 0;
+  if (grp >= groups) return;
+  const int step = groups * gridDim.y;
+  for (int c = (int)threadIdx.x - grp * n; c < n; c += nt) {
+    const int a = c % rowv;
+    const int r = c / rowv;
+    const int b = r % R.ext[1];
+    const int e = r / R.ext[1];
+    const T* src = U + R.src_off + (R.s0[0] + a * V) +
+                   (long long)R.sfn[0] * ((R.s0[1] + b) + (long long)R.sfn[1] * (R.s0[2] + e));
+    T* dst = U + R.dst_off + (R.d0[0] + a * V) +
+             (long long)R.dfn[0] * ((R.d0[1] + b) + (long long)R.dfn[1] * (R.d0[2] + e));
+    for (int q0 = grp + groups * blockIdx.y; q0 < nc; q0 += kFlight * step) {
+      VT v[kFlight];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int t = t0 + j * step;
-      if (t < tot) {
-        const int q = t / n;
-        const int c = t - q * n;
-        const int a = c % rowv;
-        const int r = c / rowv;
-        const int b = r % R.ext[1];
-        const int e = r / R.ext[1];
-        const long long so = R.src_off + q * scs + (R.s0[0] + a * V) +
-                             (long long)R.sfn[0] * ((R.s0[1] + b) + (long long)R.sfn[1] * (R.s0[2] + e));
-        dof[j] = R.dst_off + q * dcs + (R.d0[0] + a * V) +
-                 (long long)R.dfn[0] * ((R.d0[1] + b) + (long long)R.dfn[1] * (R.d0[2] + e));
-        v[j] = __ldg(reinterpret_cast<const VT*>(U + so));
-      }
+      for (int j = 0; j < kFlight; ++j)
+        if (q0 + j * step < nc)
+          v[j] = __ldg(reinterpret_cast<const VT*>(src + (q0 + j * step) * scs));
+#pragma unroll
+      for (int j = 0; j < kFlight; ++j)
+        if (q0 + j * step < nc) *reinterpret_cast<VT*>(dst + (q0 + j * step) * dcs) = v[j];
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (t0 + j * step < tot) *reinterpret_cast<VT*>(U + dof[j]) = v[j];
+    if (groups > 1) break;  // n < nt: one vector per thread
   }
 }
 
-// One block per copy region.  Sources are valid cells and destinations ghost
+// One copy region per blockIdx.x.  Sources are valid cells and destinations ghost
 // cells, never the same, so the sources are read through the read-only path.
 // Rows are copied in 16-byte vectors where the region's x extent, its rows'
 // starts and the fabs' strides are multiples of the vector (the fabs start on
@@ -241,20 +256,30 @@ cudaError_t launch_dt(const DevParams& P, const double* u, const Batch& b, DtPar
 cudaError_t launch_finalize(const DevParams& P, const DtPartial* partials, const Batch& b,
                             int nt, StepState* state, int advance, cudaStream_t s, int nparts) {
   if (b.nruns <= 0) return cudaSuccess;
-  k_finalize<<<nparts > 0 ? 1 : b.nruns, 256, 0, s>>>(P, partials, b.runs, nt, state, advance,
+  k_finalize<<<nparts > 0 ? 1 : b.nruns, kFinalThreads, 0, s>>>(P, partials, b.runs, nt, state, advance,
                                                      nparts);
   return cudaGetLastError();
 }
 
+// Blocks per region: the components are shared out until `per_sm` blocks of
+// 256 threads fall on an SM.  FP64 copies are bound by the latency of their
+// loads and take many blocks (128^3: 2 per SM 0.66 ms a step with the far-field
+// fill, 60 per SM 0.55); FP32 ones, half the bytes, lose more to the repeated
+// set-up (0.57 against 0.59).
+static unsigned exchange_split(int nreg, int nc, int per_sm) {
+  const int want = (per_sm * 152 + nreg - 1) / nreg;
+  return (unsigned)(want < 1 ? 1 : want > nc ? nc : want);
+}
+
 cudaError_t launch_exchange(double* u, const CopyReg* regs, int nreg, int nc, cudaStream_t s) {
   if (nreg <= 0) return cudaSuccess;
-  k_exchange<double><<<nreg, 256, 0, s>>>(u, regs, nc);
+  k_exchange<double><<<dim3(nreg, exchange_split(nreg, nc, 60)), 256, 0, s>>>(u, regs, nc);
   return cudaGetLastError();
 }
 
 cudaError_t launch_exchange_f(float* u, const CopyReg* regs, int nreg, int nc, cudaStream_t s) {
   if (nreg <= 0) return cudaSuccess;
-  k_exchange<float><<<nreg, 256, 0, s>>>(u, regs, nc);
+  k_exchange<float><<<dim3(nreg, exchange_split(nreg, nc, 2)), 256, 0, s>>>(u, regs, nc);
   return cudaGetLastError();
 }
 

@@ -75,8 +75,8 @@ __device__ __forceinline__ void block_dt_min(double dtc, int myidx,
       myidx = oi;
     }
   }
-  constexpr int kWarps = kCellBlock * MF_MAX_FLUIDS / 32;  // the largest block
-  static_assert(kWarps >= kMaxBlock / 32, "a slot per warp");
+  constexpr int kMost = kCellBlock * MF_MAX_FLUIDS > kMaxBlock ? kCellBlock * MF_MAX_FLUIDS : kMaxBlock;
+  constexpr int kWarps = kMost / 32;  // of the largest block
   __shared__ double sdt[kWarps];
   __shared__ int sidx[kWarps];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -105,26 +105,6 @@ __device__ __forceinline__ void block_dt_min(double dtc, int myidx,
     }
     partials[slot] = pr;
   }
-}
-
-// GLM damping factor exp(-dt Ch^2 / Cp^2) of PSIPARABOLIC (src/DednerF.ChF:
-// 65-87) for the run of the calling warp: one evaluation per warp instead of
-// one per cell (the same expression on the same values), by the first lane
-// with a cell, broadcast by shuffle.  A warp never holds cells of two runs
-// (each run's cells start on a multiple of kRunAlign); every lane calls.
-__device__ __forceinline__ double warp_psi_damping(const StageDesc* Dp,
-                                                   const StepState* __restrict__ states,
-                                                   double dt_scale) {
-  const unsigned m = __ballot_sync(0xffffffffu, Dp != nullptr);
-  if (!m) return 1.0;
-  const int src = __ffs(m) - 1;
-  double v = 1.0;
-  if ((int)(threadIdx.x & 31) == src) {
-    const StepState& S = states[Dp->run];
-    const double dt = S.dt * dt_scale;
-    v = exp(-dt * S.ch * S.ch / (S.cp * S.cp));
-  }
-  return __shfl_sync(0xffffffffu, v, src);
 }
 
 // The stage-start primitive state of a cell as the update tail reads it:
@@ -241,7 +221,7 @@ __device__ __forceinline__ void update_cells(const DevParams& P, const StageBuff
     lin = g - Dp->g0[kRegV];
     if (lin >= Dp->vn[0] * Dp->vn[1] * Dp->vn[2]) Dp = nullptr;  // run-alignment gap
   }
-  const double psi_damp = GLM ? warp_psi_damping(Dp, states, dt_scale) : 1.0;
+  const double psi_damp = (GLM && Dp) ? states[Dp->run].damp : 1.0;
   if (Dp) {
     const StageDesc& D = *Dp;
     const RunParams& RP = runs[D.run];
