@@ -241,6 +241,10 @@ DevParams make_dev(const mf_params& p) {
   P.smallp = p.smallp;
   P.del2 = p.entropy_fix;
   P.smallB = p.small_b;
+  P.smallB2 = p.small_b * p.small_b;
+  P.r0_2 = p.reinit_r0 * p.reinit_r0;
+  P.sun_r2 = p.sun_r * p.sun_r;
+  P.lim_sun = 0.6 * p.sun_v;
   P.dx = p.dx;
   P.invdx = 1.0 / p.dx;
   P.factor_ch = p.factor_ch;

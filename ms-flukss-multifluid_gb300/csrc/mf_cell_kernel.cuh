@@ -1,5 +1,6 @@
-// mf_cell_kernel.cuh - the update kernel with one thread per cell and fluid.  Included by mf_cell_exact.cu (parity physics) and
-// mf_cell.cu (fast physics); MF_PHYS names the physics namespace.
+// mf_cell_kernel.cuh - the update kernel with one thread per cell and fluid.
+// Included by mf_cell_exact.cu (parity physics) and mf_cell.cu (fast physics);
+// MF_PHYS names the physics namespace, MF_CELL_REGS the registers per thread.
 //
 // Bound by the FP64 pipe while enough warps are resident.  With one thread
 // per cell a whole cell's state, its sources and their temporaries took 222
@@ -23,21 +24,17 @@ using namespace MF_PHYS;
 
 constexpr int kCells = kCellBlock;
 
-#ifndef MF_CELL_REGS
-#define MF_CELL_REGS 128
-#endif
 constexpr int cell_blocks(int nf) { return 65536 / (MF_CELL_REGS * kCells * nf); }
 
-// R: type of the face fluxes and wave speeds; T: type of the charge-exchange rates.
-template <int NF, typename R, typename T>
+// R: type of the face fluxes and wave speeds.
+template <int NF, typename R>
 __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     k_cells(const __grid_constant__ DevParams P, const __grid_constant__ StageBuffers B,
             const StageDesc* __restrict__ descs, int ndesc, int total, int flags,
             const RunParams* __restrict__ runs, StepState* __restrict__ states,
             const double dt_scale, DtPartial* __restrict__ partials) {
   constexpr int NN = NF - 1;
-  using Terms = CeTermsT<T>;
-  __shared__ T terms[NN > 0 ? NN : 1][Terms::kShared][kCells];
+  __shared__ double terms[NN > 0 ? NN : 1][CeTerms::kShared][kCells];
   __shared__ R speed[NF][kCells];
   __shared__ int region[kCells];
   const int role = threadIdx.x / kCells, lane = threadIdx.x % kCells;  // role 0: the plasma
@@ -54,15 +51,15 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
   const int s = plasma ? 0 : P.irhon + (role - 1) * 5;  // first component of the thread's fluid
   int i = 0, j = 0, k = 0;
   long long cs = 0, base = 0;
-  double dt = 0.0, u[9];
-  Terms t;
+  double dt = 0.0, r2 = -1.0, u[9];
+  CeTerms t;
   if (Dp) {
     const StageDesc& D = *Dp;
     const RunParams& RP = runs[D.run];
     decode(lin, D.vlo, D.vn, i, j, k);
     cs = (long long)D.fn[0] * D.fn[1] * D.fn[2];
     base = D.u_off + loc(D.flo, D.fn, i, j, k);
-    dt = states[D.run].dt * dt_scale;
+    dt = dt_scale == 1.0 ? states[D.run].dt : states[D.run].dt * dt_scale;
     const double dtinv = dt * RP.invdx;
     const WColumn w{B.w + base, cs};
 #pragma unroll
@@ -112,11 +109,11 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
         if ((flags & kStageDt) && B.divb) B.divb[loc(B.divb_lo, B.divb_n, i, j, k)] = divB;
       }
       if (P.glm) u[8] = states[D.run].damp * u[8];  // PSIPARABOLIC (src/DednerF.ChF:65-87)
-      if (ce) region[lane] = region_cell(P, RP.dx, i, j, k, w, 0.0);
+      if (ce) region[lane] = region_cell(P, RP.dx, i, j, k, w, 0.0, r2);
     } else if (ce) {
-      charge_exchange_terms<T>(P, w, s, t);
+      charge_exchange_terms(P, w, s, t);
 #pragma unroll
-      for (int q = 0; q < Terms::kShared; ++q) terms[role - 1][q][lane] = t.shared[q];
+      for (int q = 0; q < CeTerms::kShared; ++q) terms[role - 1][q][lane] = t.shared[q];
     }
   }
   if (ce) __syncthreads();
@@ -128,17 +125,17 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
     // the recalculation of B
     if (plasma) {
       if constexpr (NN > 0) {
-        if (ce) charge_exchange_plasma<NN, T>(dt, u, at);
+        if (ce) charge_exchange_plasma<NN>(dt, u, at);
       }
       if (!P.ct) {
-        if (P.reinit) reinit_plasma(P, runs[Dp->run].dx, i, j, k, stage_time(states[Dp->run], dt), u);
+        if (P.reinit) reinit_plasma(P, runs[Dp->run].dx, i, j, k, stage_time(states[Dp->run], dt), r2, u);
         positivity_plasma(P, u);
       }
     } else {
       if constexpr (NN > 0) {
         if (ce) {
           const bool rec = ce_recipient(NN, region[lane]) == role;
-          charge_exchange_neutral<NN, T>(rec, role - 1, WColumn{B.w + base, cs}, t, dt, u, at);
+          charge_exchange_neutral<NN>(rec, role - 1, WColumn{B.w + base, cs}, t, dt, u, at);
         }
       }
       if (!P.ct) positivity_neutral(P, role, u);
@@ -173,7 +170,7 @@ __global__ void __launch_bounds__(kCells* NF, cell_blocks(NF))
   }
 }
 
-template <typename R, typename T>
+template <typename R>
 cudaError_t launch_cells_t(const DevParams& P, const StageBuffers& B, const Batch& b,
                                   int flags, double dt_scale, StepState* state,
                                   DtPartial* partials, int* nblocks_v, cudaStream_t s) {
@@ -181,7 +178,7 @@ cudaError_t launch_cells_t(const DevParams& P, const StageBuffers& B, const Batc
   if (nblocks_v) *nblocks_v = (int)nb;
   if (b.tot_v <= 0) return cudaSuccess;
 #define MF_CELLS(NF)                                                                             \
-  k_cells<NF, R, T><<<nb, kCells * NF, 0, s>>>(P, B, b.desc, b.ndesc, b.tot_v, flags, b.runs, \
+  k_cells<NF, R><<<nb, kCells * NF, 0, s>>>(P, B, b.desc, b.ndesc, b.tot_v, flags, b.runs, \
                                                state, dt_scale, partials)
   switch (P.nf) {
     case 1: MF_CELLS(1); break;

@@ -53,6 +53,8 @@ struct DevParams {
   double max_growth;          // assignDt growth cap of chained time steps (<= 0: none)
   double bc_plasma[8], bc_n1[5];
   double lism_u[3];
+  // products of the above that every face or cell would form again
+  double smallB2, r0_2, sun_r2, lim_sun;
 };
 
 // Values that change from step to step; kept in device memory so that a
@@ -144,6 +146,16 @@ __device__ __host__ __forceinline__ ReinitIn reinit_in(const DevParams& P) {
   r.cos_tilt = P.cos_tilt;
   r.monopolar = P.monopolar;
   return r;
+}
+
+// Cell centre i + 1/2, exactly, on the integer pipes.
+__device__ __forceinline__ double cell_centre(int i) {
+  const int n = 2 * i + 1;
+  const uint32_t m = (uint32_t)(n < 0 ? -n : n);
+  const int k = 31 - __clz((int)m);  // m = 2^k + ...
+  const uint64_t f = (uint64_t)m << (52 - k);
+  return ieee64::pack(((uint32_t)(f >> 32) + ((uint32_t)(1021 + k) << 20)) | ((uint32_t)n & 0x80000000u),
+                      (uint32_t)f);
 }
 
 // sin and cos of a phase through sincospi(phase / pi) on the device (exact

@@ -347,9 +347,10 @@ inline unsigned flat_blocks(long long n, int nt) {
 }
 
 // The update with a thread per cell and fluid (mf_cell_kernel.cuh; blocks of
-// kCellBlock cells): every option but tracking surfaces.
+// kCellBlock cells): every option but tracking surfaces and FP32
+// charge-exchange rates (charge_exchange_add_32).
 constexpr int kCellBlock = 64;
-inline bool update_by_fluid(const DevParams& P) { return P.nls == 0; }
+inline bool update_by_fluid(const DevParams& P) { return P.nls == 0 && !P.ce32; }
 template <typename R>
 cudaError_t launch_cells_fast(const DevParams& P, const StageBuffers& B, const Batch& b,
                               int flags, double dt_scale, StepState* state,

@@ -129,8 +129,7 @@ __device__ __forceinline__ void roe_mhd(const DevParams& P, const R* wl, const R
   const double c = root(cc);
 
   double hyy, hzz, aaf, aas, af, as;
-  const double smallB = P.smallB;
-  if (lt(BYZ2, smallB * smallB)) {
+  if (lt(BYZ2, P.smallB2)) {
     hyy = sq2;
     hzz = sq2;
     const bool alfven = lt(cc, bb);

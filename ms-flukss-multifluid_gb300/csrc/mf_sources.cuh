@@ -69,38 +69,41 @@ __device__ __forceinline__ int region_tracer_cell(const DevParams& P, double dx,
 // DEFINE_REGIONS_2F (swlism/SWLISMF.ChF:654-742), Cartesian branch, or the
 // tracer variant above (HeliosphericProblem::defineRegions,
 // swlism/HeliosphericProblem.cpp:2538-2575).
+// r2: receives the squared distance to the sun.
 template <typename WA>
 __device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i, int j, int k,
-                                           const WA& w, double regtr) {
-  if (P.reg_tracer) return region_tracer_cell(P, dx, i, j, k, w, regtr);
-  const double x = __dadd_rn(__dmul_rn(i + 0.5, dx), -P.sun_c[0]);
-  const double y = __dadd_rn(__dmul_rn(j + 0.5, dx), -P.sun_c[1]);
-  double z = 0.0, r2, invr, ur;
+                                           const WA& w, double regtr, double& r2) {
+  using namespace ieee64;
+  const double x = __dadd_rn(__dmul_rn(cell_centre(i), dx), -P.sun_c[0]);
+  const double y = __dadd_rn(__dmul_rn(cell_centre(j), dx), -P.sun_c[1]);
+  double z = 0.0;
+  r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
   if (P.sd == 3) {
-    z = __dadd_rn(__dmul_rn(k + 0.5, dx), -P.sun_c[2]);
-    r2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
-    invr = __ddiv_rn(1.0, __dsqrt_rn(r2));
-    ur = __dadd_rn(__dadd_rn(__dmul_rn(w[1], __dmul_rn(x, invr)), __dmul_rn(w[2], __dmul_rn(y, invr))),
-                   __dmul_rn(w[3], __dmul_rn(z, invr)));
-  } else {
-    r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
-    invr = __ddiv_rn(1.0, __dsqrt_rn(r2));
-    ur = __dadd_rn(__dmul_rn(w[1], __dmul_rn(x, invr)), __dmul_rn(w[2], __dmul_rn(y, invr)));
+    z = __dadd_rn(__dmul_rn(cell_centre(k), dx), -P.sun_c[2]);
+    r2 = __dadd_rn(r2, __dmul_rn(z, z));
   }
-  const double TEMP = __ddiv_rn(__dmul_rn(P.t_coeff, w[4]), w[0]);
-  const double LIMSUN = __dmul_rn(0.6, P.sun_v);
-  const double sunR2 = __dmul_rn(P.sun_r, P.sun_r);
-  const bool zout = (P.sd == 3) && ((z < P.zbot) || (z > P.ztop));
+  if (P.reg_tracer) return region_tracer_cell(P, dx, i, j, k, w, regtr);
+  const double invr = div(1.0, root(r2));
+  double ur = __dadd_rn(__dmul_rn(w[1], __dmul_rn(x, invr)), __dmul_rn(w[2], __dmul_rn(y, invr)));
+  if (P.sd == 3) ur = __dadd_rn(ur, __dmul_rn(w[3], __dmul_rn(z, invr)));
+  const double TEMP = div(__dmul_rn(P.t_coeff, w[4]), w[0]);
+  const bool zout = (P.sd == 3) && (lt(z, P.zbot) || lt(P.ztop, z));
   int reg;
-  if (fabs(ur) >= LIMSUN) {
-    reg = ((TEMP >= 1.0e6) && (r2 > sunR2)) ? 2 : 3;
+  if (le(P.lim_sun, absval(ur))) {
+    reg = (le(1.0e6, TEMP) && lt(P.sun_r2, r2)) ? 2 : 3;
     if (zout) reg = 1;
-  } else if (TEMP >= P.tmlim) {
+  } else if (le(P.tmlim, TEMP)) {
     reg = zout ? 1 : 2;
   } else {
     reg = 1;
   }
   return reg;
+}
+template <typename WA>
+__device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i, int j, int k,
+                                           const WA& w, double regtr) {
+  double r2;
+  return region_cell(P, dx, i, j, k, w, regtr, r2);
 }
 
 // Recipient of newly created neutrals: CHARGE_EXCHANGE_2F/3F/4F/MF
@@ -118,21 +121,11 @@ __device__ __forceinline__ int ce_recipient(int nN, int reg) {
 // The FP64 forms take division and square root from the integer pipes
 // (mf_ieee64.cuh) and the logarithm of mf_fp64.cuh.  Products and sums are
 // written as fused operations (mad), or the product by prod() where it must
-// not fuse, so that every kernel that inlines these routines rounds alike.  The state update itself is
-// FP64 either way.
+// not fuse, so that every kernel that inlines these routines rounds alike.
+// The state update itself is FP64 either way.
 __device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float mad(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ double prod(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float prod(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double quotient(double a, double b) { return ieee64::div(a, b); }
-__device__ __forceinline__ float quotient(float a, float b) { return a * (1.0f / b); }
-// sqrt(x) and a / sqrt(x) for x > 0
-__device__ __forceinline__ double root_of(double x) { return ieee64::root(x); }
-__device__ __forceinline__ float root_of(float x) { return x * rsqrtf(x); }
-__device__ __forceinline__ double over_root(double a, double x) {
-  return ieee64::div(a, ieee64::root(x));
-}
-__device__ __forceinline__ float over_root(float a, float x) { return a * rsqrtf(x); }
 template <int K>
 __device__ __forceinline__ double pow2(double x) { return ieee64::scale<K>(x); }
 template <int K>
@@ -157,52 +150,51 @@ __device__ __forceinline__ double to_d(double x) { return x; }
 // Pauls & Zank charge exchange of the plasma with one neutral population
 // (HeliosphericProblem::explicitSource, swlism/HeliosphericProblem.cpp:1394-1539,
 // CHARGE_EXCHANGE_4F swlism/ChargeExchange2F.ChF:673-993 and _MF :995-1149).
-// T: arithmetic type of the rates.  The products ARR UD, ARR VVTHU and
-// ARR VP_UHM that several terms share are formed once; the plasma's terms
-// that carry a cell factor (ux, U2/2) are summed without it and scaled after
-// the sum: the reference's H in another order.
-template <typename T>
-struct CeTermsT {
+// FP64 rates.  The products ARR UD, ARR VVTHU and ARR VP_UHM that several
+// terms share are formed once; the plasma's terms that carry a cell factor
+// (ux, U2/2) are summed without it and scaled after the sum: the reference's
+// H in another order.
+struct CeTerms {
   static constexpr int kShared = 9;
   // what the plasma sums over the populations: h2..h4, the S of PPLUX..Z,
   // ARR UD (-DENPLU), G (in the energy source and the recipient's energy
   // gain) and the rest of h5
-  T shared[kShared];
-  T own[4];  // PMIX, PMIY, PMIZ, ENMI
+  double shared[kShared];
+  double own[4];  // PMIX, PMIY, PMIZ, ENMI
 };
-using CeTerms = CeTermsT<double>;
 
 // w: the stage-start primitive state; o: the population's first component
-template <typename T, typename WA>
+template <typename WA>
 __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const WA& w, int o,
-                                                      CeTermsT<T>& c) {
-  constexpr T c4p = T(4.0 * kInvPi), c16p = T(16.0 * kInvPi), c94pi = T(2.25 * kPi);
-  constexpr T c649ip = T(64.0 / 9.0 * kInvPi);
-  const T rho = to_t<T>(w[0]), ux = to_t<T>(w[1]), uy = to_t<T>(w[2]), uz = to_t<T>(w[3]);
-  const T rhoN = to_t<T>(w[o]), uxN = to_t<T>(w[o + 1]), uyN = to_t<T>(w[o + 2]), uzN = to_t<T>(w[o + 3]);
-  const T VVTP = quotient(to_t<T>(w[4]), rho);
-  const T VVTH = quotient(pow2<1>(to_t<T>(w[o + 4])), rhoN);
-  const T dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
-  const T hU2 = pow2<-1>(mad(uz, uz, mad(uy, uy, ux * ux)));
-  const T hUH2 = pow2<-1>(mad(uzN, uzN, mad(uyN, uyN, uxN * uxN)));
-  const T DU2 = mad(dz_, dz_, mad(dy_, dy_, dx_ * dx_)), DU24 = pow2<2>(DU2);
-  const T VPHH = mad(dz_, uzN, mad(dy_, uyN, dx_ * uxN));
-  const T VPHP = mad(dz_, uz, mad(dy_, uy, dx_ * ux));
+                                                      CeTerms& c) {
+  using namespace ieee64;
+  constexpr double c4p = 4.0 * kInvPi, c16p = 16.0 * kInvPi, c94pi = 2.25 * kPi;
+  constexpr double c649ip = 64.0 / 9.0 * kInvPi;
+  const double rho = w[0], ux = w[1], uy = w[2], uz = w[3];
+  const double rhoN = w[o], uxN = w[o + 1], uyN = w[o + 2], uzN = w[o + 3];
+  const double VVTP = div(w[4], rho);
+  const double VVTH = div(scale<1>(w[o + 4]), rhoN);
+  const double dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
+  const double hU2 = half(mad(uz, uz, mad(uy, uy, ux * ux)));
+  const double hUH2 = half(mad(uzN, uzN, mad(uyN, uyN, uxN * uxN)));
+  const double DU2 = mad(dz_, dz_, mad(dy_, dy_, dx_ * dx_)), DU24 = scale<2>(DU2);
+  const double VPHH = mad(dz_, uzN, mad(dy_, uyN, dx_ * uxN));
+  const double VPHP = mad(dz_, uz, mad(dy_, uy, dx_ * ux));
   // thermal + relative speeds; every radicand is > 0
-  const T UD = root_of(mad(c4p, VVTH, mad(c4p, VVTP, DU2)));
-  const T VVTHU = over_root(VVTH, mad(c94pi, VVTH, mad(c16p, VVTP, DU24)));
-  const T VP_UHM = over_root(VVTP, mad(c16p, VVTH, mad(c94pi, VVTP, DU24)));
-  const T UPE = root_of(mad(c649ip, VVTH, mad(c4p, VVTP, DU2)));
-  const T UHE = root_of(mad(c4p, VVTH, mad(c649ip, VVTP, DU2)));
-  const T UDS = to_t<T>(P.ce_scale_vel) * UD;
-  const T t = mad(-to_t<T>(P.ce_b), ce_log(UDS), to_t<T>(P.ce_a));
-  T SIG = t * t;
-  const T damp_c = to_t<T>(P.ce_damp_c);
-  if (damp_c > T(0)) SIG = SIG * ce_pow(T(1) - ce_exp(-damp_c / UDS), to_t<T>(P.ce_damp_pow));
-  const T ARR = SIG * (rhoN * (to_t<T>(P.ce_sigma_scale) * rho));
-  const T aU = prod(ARR, UD), aT = prod(ARR, VVTHU), aV = prod(ARR, VP_UHM);
-  const T Y = T(0.75) * ((ARR * UPE) * VVTH);
-  const T hv = aU + aT + aV;
+  const double UD = root(mad(c4p, VVTH, mad(c4p, VVTP, DU2)));
+  const double VVTHU = div(VVTH, root(mad(c94pi, VVTH, mad(c16p, VVTP, DU24))));
+  const double VP_UHM = div(VVTP, root(mad(c16p, VVTH, mad(c94pi, VVTP, DU24))));
+  const double UPE = root(mad(c649ip, VVTH, mad(c4p, VVTP, DU2)));
+  const double UHE = root(mad(c4p, VVTH, mad(c649ip, VVTP, DU2)));
+  const double UDS = P.ce_scale_vel * UD;
+  const double t = mad(-P.ce_b, ce_log(UDS), P.ce_a);
+  double SIG = t * t;
+  const double damp_c = P.ce_damp_c;
+  if (damp_c > 0.0) SIG = SIG * ce_pow(1.0 - ce_exp(-damp_c / UDS), P.ce_damp_pow);
+  const double ARR = SIG * (rhoN * (P.ce_sigma_scale * rho));
+  const double aU = prod(ARR, UD), aT = prod(ARR, VVTHU), aV = prod(ARR, VP_UHM);
+  const double Y = 0.75 * ((ARR * UPE) * VVTH);
+  const double hv = aU + aT + aV;
   c.shared[0] = prod(hv, dx_);
   c.shared[1] = prod(hv, dy_);
   c.shared[2] = prod(hv, dz_);
@@ -210,7 +202,7 @@ __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const 
   c.shared[4] = prod(aV, dy_);
   c.shared[5] = prod(aV, dz_);
   c.shared[6] = aU;
-  c.shared[7] = mad(aV, VPHP, (T(0.75) * VVTP) * (ARR * UHE));
+  c.shared[7] = mad(aV, VPHP, (0.75 * VVTP) * (ARR * UHE));
   c.shared[8] = mad(aT, VPHH, mad(aU, hU2 - hUH2, -Y));
   c.own[0] = mad(uxN, aU, -(dx_ * aT));
   c.own[1] = mad(uyN, aU, -(dy_ * aT));
@@ -220,60 +212,157 @@ __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const 
 
 // S = -dt H of the plasma (momentum and energy; the magnetic field's and
 // psi's S is zero) from the sums over the populations, sum[q] of shared[q].
-template <typename T>
-__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const T* sum) {
+__device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const double* sum) {
 #pragma unroll
-  for (int q = 0; q < 3; ++q) u[1 + q] = fma(-dt, to_d(sum[q]), u[1 + q]);
-  u[4] = fma(-dt, to_d(sum[7] + sum[8]), u[4]);
+  for (int q = 0; q < 3; ++q) u[1 + q] = fma(-dt, sum[q], u[1 + q]);
+  u[4] = fma(-dt, sum[7] + sum[8], u[4]);
 }
 
 // S = -dt H of a population's own loss and gain
-template <typename T>
-__device__ __forceinline__ void charge_exchange_own(const CeTermsT<T>& c, double dt, double* un) {
-  un[0] = fma(-dt, to_d(c.shared[6]), un[0]);
+__device__ __forceinline__ void charge_exchange_own(const CeTerms& c, double dt, double* un) {
+  un[0] = fma(-dt, c.shared[6], un[0]);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) un[1 + q] = fma(-dt, to_d(c.own[q]), un[1 + q]);
+  for (int q = 0; q < 4; ++q) un[1 + q] = fma(-dt, c.own[q], un[1 + q]);
 }
 
 // The newly created neutrals that the recipient gains (its own loss, already
 // applied, cancels): from the sums; w: the plasma's primitive state.
-template <typename T, typename WA>
-__device__ __forceinline__ void charge_exchange_gain(const WA& w, const T* sum, double dt,
+template <typename WA>
+__device__ __forceinline__ void charge_exchange_gain(const WA& w, const double* sum, double dt,
                                                      double* un) {
-  const T ux = to_t<T>(w[1]), uy = to_t<T>(w[2]), uz = to_t<T>(w[3]), D = sum[6];
-  const T hU2 = pow2<-1>(mad(uz, uz, mad(uy, uy, ux * ux)));
-  un[0] = fma(dt, to_d(D), un[0]);
-  un[1] = fma(dt, to_d(mad(ux, D, sum[3])), un[1]);
-  un[2] = fma(dt, to_d(mad(uy, D, sum[4])), un[2]);
-  un[3] = fma(dt, to_d(mad(uz, D, sum[5])), un[3]);
-  un[4] = fma(dt, to_d(mad(hU2, D, sum[7])), un[4]);
+  const double ux = w[1], uy = w[2], uz = w[3], D = sum[6];
+  const double hU2 = ieee64::half(mad(uz, uz, mad(uy, uy, ux * ux)));
+  un[0] = fma(dt, D, un[0]);
+  un[1] = fma(dt, mad(ux, D, sum[3]), un[1]);
+  un[2] = fma(dt, mad(uy, D, sum[4]), un[2]);
+  un[3] = fma(dt, mad(uz, D, sum[5]), un[3]);
+  un[4] = fma(dt, mad(hU2, D, sum[7]), un[4]);
 }
 
 // The same for a thread per fluid; at(f, q): shared[q] of population f (from 0)
-template <int NN, typename T, typename AT>
-__device__ __forceinline__ void charge_exchange_sums(T* sum, const AT& at) {
+template <int NN, typename AT>
+__device__ __forceinline__ void charge_exchange_sums(double* sum, const AT& at) {
 #pragma unroll
-  for (int q = 0; q < CeTermsT<T>::kShared; ++q) {
+  for (int q = 0; q < CeTerms::kShared; ++q) {
     sum[q] = at(0, q);
 #pragma unroll
     for (int f = 1; f < NN; ++f) sum[q] = sum[q] + at(f, q);
   }
 }
-template <int NN, typename T, typename AT>
+template <int NN, typename AT>
 __device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at) {
-  T sum[CeTermsT<T>::kShared];
+  double sum[CeTerms::kShared];
   charge_exchange_sums<NN>(sum, at);
   charge_exchange_plasma(dt, u, sum);
 }
-template <int NN, typename T, typename WA, typename AT>
+template <int NN, typename WA, typename AT>
 __device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const WA& w,
-                                                        const CeTermsT<T>& c, double dt,
+                                                        const CeTerms& c, double dt,
                                                         double* un, const AT& at) {
   charge_exchange_own(c, dt, un);
   if (!rec) return;
-  T sum[CeTermsT<T>::kShared];
+  double sum[CeTerms::kShared];
   charge_exchange_sums<NN>(sum, at);
   charge_exchange_gain(w, sum, dt, un);
+}
+
+// All populations of one cell by one thread with FP32 rates
+// (MF_PREC_MIXED_CE32).  The update stays with one thread per cell there
+// (update_by_fluid): the sums over the populations fuse into running totals,
+// which a thread per population would round otherwise, and FP32 rounding of
+// the rates moves the state by more than any FP64 order of the sums does.
+template <int IRHON, typename WA, int NN>
+__device__ __forceinline__ void charge_exchange_add_32(const DevParams& P, const WA& w, int reg,
+                                                    double dt, double* u) {
+  using T = float;
+  const int nN = NN > 0 ? NN : P.nf - 1;
+  constexpr T c4p = T(4.0 * kInvPi), c16p = T(16.0 * kInvPi), c94pi = T(2.25 * kPi);
+  constexpr T c4ip = T(4.0 * kInvPi), c649ip = T(64.0 / 9.0 * kInvPi);
+  const T rho = to_t<T>(w[0]), ux = to_t<T>(w[1]), uy = to_t<T>(w[2]), uz = to_t<T>(w[3]);
+  const T U2 = ux * ux + uy * uy + uz * uz, hU2 = T(0.5) * U2;
+  const T VVTP = to_t<T>(w[4]) * (T(1) / rho);
+  // plasma thermal-speed terms of the five speed arguments
+  const T aUDp = c4p * VVTP, aUPMp = c16p * VVTP, aUHMp = c94pi * VVTP;
+  const T aPEp = c4ip * VVTP, aHEp = c649ip * VVTP, q75VP = T(0.75) * VVTP;
+  const T scale_vel = to_t<T>(P.ce_scale_vel), ce_a = to_t<T>(P.ce_a), ce_b = to_t<T>(P.ce_b);
+  const T damp_c = to_t<T>(P.ce_damp_c), damp_pow = to_t<T>(P.ce_damp_pow);
+  const T srho = to_t<T>(P.ce_sigma_scale) * rho;
+  // Each population's own loss / gain is applied inside the loop; the
+  // recipient of the newly created neutrals (region-dependent) then also
+  // receives the plasma's totals.  The products ARR*UD, ARR*VVTHU and
+  // ARR*VP_UHM that several terms share are formed once, and the plasma's
+  // terms that carry a cell factor (ux, U2/2, 3 VVTP/4) are summed without it
+  // and scaled after the loop: the reference's H, summed in another order.
+  // G: the sum of ARR (VPHP VP_UHM + 3 VVTP UHE / 4), which both the energy
+  // source and the recipient's energy gain hold; H5: the rest of h5.
+  T h2 = 0, h3 = 0, h4 = 0, DSUM = 0, S1x = 0, S1y = 0, S1z = 0, G = 0, H5 = 0;
+#pragma unroll
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
+    if (f > nN) break;
+    const int o = IRHON + (f - 1) * 5;
+    const T rhoN = to_t<T>(w[o]), uxN = to_t<T>(w[o + 1]), uyN = to_t<T>(w[o + 2]), uzN = to_t<T>(w[o + 3]);
+    const T dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
+    const T UH2 = uxN * uxN + uyN * uyN + uzN * uzN;
+    const T DU2 = dx_ * dx_ + dy_ * dy_ + dz_ * dz_, DU2x4 = T(4) * DU2;
+    const T VPHH = dx_ * uxN + dy_ * uyN + dz_ * uzN;
+    const T VPHP = dx_ * ux + dy_ * uy + dz_ * uz;
+    const T VVTH = T(2) * (to_t<T>(w[o + 4]) * (T(1) / rhoN));
+    // thermal + relative speeds; every argument is > 0, so sqrt(a) = a*rsqrt(a)
+    const T aUD = (aUDp + c4p * VVTH) + DU2;
+    const T UD = aUD * rsqrtf(aUD);
+    const T iUPM = rsqrtf((aUPMp + c94pi * VVTH) + DU2x4);
+    const T iUHM = rsqrtf((aUHMp + c16p * VVTH) + DU2x4);
+    const T aPE = (aPEp + c649ip * VVTH) + DU2;
+    const T UPE = aPE * rsqrtf(aPE);
+    const T aHE = (aHEp + c4ip * VVTH) + DU2;
+    const T UHE = aHE * rsqrtf(aHE);
+    const T UDS = scale_vel * UD;
+    const T t = ce_a - ce_b * ce_log(UDS);
+    T SIG = t * t;
+    if (damp_c > T(0)) SIG = SIG * ce_pow(T(1) - ce_exp(-damp_c / UDS), damp_pow);
+    const T ARR = SIG * (rhoN * srho);
+    const T aU = ARR * UD;                  // -DENPLU
+    const T aT = ARR * (VVTH * iUPM);       // ARR*VVTHU
+    const T aV = ARR * (VVTP * iUHM);       // ARR*VP_UHM
+    const T Y = (ARR * UPE) * VVTH;
+    const T hv = aU + aT + aV;
+    h2 = h2 + hv * dx_;
+    h3 = h3 + hv * dy_;
+    h4 = h4 + hv * dz_;
+    S1x = S1x + aV * dx_;
+    S1y = S1y + aV * dy_;
+    S1z = S1z + aV * dz_;
+    DSUM = DSUM - aU;
+    G = G + aV * VPHP + q75VP * (ARR * UHE);
+    H5 = H5 + aT * VPHH + aU * (hU2 - T(0.5) * UH2) - T(0.75) * Y;
+    double* un = u + IRHON + (f - 1) * 5;
+    un[0] = un[0] - dt * to_d(aU);
+    un[1] = un[1] - dt * to_d(uxN * aU - dx_ * aT);
+    un[2] = un[2] - dt * to_d(uyN * aU - dy_ * aT);
+    un[3] = un[3] - dt * to_d(uzN * aU - dz_ * aT);
+    un[4] = un[4] - dt * to_d((T(0.5) * UH2) * aU - VPHH * aT + T(0.75) * Y);
+  }
+  const T h5 = G + H5;
+  const T PPLUX = ux * DSUM - S1x, PPLUY = uy * DSUM - S1y, PPLUZ = uz * DSUM - S1z;
+  const T ENPLU = hU2 * DSUM - G;
+  u[1] = u[1] - dt * to_d(h2);
+  u[2] = u[2] - dt * to_d(h3);
+  u[3] = u[3] - dt * to_d(h4);
+  u[4] = u[4] - dt * to_d(h5);
+  // S of the magnetic field (and of psi) is zero; the recipient gets the
+  // other populations' lost density (DSUM less its own, already applied)
+  const int rk = ce_recipient(nN, reg);
+#pragma unroll
+  for (int f = 1; f < MF_MAX_FLUIDS; ++f) {
+    if (f > nN) break;
+    const bool rec = (f == rk);
+    double* un = u + IRHON + (f - 1) * 5;
+    un[0] = rec ? un[0] - dt * to_d(DSUM) : un[0];
+    un[1] = rec ? un[1] - dt * to_d(PPLUX) : un[1];
+    un[2] = rec ? un[2] - dt * to_d(PPLUY) : un[2];
+    un[3] = rec ? un[3] - dt * to_d(PPLUZ) : un[3];
+    un[4] = rec ? un[4] - dt * to_d(ENPLU) : un[4];
+  }
 }
 
 // All populations of one cell by one thread.  w: the stage-start primitive
@@ -283,24 +372,28 @@ __device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const W
 template <int IRHON, typename T = double, typename WA = const double*, int NN = 0>
 __device__ __forceinline__ void charge_exchange_add(const DevParams& P, const WA& w, int reg,
                                                     double dt, double* u) {
-  const int nN = NN > 0 ? NN : P.nf - 1;
-  T sum[CeTermsT<T>::kShared];
+  if constexpr (sizeof(T) == 4) {
+    charge_exchange_add_32<IRHON, WA, NN>(P, w, reg, dt, u);
+  } else {
+    const int nN = NN > 0 ? NN : P.nf - 1;
+    double sum[CeTerms::kShared];
 #pragma unroll
-  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f) {
-    if (f < nN) {
-      CeTermsT<T> c;
-      charge_exchange_terms<T>(P, w, IRHON + f * 5, c);
-      charge_exchange_own(c, dt, u + IRHON + f * 5);
+    for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f) {
+      if (f < nN) {
+        CeTerms c;
+        charge_exchange_terms(P, w, IRHON + f * 5, c);
+        charge_exchange_own(c, dt, u + IRHON + f * 5);
 #pragma unroll
-      for (int q = 0; q < CeTermsT<T>::kShared; ++q)
-        sum[q] = (f == 0) ? c.shared[q] : sum[q] + c.shared[q];
+        for (int q = 0; q < CeTerms::kShared; ++q)
+          sum[q] = (f == 0) ? c.shared[q] : sum[q] + c.shared[q];
+      }
     }
-  }
-  charge_exchange_plasma(dt, u, sum);
-  const int rk = ce_recipient(nN, reg);
+    charge_exchange_plasma(dt, u, sum);
+    const int rk = ce_recipient(nN, reg);
 #pragma unroll
-  for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
-    if (f < nN && f + 1 == rk) charge_exchange_gain(w, sum, dt, u + IRHON + f * 5);
+    for (int f = 0; f < MF_MAX_FLUIDS - 1; ++f)
+      if (f < nN && f + 1 == rk) charge_exchange_gain(w, sum, dt, u + IRHON + f * 5);
+  }
 }
 
 // SOURCE8WAVES (srcIdeal/PatchIdealMHDF.ChF:681-722) + ADDSOURCES
@@ -411,11 +504,12 @@ __device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double 
   }
 }
 
-// The plasma alone (no tracking surfaces).
+// The plasma alone (no tracking surfaces).  r2: the squared distance to the
+// sun of region_cell, or < 0 where that did not run.
 __device__ __forceinline__ void reinit_plasma(const DevParams& P, double dx, int i, int j, int k,
-                                              double t, double* u) {
+                                              double t, double r2, double* u) {
   ReinitState o;
-  if (!reinit_wind(P, dx, i, j, k, t, o)) return;
+  if (ieee64::lt(P.r0_2, r2) || !reinit_wind(P, dx, i, j, k, t, o)) return;
 #pragma unroll
   for (int q = 0; q < 8; ++q) u[q] = o.u[q];
 }
@@ -428,21 +522,21 @@ __device__ __forceinline__ void positivity_plasma(const DevParams& P, double* u)
   double Rho = u[0];
   bool was = lt(Rho, smallR);
   if (P.nf == 1 && was) Rho = smallR;  // one fluid: the velocities of the floored density
-  const double invRho = div(1.0, Rho);
-  const double Ux = u[1] * invRho, Uy = u[2] * invRho, Uz = u[3] * invRho;
+  // kinetic energy from the momenta; the velocities only where a floor acts
+  const double ke = half(div(mad(u[3], u[3], mad(u[2], u[2], u[1] * u[1])), Rho));
+  const double Rho0 = Rho;
   const double BxB = prod(kInv8Pi, mad(u[7], u[7], mad(u[6], u[6], u[5] * u[5])));
-  const double UxU = half(mad(Uz, Uz, mad(Uy, Uy, Ux * Ux)));
-  double Pr = hg * mad(-Rho, UxU, u[4] - BxB);
+  double Pr = hg * ((u[4] - BxB) - ke);
   if (was) Rho = smallR;
   if (lt(Pr, smallP)) { Pr = smallP; was = true; }
   if (was) {
+    const double f = div(Rho, Rho0);
     u[0] = Rho;
     if (P.nf > 1) {
-      u[1] = Rho * Ux;
-      u[2] = Rho * Uy;
-      u[3] = Rho * Uz;
+#pragma unroll
+      for (int q = 1; q < 4; ++q) u[q] = u[q] * f;
     }
-    u[4] = mad(Pr, ihg, mad(Rho, UxU, BxB));
+    u[4] = mad(Pr, ihg, mad(ke, f, BxB));
   }
 }
 
@@ -453,19 +547,17 @@ __device__ __forceinline__ void positivity_neutral(const DevParams& P, int f, do
   const double fd = (f == 1) ? P.smallr : (f == 3) ? kNet3Dens : kNet2Dens;
   const double fp = (f == 1) ? P.smallp : (f == 3) ? kNet3Pres : kNet2Pres;
   double Rho = un[0];
-  const double invRho = div(1.0, Rho);
-  const double Ux = un[1] * invRho, Uy = un[2] * invRho, Uz = un[3] * invRho;
-  const double UxU = half(mad(Uz, Uz, mad(Uy, Uy, Ux * Ux)));
-  double Pr = hg * mad(-Rho, UxU, un[4]);
+  const double ke = half(div(mad(un[3], un[3], mad(un[2], un[2], un[1] * un[1])), Rho));
+  double Pr = hg * (un[4] - ke);
   bool was = false;
   if (lt(Rho, fd)) { Rho = fd; was = true; }
   if (lt(Pr, fp)) { Pr = fp; was = true; }
   if (was) {
+    const double f = div(Rho, un[0]);
     un[0] = Rho;
-    un[1] = Rho * Ux;
-    un[2] = Rho * Uy;
-    un[3] = Rho * Uz;
-    un[4] = mad(Pr, ihg, Rho * UxU);
+#pragma unroll
+    for (int q = 1; q < 4; ++q) un[q] = un[q] * f;
+    un[4] = mad(Pr, ihg, ke * f);
   }
 }
 

@@ -59,29 +59,28 @@ __device__ __forceinline__ int region_tracer_cell(const DevParams& P, double dx,
 // DEFINE_REGIONS_2F (swlism/SWLISMF.ChF:654-742), Cartesian branch, or the
 // tracer variant above (HeliosphericProblem::defineRegions,
 // swlism/HeliosphericProblem.cpp:2538-2575).
+// r2: receives the squared distance to the sun.
 template <typename WA>
 __device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i, int j, int k,
-                                           const WA& w, double regtr) {
-  if (P.reg_tracer) return region_tracer_cell(P, dx, i, j, k, w, regtr);
+                                           const WA& w, double regtr, double& r2) {
   using namespace ieee64;
-  double x = (i + 0.5) * dx - P.sun_c[0];
-  double y = (j + 0.5) * dx - P.sun_c[1];
-  double z = 0.0, r2, invr, ur;
+  const double x = cell_centre(i) * dx - P.sun_c[0];
+  const double y = cell_centre(j) * dx - P.sun_c[1];
+  double z = 0.0;
+  r2 = x * x + y * y;
   if (P.sd == 3) {
-    z = (k + 0.5) * dx - P.sun_c[2];
-    r2 = x * x + y * y + z * z;
-    invr = div(1.0, root(r2));
-    ur = w[1] * (x * invr) + w[2] * (y * invr) + w[3] * (z * invr);
-  } else {
-    r2 = x * x + y * y;
-    invr = div(1.0, root(r2));
-    ur = w[1] * (x * invr) + w[2] * (y * invr);
+    z = cell_centre(k) * dx - P.sun_c[2];
+    r2 = r2 + z * z;
   }
+  if (P.reg_tracer) return region_tracer_cell(P, dx, i, j, k, w, regtr);
+  const double invr = div(1.0, root(r2));
+  double ur = w[1] * (x * invr) + w[2] * (y * invr);
+  if (P.sd == 3) ur = ur + w[3] * (z * invr);
   double TEMP = div(P.t_coeff * w[4], w[0]);
   int reg;
   bool zout = (P.sd == 3) && (lt(z, P.zbot) || lt(P.ztop, z));
-  if (le(0.6 * P.sun_v, absval(ur))) {
-    reg = (le(1.0e6, TEMP) && lt(P.sun_r * P.sun_r, r2)) ? 2 : 3;
+  if (le(P.lim_sun, absval(ur))) {
+    reg = (le(1.0e6, TEMP) && lt(P.sun_r2, r2)) ? 2 : 3;
     if (zout) reg = 1;
   } else {
     if (le(P.tmlim, TEMP)) {
@@ -92,6 +91,12 @@ __device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i,
     }
   }
   return reg;
+}
+template <typename WA>
+__device__ __forceinline__ int region_cell(const DevParams& P, double dx, int i, int j, int k,
+                                           const WA& w, double regtr) {
+  double r2;
+  return region_cell(P, dx, i, j, k, w, regtr, r2);
 }
 
 // Recipient of newly created neutrals: CHARGE_EXCHANGE_2F/3F/4F/MF
@@ -113,8 +118,6 @@ struct CeTerms {
   double shared[kShared];
   double pmi[3], enmi;  // PMIX, PMIY, PMIZ, ENMI
 };
-template <typename T>
-using CeTermsT = CeTerms;
 
 // w: the stage-start primitive state; o: the population's first component.
 // Factors that are powers of two scale exactly and move out of the products.
@@ -197,7 +200,7 @@ __device__ __forceinline__ double new_neutrals(int nN, int f, const L& lost) {
 }
 
 // The same for a thread per fluid; at(f, q): CeTerms::shared[q] of population f.
-template <int NN, typename T = double, typename AT>
+template <int NN, typename AT>
 __device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, const AT& at) {
   double h[4];
 #pragma unroll
@@ -208,7 +211,7 @@ __device__ __forceinline__ void charge_exchange_plasma(double dt, double* u, con
   }
   charge_exchange_source(dt, u, h);
 }
-template <int NN, typename T = double, typename WA, typename AT>
+template <int NN, typename WA, typename AT>
 __device__ __forceinline__ void charge_exchange_neutral(bool rec, int f, const WA&,
                                                         const CeTerms& c, double dt, double* un,
                                                         const AT& at) {
@@ -356,11 +359,12 @@ __device__ __host__ __forceinline__ void reinit_cell(const DevParams& P, double 
   }
 }
 
-// The plasma alone (no tracking surfaces).
+// The plasma alone (no tracking surfaces).  r2: the squared distance to the
+// sun of region_cell, or < 0 where that did not run.
 __device__ __forceinline__ void reinit_plasma(const DevParams& P, double dx, int i, int j, int k,
-                                              double t, double* u) {
+                                              double t, double r2, double* u) {
   ReinitState o;
-  if (!reinit_wind(P, dx, i, j, k, t, o)) return;
+  if (ieee64::lt(P.r0_2, r2) || !reinit_wind(P, dx, i, j, k, t, o)) return;
 #pragma unroll
   for (int q = 0; q < 8; ++q) u[q] = o.u[q];
 }
