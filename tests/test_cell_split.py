@@ -21,6 +21,7 @@ def _params(nf, glm, ce):
     p = mfgpu.helio_params(N)
     p.n_fluids = nf
     p.charge_exchange = int(ce and nf > 1)
+    p.neutral_sun_bc = int(nf > 1)
     if not glm:
         p.divb_cleaning, p.use_8wave = 0, 1
     return p
@@ -68,7 +69,7 @@ def test_level_ghosts_equal_single_patches(gpulib, nf, n, patch):
     for size in (patch, n):
         p = mfgpu.helio_params(n)
         p.n_fluids = nf
-        p.charge_exchange = int(nf > 1)
+        p.charge_exchange = p.neutral_sun_bc = int(nf > 1)
         ctx = mfgpu.Context(p)
         lev = mfgpu.Level(ctx, mfgpu.tile_boxes(n, size, 3))
         flat = np.zeros(lev.ndoubles)
