@@ -8,12 +8,13 @@
 // parts in one kernel, 200 registers, 2 warps per scheduler: pipe 53 % busy).
 // The parts share nothing but the face, so the neutral populations run one
 // per thread with a third of the registers, and the plasma solver alone fits
-// six blocks of 64 per SM.  The state is loaded in the face's
+// eight blocks of 64 per SM.  The state is loaded in the face's
 // frame (normal, then the two transverse components), which makes the code
 // the same for the three directions: one kernel instead of three, a third of
 // the instruction cache.  Fluxes of a 64^3 heliosphere step: 3.68 -> 2.33 ms
-// (pipe 75 % busy); 5 to 8 blocks of the plasma kernel per SM measured the
-// same within 2 %.  The neutral kernel takes 8 blocks (64 registers): its
+// (pipe 75 % busy).  The plasma kernel takes 8 blocks per SM (128 registers;
+// 128^3, plasma fluxes of a stage in ms, 6 / 8 / 10 blocks: parity 6.08 / 5.98 /
+// 6.13, fast FP64 5.27 / 4.68 / 4.75).  The neutral kernel takes 8 blocks (64 registers): its
 // products run on the integer pipes (vanleer_euler), whose latency more warps
 // hide (128^3, three populations: 6.04 ms a step with the products on the
 // FP64 pipe and 4 blocks, 5.67 with both changed).
@@ -26,7 +27,7 @@ namespace {
 using namespace MF_PHYS;
 
 constexpr int kPlasmaThreads = 64, kNeutralThreads = 128;
-constexpr int kPlasmaBlocks = 6, kNeutralBlocks = 8;  // per SM
+constexpr int kPlasmaBlocks = 8, kNeutralBlocks = 8;  // per SM
 
 // The faces of a batch in every direction: the launch's blocks cover those of
 // direction 0, then 1, then 2 (nb blocks each).  w: the primitive state whose
