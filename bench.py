@@ -285,6 +285,8 @@ def run_ours(a):
     dom_avg_ms = by_kind[dom][0] / by_kind[dom][1]
     nc = ctx.nc
     alg = _algorithmic_bytes(dom, p64, boxes, nc, 8)
+    if dom == "flux":  # of one direction; a launch may hold a part of every direction
+        alg = alg * p64.space_dim * by_kind["update"][1] // by_kind[dom][1]
     peak, peak_kind = _peaks()
     achieved = alg / (dom_avg_ms * 1e-3) / 1e9
     traffic = _traffic_table().get(f"fp64_{dom}") if n == N_DEFAULT else None
