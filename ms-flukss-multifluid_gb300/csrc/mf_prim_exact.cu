@@ -118,8 +118,9 @@ __global__ void __launch_bounds__(kMaxBlock)
 // branch fills them, for the levels whose valid-cell primitives and ghost
 // copies come first: plasma and neutral fluid 1 from the boundary state, the
 // other neutral fluids from the primitive state of the nearest cell along the
-// boundary normal, a valid cell of the patch.  One block per box, fluid and
-// 256 cells.
+// boundary normal: a valid cell of the patch or, one cell off the boundary, a
+// ghost that the sibling copy filled (in the FP32 copy alone where the FP64
+// state is not exchanged).  One block per box, fluid and 256 cells.
 __global__ void __launch_bounds__(256)
     k_farfield(const __grid_constant__ DevParams P, const double* __restrict__ U, double* W,
                float* __restrict__ Wf, const FarReg* __restrict__ regs,
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(256)
   int x[3];
   decode(t, F.lo, F.ext, x[0], x[1], x[2]);
   const long long base = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]);
-  double* Ww = write_w ? W : nullptr;  // (else only the FP32 ghosts are read)
+  double* Ww = write_w ? W : nullptr;  // (else only the FP32 ghosts are filled and read)
   if (f == 0) {
     far_plasma(P, R, U, Ww, Wf, base, cs);
     return;
@@ -147,6 +148,11 @@ __global__ void __launch_bounds__(256)
     for (int d = 0; d < P.sd; ++d)
       if (!P.periodic[d]) x[d] = min(max(x[d], R.dlo[d]), R.dhi[d]);
     const long long from = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]) + s * cs;
+    if (!write_w) {  // the FP64 ghosts were not copied: the FP32 copy of both
+#pragma unroll
+      for (int q = 0; q < 5; ++q) Wf[base + (s + q) * cs] = Wf[from + q * cs];
+      return;
+    }
 #pragma unroll
     for (int q = 0; q < 5; ++q) w[q] = W[from + q * cs];
   }
