@@ -148,20 +148,21 @@ __device__ __forceinline__ double mul(double a, double b) {
   return zero ? pack(sg, 0u) : pack(((uint32_t)(q >> 32) + ex) | sg, (uint32_t)q);
 }
 
-// Sign-magnitude bits as an ordered integer (-0 and +0 equal).
+// Sign-magnitude bits as an ordered integer (-0 and +0 equal): the NaN lie
+// outside [-kInf, kInf], so the same 64-bit comparisons keep all of them out,
+// those with their payload in the low word too.
+constexpr int64_t kInf = 0x7ff0000000000000ll;
 __device__ __forceinline__ int64_t key(double x) {
   const int64_t s = (int64_t)((int32_t)hi_of(x) >> 31);
   return ((int64_t)join(hi_of(x) & 0x7fffffffu, lo_of(x)) ^ s) - s;
 }
-// NaN (the quiet ones that arithmetic produces)
-__device__ __forceinline__ bool is_nan(double x) {
-  return (hi_of(x) & 0x7fffffffu) > 0x7ff00000u;
-}
 __device__ __forceinline__ bool lt(double a, double b) {
-  return (key(a) < key(b)) & !is_nan(a) & !is_nan(b);
+  const int64_t ka = key(a), kb = key(b);
+  return (ka < kb) & (ka >= -kInf) & (kb <= kInf);
 }
 __device__ __forceinline__ bool le(double a, double b) {
-  return (key(a) <= key(b)) & !is_nan(a) & !is_nan(b);
+  const int64_t ka = key(a), kb = key(b);
+  return (ka <= kb) & (ka >= -kInf) & (kb <= kInf);
 }
 __device__ __forceinline__ double absval(double x) { return pack(hi_of(x) & 0x7fffffffu, lo_of(x)); }
 // x with its sign changed where the top bit of s is set
@@ -170,10 +171,12 @@ __device__ __forceinline__ double flip(double x, uint32_t s) {
 }
 // fmax: the other operand where one is NaN
 __device__ __forceinline__ double maxnum(double a, double b) {
-  return ((key(a) < key(b)) & !is_nan(b)) | is_nan(a) ? b : a;
+  const int64_t ka = key(a), kb = key(b);
+  return ((ka < kb) & (kb <= kInf)) | (ka > kInf) ? b : a;
 }
 __device__ __forceinline__ double minnum(double a, double b) {
-  return ((key(b) < key(a)) & !is_nan(b)) | is_nan(a) ? b : a;
+  const int64_t ka = key(a), kb = key(b);
+  return ((kb < ka) & (kb >= -kInf)) | (ka < -kInf) ? b : a;
 }
 
 // x 2^K (|K| <= 8): the exponent moved, where x and the result are normal or
