@@ -193,13 +193,19 @@ __device__ __forceinline__ double scale(double x) {
 __device__ __forceinline__ double half(double x) { return scale<-1>(x); }
 
 // minmod of two differences (reconstructionF.ChF:5-13): the one of smaller
-// magnitude where the signs agree, else a zero of a's sign.
+// magnitude where the signs agree, else a zero of a's sign.  As in the FP64
+// form, sign(a) max(0, min(|a|, sign(a) b)), a NaN gives way to the other
+// difference: a where b alone is NaN, b or zero by the signs where a alone is,
+// a zero where both are.  (A NaN has the larger magnitude; differences are
+// quiet NaN, whose high word tells.)
 __device__ __forceinline__ double minmod(double a, double b) {
   const uint32_t ha = hi_of(a), hb = hi_of(b);
   const uint64_t ua = join(ha & 0x7fffffffu, lo_of(a)), ub = join(hb & 0x7fffffffu, lo_of(b));
-  const bool same = (int32_t)(ha ^ hb) >= 0, first = ua <= ub;
+  const bool first = ua <= ub;
   const uint32_t h = first ? ha : hb, l = first ? lo_of(a) : lo_of(b);
-  return pack(same ? h : ha & 0x80000000u, same ? l : 0u);
+  const bool take = ((int32_t)(ha ^ hb) >= 0) | ((hb & 0x7fffffffu) > 0x7ff00000u);
+  const bool keep = take & ((h & 0x7fffffffu) <= 0x7ff00000u);
+  return pack(keep ? h : ha & 0x80000000u, keep ? l : 0u);
 }
 
 }  // namespace ieee64

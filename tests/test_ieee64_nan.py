@@ -1,10 +1,16 @@
-"""NaN in the integer-pipe forms of csrc/mf_ieee64.cuh: maxima and comparisons
-against the FP64 forms for every pair of special values."""
+"""NaN in the integer-pipe forms of csrc/mf_ieee64.cuh: minmod, maxima and
+comparisons against the FP64 forms for every pair of special values; and a
+step beside a cell that holds NaN, whose neighbours' slopes come from the
+finite difference alone."""
 import os
 import shutil
 import subprocess
 
+import numpy as np
 import pytest
+
+import mfgpu
+from helpers import to_device, to_host
 
 pytestmark = pytest.mark.gpu
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -24,7 +30,36 @@ def counts(tmp_path_factory):
     return dict(line.split(maxsplit=1) for line in r.stdout.strip().splitlines())
 
 
-@pytest.mark.parametrize("name", ["maxmin", "compare"])
+@pytest.mark.parametrize("name", ["minmod", "maxmin", "compare"])
 def test_special_values_equal_the_fp64_forms(counts, name):
     assert counts["status"] == "no error"
     assert int(counts[name]) == 0
+
+
+@pytest.mark.parametrize("prec", [mfgpu.PREC_FP64, mfgpu.PREC_FP64_FAST])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_second_cell_beside_nan_equals_oracle(gpulib, oracle, prec, axis):
+    """One first-order step with one NaN cell c: cell c+2 along axis is
+    reached by c through the limiter of c+1 alone."""
+    n = 9
+    p = mfgpu.helio_params(64, time_approximation=mfgpu.TA_FIRST_ORDER, precision=prec)
+    ctx = mfgpu.Context(p)
+    vlo = [34, 30, 29]
+    vhi = [v + n - 1 for v in vlo]
+    lo, hi = mfgpu.grow(vlo, vhi, ctx.ng, 3)
+    U = mfgpu.init_host_fab(p, lo, hi, "helio")
+    U *= 1.0 + 0.02 * np.random.default_rng(9).standard_normal(U.shape)
+    dt = 0.2 * oracle.compute_dt(p, U, lo, hi, vlo, vhi)[1]
+    c = [ctx.ng + 3] * 3  # (z, y, x) in the fab
+    U[(slice(None), *c)] = np.nan
+    t = to_device(U)
+    st, _, _ = ctx.patch_update(t.data_ptr(), lo, hi, vlo, vhi, dt, allow_error=True)
+    assert st == mfgpu.MF_ERR_NONFINITE
+    oracle.patch_update(p, U, lo, hi, vlo, vhi, dt)
+    at = list(c)
+    at[2 - axis] += 2
+    g, o = to_host(t)[(slice(None), *at)], U[(slice(None), *at)]
+    assert np.all(np.isfinite(o))
+    scale = np.maximum(np.abs(o), 1e-3 * np.max(np.abs(U[:, ctx.ng, ctx.ng, ctx.ng])))
+    assert np.all(np.abs(g - o) <= (1e-12 if prec == mfgpu.PREC_FP64 else 1e-7) * scale)
+    ctx.close()
