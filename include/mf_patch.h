@@ -441,7 +441,8 @@ mf_status mf_face_fluxes(mf_ctx* ctx, int dir, int n, const double* wl, const do
    per patch).  Times the prim, flux and update kernels of the level's batch
    at 64, 128 and 256 threads per block (reps launches each, stage-1 form, so
    the level's state is not changed) and keeps the fastest shape of each
-   kind for later steps.  Where the fused kernel covers the level's options
+   kind for later steps; a kind whose kernels have blocks of their own (the
+   FP64 fluxes and the update split by fluid) keeps 128.  Where the fused kernel covers the level's options
    (see mf_level_set_schedule) and no flux registers are attached, it then
    times stage 1 with the split kernels against the fused kernel at the tile
    shapes 8x8x4, 8x4x4, 16x8x2, 8x8x2 and 4x4x4 (16x16, 32x8, 16x8, 8x8 in

@@ -2262,7 +2262,8 @@ mf_status mf_level_profile_step(mf_level* L, double dt, float* ms, int* kinds, i
 // Time `reps` launches of one kernel kind of stage 1 (0 prim, 1 fluxes of
 // every direction, 2 update without averaging, 3 the fused flux + update
 // kernel on the work list in fp1, 4 the fluxes and update in the level's
-// overlap chunks) with the level's current threads.
+// overlap chunks, 5 update with one thread per cell) with the level's current
+// threads.
 // Stage 1 reads U and writes only W, F, Bn and U1, so the level's state is
 // left as it was; the step state used is a private copy with dt = 0.
 static mf_status time_kind(mf_level* L, int kind, int reps, cudaEvent_t e0, cudaEvent_t e1,
@@ -2303,6 +2304,7 @@ static mf_status time_kind(mf_level* L, int kind, int reps, cudaEvent_t e0, cuda
                            parts, L->s);
     } else {
       int nb = 0;
+      B.by_cell = kind == 5;
       if (p.precision == MF_PREC_MIXED)
         e = mf::launch_update_fast<float>(c->dp, B, b, 0, 1.0, ds, parts, &nb, L->s);
       else if (p.precision == MF_PREC_FP64_FAST)
@@ -2338,14 +2340,26 @@ mf_status mf_level_autotune(mf_level* L, int reps, int threads[3]) {
   }
   static const int cand[3] = {64, 128, 256};
   mf_status st = MF_OK;
+  // The blocks of the fluxes and the update split by fluid are fixed: timing
+  // them at three sizes would let noise pick nt[1] and nt[2], which other
+  // kernels take (constrained transport, the dt kernel).  Their default stays,
+  // but for the overlapped launches tried below, whose update has one thread
+  // per cell in blocks of nt[2].
+  const mf_params& p = c->p;
+  const bool chunks = L->gathers.empty() && p.precision == MF_PREC_MIXED && !c->dp.ct &&
+                      (p.time_approximation == MF_TA_RK2 ||
+                       p.time_approximation == MF_TA_FIRST_ORDER);
+  const int timed[3] = {0, mf::flux_split(c->dp, p.precision) ? -1 : 1,
+                        !mf::update_by_fluid(c->dp) ? 2 : chunks ? 5 : -1};
   for (int kind = 0; kind < 3 && st == MF_OK; ++kind) {
+    if (timed[kind] < 0) continue;
     float best = 0.f;
     int bnt = L->b1.nt[kind];
     for (int q = 0; q < 3 && st == MF_OK; ++q) {
       L->b1.nt[kind] = L->b2.nt[kind] = L->bp.nt[kind] = cand[q];
       float ms = 0.f;
-      st = time_kind(L, kind, 1, e0, e1, &ms);  // warm-up
-      if (st == MF_OK) st = time_kind(L, kind, reps, e0, e1, &ms);
+      st = time_kind(L, timed[kind], 1, e0, e1, &ms);  // warm-up
+      if (st == MF_OK) st = time_kind(L, timed[kind], reps, e0, e1, &ms);
       if (st == MF_OK && (q == 0 || ms < best)) {
         best = ms;
         bnt = cand[q];
@@ -2357,7 +2371,6 @@ mf_status mf_level_autotune(mf_level* L, int reps, int threads[3]) {
   // unchunked or in 2, 4, 8 overlapped chunks (mixed precision), against the
   // fused kernel at each tile shape that fits the options.  A level feeding
   // flux registers keeps the split, unchunked kernels, which store the fluxes.
-  const mf_params& p = c->p;
   const int sd = p.space_dim;
   // FP64 paths: the face fluxes per face against by lines
   if (st == MF_OK && p.precision != MF_PREC_MIXED && p.time_approximation != MF_TA_HANCOCK) {
@@ -2379,8 +2392,7 @@ mf_status mf_level_autotune(mf_level* L, int reps, int threads[3]) {
     if (st == MF_OK) st = time_kind(L, 2, reps, e0, e1, &tu);
     float best = tf + tu;
     int bk = 1;
-    if (p.precision == MF_PREC_MIXED && !c->dp.ct &&
-        (p.time_approximation == MF_TA_RK2 || p.time_approximation == MF_TA_FIRST_ORDER)) {
+    if (chunks) {
       static const int ck[3] = {2, 4, 8};
       for (int q = 0; q < 3 && st == MF_OK; ++q) {
         st = level_set_chunks(L, ck[q]);
