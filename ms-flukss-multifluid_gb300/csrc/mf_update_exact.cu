@@ -266,20 +266,30 @@ cudaError_t launch_finalize(const DevParams& P, const DtPartial* partials, const
 // loads and take many blocks (128^3: 2 per SM 0.66 ms a step with the far-field
 // fill, 60 per SM 0.55); FP32 ones, half the bytes, lose more to the repeated
 // set-up (0.57 against 0.59).
-static unsigned exchange_split(int nreg, int nc, int per_sm) {
-  const int want = (per_sm * 152 + nreg - 1) / nreg;
-  return (unsigned)(want < 1 ? 1 : want > nc ? nc : want);
+static cudaError_t exchange_split(int nreg, int nc, int per_sm, dim3* grid) {
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int want = (per_sm * sms + nreg - 1) / nreg;
+  *grid = dim3(nreg, want < 1 ? 1 : want > nc ? nc : want);
+  return e;
 }
 
 cudaError_t launch_exchange(double* u, const CopyReg* regs, int nreg, int nc, cudaStream_t s) {
   if (nreg <= 0) return cudaSuccess;
-  k_exchange<double><<<dim3(nreg, exchange_split(nreg, nc, 60)), 256, 0, s>>>(u, regs, nc);
+  dim3 grid;
+  const cudaError_t e = exchange_split(nreg, nc, 60, &grid);
+  if (e != cudaSuccess) return e;
+  k_exchange<double><<<grid, 256, 0, s>>>(u, regs, nc);
   return cudaGetLastError();
 }
 
 cudaError_t launch_exchange_f(float* u, const CopyReg* regs, int nreg, int nc, cudaStream_t s) {
   if (nreg <= 0) return cudaSuccess;
-  k_exchange<float><<<dim3(nreg, exchange_split(nreg, nc, 2)), 256, 0, s>>>(u, regs, nc);
+  dim3 grid;
+  const cudaError_t e = exchange_split(nreg, nc, 2, &grid);
+  if (e != cudaSuccess) return e;
+  k_exchange<float><<<grid, 256, 0, s>>>(u, regs, nc);
   return cudaGetLastError();
 }
 
