@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(kMaxBlock)
 // other neutral fluids from the primitive state of the nearest cell along the
 // boundary normal: a valid cell of the patch or, one cell off the boundary, a
 // ghost that the sibling copy filled (in the FP32 copy alone where the FP64
-// state is not exchanged).  One block per box, fluid and 256 cells.
+// state is not exchanged).  One block per box, fluid and 256 cells, or more
+// cells where the box has over 2^24: a grid holds 65535 blocks along z.
 __global__ void __launch_bounds__(256)
     k_farfield(const __grid_constant__ DevParams P, const double* __restrict__ U, double* W,
                float* __restrict__ Wf, const FarReg* __restrict__ regs,
@@ -128,35 +129,36 @@ __global__ void __launch_bounds__(256)
   const FarReg& F = regs[blockIdx.x];
   const RunParams& R = runs[F.run];
   const int f = blockIdx.y;
-  const int t = blockIdx.z * blockDim.x + threadIdx.x;
-  if (t >= F.ext[0] * F.ext[1] * F.ext[2]) return;
+  const int n = F.ext[0] * F.ext[1] * F.ext[2];
   const long long cs = (long long)F.fn[0] * F.fn[1] * F.fn[2];
-  int x[3];
-  decode(t, F.lo, F.ext, x[0], x[1], x[2]);
-  const long long base = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]);
   double* Ww = write_w ? W : nullptr;  // (else only the FP32 ghosts are filled and read)
-  if (f == 0) {
-    far_plasma(P, R, U, Ww, Wf, base, cs);
-    return;
-  }
   const int s = P.irhon + (f - 1) * 5;
-  double w[5];
-  if (f == 1) {
-#pragma unroll
-    for (int q = 0; q < 5; ++q) w[q] = R.bc_n1[q];
-  } else {
-    for (int d = 0; d < P.sd; ++d)
-      if (!P.periodic[d]) x[d] = min(max(x[d], R.dlo[d]), R.dhi[d]);
-    const long long from = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]) + s * cs;
-    if (!write_w) {  // the FP64 ghosts were not copied: the FP32 copy of both
-#pragma unroll
-      for (int q = 0; q < 5; ++q) Wf[base + (s + q) * cs] = Wf[from + q * cs];
-      return;
+  for (int t = blockIdx.z * blockDim.x + threadIdx.x; t < n; t += gridDim.z * blockDim.x) {
+    int x[3];
+    decode(t, F.lo, F.ext, x[0], x[1], x[2]);
+    const long long base = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]);
+    if (f == 0) {
+      far_plasma(P, R, U, Ww, Wf, base, cs);
+      continue;
     }
+    double w[5];
+    if (f == 1) {
 #pragma unroll
-    for (int q = 0; q < 5; ++q) w[q] = W[from + q * cs];
+      for (int q = 0; q < 5; ++q) w[q] = R.bc_n1[q];
+    } else {
+      for (int d = 0; d < P.sd; ++d)
+        if (!P.periodic[d]) x[d] = min(max(x[d], R.dlo[d]), R.dhi[d]);
+      const long long from = F.off + loc(F.flo, F.fn, x[0], x[1], x[2]) + s * cs;
+      if (!write_w) {  // the FP64 ghosts were not copied: the FP32 copy of both
+#pragma unroll
+        for (int q = 0; q < 5; ++q) Wf[base + (s + q) * cs] = Wf[from + q * cs];
+        continue;
+      }
+#pragma unroll
+      for (int q = 0; q < 5; ++q) w[q] = W[from + q * cs];
+    }
+    store_prim<5>(Ww, Wf, base + s * cs, cs, w);
   }
-  store_prim<5>(Ww, Wf, base + s * cs, cs, w);
 }
 
 // ---------------------------------------------------------------------------
@@ -167,7 +169,8 @@ cudaError_t launch_farfield(const DevParams& P, const double* u, double* w, floa
                             const FarReg* far, int nfar, int most, const RunParams* runs,
                             int write_w, cudaStream_t s) {
   if (nfar <= 0) return cudaSuccess;
-  const dim3 grid(nfar, P.nf, (most + 255) / 256);
+  const int blocks = (most + 255) / 256;
+  const dim3 grid(nfar, P.nf, blocks < 65535 ? blocks : 65535);
   k_farfield<<<grid, 256, 0, s>>>(P, u, w, wf, far, runs, write_w);
   return cudaGetLastError();
 }
