@@ -186,7 +186,7 @@ DevParams make_dev(const mf_params& p) {
   DevParams P;
   std::memset(&P, 0, sizeof(P));
   P.sd = p.space_dim;
-  P.nf = p.n_fluids;
+  P.nf = P.nf_face = p.n_fluids;
   P.glm = (p.divb_cleaning == 5) ? 1 : 0;
   P.nc = num_cons(p);
   P.ils = num_fluid_cons(p);
@@ -1550,7 +1550,7 @@ static mf_status enqueue_level_step(mf_level* L, int advance, cudaEvent_t* ev = 
     if (ev) {  // prim, faces, predictor, shift, fluxes, update
       const int k0[4] = {1, 1, 3, 1};
       for (int q = 0; q < 4; ++q) kinds[ne + q] = k0[q];
-      const int nh = mf::flux_launches(c->dp, p.precision, false);
+      const int nh = mf::flux_launches(c->dp, p.precision, false, true);
       for (int q = 0; q < nh; ++q) kinds[ne + 4 + q] = 2;
       kinds[ne + 4 + nh] = 3;
       ne += mf::hancock_launches(c->dp, p.precision);

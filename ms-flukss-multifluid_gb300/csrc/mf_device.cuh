@@ -29,6 +29,7 @@ enum RsKind : int { kRoe8 = 0, kRoe7 = 1, kRusanov = 2, kVFRoe = 3 };
 // Parameters as the kernels see them (mf_params + derived constants).
 struct DevParams {
   int sd, nf, glm, nc, irhon;
+  int nf_face;  // fluids whose fluxes k_flux and k_hflux form on interior faces (FP64 paths)
   int rs, aver;
   int use8, divb_method, check_pos, ce, reinit, bc_kind;
   int char_rec, check_tvd;

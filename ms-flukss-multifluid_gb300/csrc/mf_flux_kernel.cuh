@@ -310,6 +310,13 @@ __device__ __forceinline__ int helio_side(const DevParams& P, const RunParams& R
   return (f == RP.dlo[DIR]) ? 0 : (f == RP.dhi[DIR] + 1) ? 1 : -1;
 }
 
+// Fluids whose fluxes a face takes here: where the neutral populations have a
+// launch of their own (neutrals_apart), those of a HELIOBC face alone.
+template <typename R>
+__device__ __forceinline__ int face_fluids(const DevParams& P, int hside) {
+  return (sizeof(R) == sizeof(float) || hside >= 0) ? P.nf : P.nf_face;
+}
+
 // The fluxes of face gi of the batch's flat face index of direction DIR
 // (gi >= total: none).  WF: read the limiter inputs from Wf, the FP32 copy of
 // W the prim kernel wrote (R = float), instead of converting W value by
@@ -444,7 +451,8 @@ __device__ __forceinline__ void flux_face(const DevParams& P, const double* __re
   Bn[D.bn_off[DIR] + fo] = bn;
 
   // neutral fluids: minmod face states, van Leer splitting (VANLEERF)
-  for (int fl = 1; fl < P.nf; ++fl) {
+  const int nff = face_fluids<R>(P, hside);
+  for (int fl = 1; fl < nff; ++fl) {
     const int s = P.irhon + (fl - 1) * 5;
     R nl[5], nr[5], gn[5];
 #pragma unroll
@@ -567,7 +575,8 @@ __device__ __forceinline__ void riemann_face(const DevParams& P, const RunParams
   for (int q = 0; q < 8; ++q) Fo[q * fcs] = g[q];
   if (P.glm) Fo[8 * fcs] = g[8];
   Bn[D.bn_off[DIR] + loc(D.vlo, fnb, i, j, k)] = bn;
-  for (int fl = 1; fl < P.nf; ++fl) {
+  const int nff = face_fluids<R>(P, hside);
+  for (int fl = 1; fl < nff; ++fl) {
     const int s0 = P.irhon + (fl - 1) * 5;
     R nl[5], nr[5], gn[5];
 #pragma unroll

@@ -485,27 +485,30 @@ cudaError_t launch_hancock(const DevParams& P, int precision, const StageBuffers
     k_hshift<<<flat_blocks(a.tot_s, nt), nt, 0, s>>>(P, B.w, H, a.desc, a.ndesc, a.tot_s, a.runs);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   mark();
-  if (flux_split(P, precision)) {
-    const double* const fv[3] = {H.fv[0], H.fv[1], H.fv[2]};
-    const bool fast = precision == MF_PREC_FP64_FAST;
+  const double* const fv[3] = {H.fv[0], H.fv[1], H.fv[2]};
+  const bool fast = precision == MF_PREC_FP64_FAST;
+  const bool split = flux_split(P, precision), apart = neutrals_apart(P, precision, true);
+  if (split) {
     e = fast ? launch_plasma_fast(P, B.w, fv, B.f, B.bn, c, state, s)
              : launch_plasma_exact(P, B.w, fv, B.f, B.bn, c, state, s);
     if (e != cudaSuccess) return e;
     mark();
-    if (P.nf > 1) {
-      e = fast ? launch_neutral_fast(P, B.w, fv, B.f, c, s)
-               : launch_neutral_exact(P, B.w, fv, B.f, c, s);
-      if (e != cudaSuccess) return e;
-      mark();
-    }
-  } else {
+  }
+  if (apart || (split && P.nf > 1)) {
+    e = fast ? launch_neutral_fast(P, B.w, fv, B.f, c, s)
+             : launch_neutral_exact(P, B.w, fv, B.f, c, s);
+    if (e != cudaSuccess) return e;
+    mark();
+  }
+  if (!split) {
+    const DevParams Q = apart ? plasma_only(P) : P;
     for (int d = 0; d < P.sd; ++d) {
       if (precision == MF_PREC_MIXED)
-        e = launch_hflux_fast<float>(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+        e = launch_hflux_fast<float>(Q, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
       else if (precision == MF_PREC_FP64_FAST)
-        e = launch_hflux_fast<double>(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+        e = launch_hflux_fast<double>(Q, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
       else
-        e = launch_hflux_exact(P, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
+        e = launch_hflux_exact(Q, d, B.w, H.fv[d], B.f[d], B.bn[d], c, state, s);
       if (e != cudaSuccess) return e;
       mark();
     }

@@ -289,6 +289,23 @@ cudaError_t launch_update_exact(const DevParams& P, const StageBuffers& B, const
 inline bool flux_split(const DevParams& P, int precision) {
   return precision != MF_PREC_MIXED && !P.char_rec && !P.helio_bc && P.nls == 0;
 }
+// With those options, one thread of k_flux (or k_hflux) solving every fluid in
+// turn is a long chain that small launches wait for, so the neutral populations
+// run first in launch_neutral_* and k_flux adds the plasma (HELIOBC faces: and
+// their own neutral fluxes).  Fluxes of a 16^3 patch's two stages in fast FP64
+// with tracking surfaces 380 -> 289 us, characteristic 659 -> 567; of 64^3 cells
+// 3.67 -> 3.11 ms (the step with characteristic limiting 8.07 -> 7.60).  Not where characteristic face values decide
+// the positivity fallback of the neutral ones (limited before the predictor in
+// the Hancock step).
+inline bool neutrals_apart(const DevParams& P, int precision, bool hancock) {
+  return precision != MF_PREC_MIXED && !flux_split(P, precision) && P.nf > 1 &&
+         (hancock || !(P.char_rec && P.check_pos));
+}
+inline DevParams plasma_only(const DevParams& P) {
+  DevParams Q = P;
+  Q.nf_face = 1;
+  return Q;
+}
 // fv: null, or the Hancock corrector's face values per direction.
 cudaError_t launch_plasma_exact(const DevParams& P, const double* w, const double* const* fv,
                                 void* const f[3], void* const bn[3], const Batch& b,
@@ -304,8 +321,10 @@ cudaError_t launch_neutral_fast(const DevParams& P, const double* w, const doubl
 // flux_launches launches, with B.ev's events from *ne on after each.
 cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers& B,
                           const Batch& b, const StepState* state, cudaStream_t s, int* ne);
-inline int flux_launches(const DevParams& P, int precision, bool lines) {
-  return (!lines && flux_split(P, precision)) ? 1 + (P.nf > 1 ? 1 : 0) : P.sd;
+inline int flux_launches(const DevParams& P, int precision, bool lines, bool hancock = false) {
+  if (lines) return P.sd;
+  if (flux_split(P, precision)) return 1 + (P.nf > 1 ? 1 : 0);
+  return P.sd + (neutrals_apart(P, precision, hancock) ? 1 : 0);
 }
 // fast physics: R = float (mixed precision) or double (fast FP64)
 // wf (R = float only, nullable): the FP32 copy of w the prim kernel wrote
@@ -484,7 +503,7 @@ cudaError_t launch_hancock(const DevParams& P, int precision, const StageBuffers
                            StepState* state, DtPartial* partials, int* nblocks_v,
                            cudaStream_t s, int corrector_flags = kStageDt);
 inline int hancock_launches(const DevParams& P, int precision) {
-  return 5 + flux_launches(P, precision, false);
+  return 5 + flux_launches(P, precision, false, true);
 }
 
 // Corrector fluxes of the Hancock step from the shifted face values.

@@ -4,8 +4,10 @@
 
 namespace mf {
 
-cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers& B,
+cudaError_t launch_fluxes(const DevParams& P0, int precision, const StageBuffers& B,
                           const Batch& b, const StepState* state, cudaStream_t s, int* ne) {
+  const bool apart = !B.lines && neutrals_apart(P0, precision, false);
+  const DevParams P = apart ? plasma_only(P0) : P0;
   cudaError_t e = cudaSuccess;
   auto done = [&]() {
     if (e == cudaSuccess && B.ev) cudaEventRecord(B.ev[(*ne)++], s);
@@ -19,6 +21,11 @@ cudaError_t launch_fluxes(const DevParams& P, int precision, const StageBuffers&
     e = fast ? launch_neutral_fast(P, B.w, nullptr, B.f, b, s)
              : launch_neutral_exact(P, B.w, nullptr, B.f, b, s);
     return done();
+  }
+  if (apart) {
+    e = precision == MF_PREC_FP64_FAST ? launch_neutral_fast(P, B.w, nullptr, B.f, b, s)
+                                       : launch_neutral_exact(P, B.w, nullptr, B.f, b, s);
+    if (done() != cudaSuccess) return e;
   }
   for (int d = 0; d < P.sd; ++d) {
     if (precision == MF_PREC_MIXED)
