@@ -337,7 +337,7 @@ def run_ours(a):
         fast = {"value": ws * zones * a.steps / (msf * 1e-3), "ms_per_step": msf / a.steps,
                 "speedup_vs_fp64": (ws * zones * a.steps / (msf * 1e-3)) / value,
                 "per_kind_ms": {}, "autotuned": tunedf,
-                "dtype": "f64 with fused multiply-adds and reused reciprocals"}
+                "dtype": "f64 with fused multiply-adds"}
         for kind, t in proff:
             fast["per_kind_ms"][kind] = fast["per_kind_ms"].get(kind, 0.0) + t
         levf.close()

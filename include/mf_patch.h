@@ -75,14 +75,13 @@ enum { MF_TA_FIRST_ORDER = 0, MF_TA_HANCOCK = 1, MF_TA_RK2 = 2 };
                       conserved state, flux-divergence accumulation, pressure
                       recovery, positivity fix and the charge-exchange rates
                       FP64.
-   MF_PREC_FP64_FAST  FP64 everywhere with fused multiply-adds and reused
-                      reciprocals (results differ from MF_PREC_FP64 at the
-                      rounding level; limiter and region decisions identical
-                      for identical input states).
+   MF_PREC_FP64_FAST  FP64 everywhere with fused multiply-adds and products
+                      shared between terms (results differ from MF_PREC_FP64
+                      at the rounding level; limiter and region decisions
+                      identical for identical input states).
    MF_PREC_MIXED_CE32 MF_PREC_MIXED with the charge-exchange rates in FP32 as
-                      well (opt-in: the rates are the dominant FP64 work of the
-                      update; the source they scale is still added to the
-                      FP64 state in FP64). */
+                      well (opt-in; no faster than MF_PREC_MIXED; the source
+                      they scale is still added to the FP64 state in FP64). */
 enum { MF_PREC_FP64 = 0, MF_PREC_MIXED = 1, MF_PREC_FP64_FAST = 2, MF_PREC_MIXED_CE32 = 3 };
 /* physical (non-periodic) boundary treatment of primitive ghost cells */
 enum { MF_BC_NONE = 0, MF_BC_FARFIELD = 1 };

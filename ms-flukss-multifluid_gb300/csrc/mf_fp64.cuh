@@ -1,9 +1,11 @@
-// mf_fp64.cuh - FP64 reciprocal and logarithm with fewer FP64-pipe
-// instructions than the correctly rounded library forms, for the paths that
-// do not reproduce the reference's rounding (MF_PREC_FP64_FAST and the FP64
-// charge-exchange rates of MF_PREC_MIXED).  GB300 issues FP64 arithmetic at a
-// small fraction of its FP32 rate, so on those paths every FP64 instruction
-// counts against the step time.
+// mf_fp64.cuh - FP64 logarithm and conversions with fewer FP64-pipe
+// instructions than the library forms, for the paths that do not reproduce the
+// reference's rounding (the fast physics: MF_PREC_FP64_FAST and the FP64
+// charge-exchange rates of MF_PREC_MIXED) and for the FP32 values of the mixed
+// paths; and a reciprocal, which no kernel takes since ieee64::div is exact
+// and free beside FP64 work.  GB300 issues FP64 arithmetic at a small fraction
+// of its FP32 rate, so on those paths every FP64 instruction counts against
+// the step time.
 //
 // rcp64: the hardware's approximate FP64 reciprocal (rcp.approx.ftz.f64,
 // relative error about 2^-20) refined by one third-order Newton-Raphson step

@@ -6,7 +6,8 @@
 // holds the pipe for as long as the other pipes need for some 40 to 80 integer
 // instructions.  The library's division takes 7 and its square root 7.3 such
 // slots (measured: 576 and 601 clocks per warp and scheduler against 82 for an
-// add, a multiply, a fused multiply-add or a comparison).  div() and root()
+// add, a multiply, a fused multiply-add or a comparison in the same loop;
+// 77 with the pipe saturated).  div() and root()
 // below take 117 and 115 clocks of integer issue when nothing else runs and
 // nothing at all beside FP64 arithmetic (four fused multiply-adds and a div()
 // take the 320 clocks of the four alone), so a kernel bound by the FP64 pipe
@@ -127,7 +128,7 @@ __device__ __forceinline__ double mul(double a, double b) {
   const uint32_t ea = ha & 0x7ff00000u, eb = hb & 0x7ff00000u;
   const bool zero = (((ha << 1) | la) == 0u) | (((hb << 1) | lb) == 0u);
   const bool na = ea - 0x00100000u < 0x7fe00000u, nb = eb - 0x00100000u < 0x7fe00000u;
-  // exponent fields' sum in (1024, 3069): a normal result either way of the shift
+  // exponent fields' sum in [1024, 3067]: a normal result either way of the shift
   const bool in = na & nb & (((ea >> 1) + (eb >> 1)) - 0x20000000u < 0x3fe00000u);
   if (!(in | (zero & (ea != 0x7ff00000u) & (eb != 0x7ff00000u)))) return a * b;
   const uint32_t Ah = __funnelshift_l(la, ha, 11) | 0x80000000u, Al = la << 11;

@@ -1,13 +1,12 @@
 // mf_riemann.cuh - face fluxes: Roe 8/7-wave MHD, Rusanov MHD, Dedner (GLM)
 // 2x2 system and van Leer flux-vector splitting of the neutral fluids.
 //
-// Each routine computes the same fluxes as the cited reference kernel.  The
-// FP64 budget of GB300 makes every FP64 instruction count, so repeated
-// divisions by one denominator become one reciprocal and multiplications,
-// square roots that are also needed as reciprocals come from rsqrt, and the
-// structurally zero entries of the 8x8 eigenmatrices are skipped.  These
-// change results only at the rounding level (continuous functions of their
-// inputs); the limiter and region decisions upstream stay bit-exact.
+// The FP32 fluxes of the mixed-precision paths, and in FP64 their HELIOBC faces
+// (the FP64 paths take mf_riemann_exact.cuh).  Each routine computes the same fluxes as the cited
+// reference kernel; repeated divisions by one denominator become one
+// reciprocal and multiplications, square roots that are also needed as
+// reciprocals come from rsqrt, and the structurally zero entries of the 8x8
+// eigenmatrices are skipped.  These change results only at the rounding level.
 #pragma once
 
 #include "mf_device.cuh"

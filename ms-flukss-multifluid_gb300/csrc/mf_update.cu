@@ -1,5 +1,6 @@
-// mf_update.cu - update kernel with the fast physics (contraction allowed,
-// reciprocals reused): the mixed-precision path and the fast FP64 path.
+// mf_update.cu - update kernel with the fast physics (mf_sources.cuh): the
+// mixed-precision paths and the fast FP64 path where the update does not run
+// by fluid (mf_cell.cu).
 #define MF_PHYS fast
 #include "mf_sources.cuh"
 #include "mf_update_kernel.cuh"
