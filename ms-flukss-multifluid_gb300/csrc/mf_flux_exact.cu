@@ -11,7 +11,8 @@ cudaError_t launch_flux_exact(const DevParams& P, int dir, const double* w, void
   const int tot = b.tot_f[dir];
   if (tot <= 0) return cudaSuccess;
   const int nt = b.nt[1];
-  const unsigned gf = flat_blocks(tot, nt);
+  const unsigned nb = flat_blocks(tot, nt);
+  const dim3 gf(nb, helio_parts<double>(P, nb));
   double* F = (double*)f;
   double* Bn = (double*)bn;
   if (dir == 0)

@@ -16,7 +16,8 @@ cudaError_t launch_flux_fast<double>(const DevParams& P, int dir, const double* 
   if (end < 0) end = b.tot_f[dir];
   if (end - first <= 0) return cudaSuccess;
   const int nt = b.nt[1];
-  const unsigned gf = flat_blocks(end - first, nt);
+  const unsigned nb = flat_blocks(end - first, nt);
+  const dim3 gf(nb, helio_parts<double>(P, nb));
   double* F = (double*)f;
   double* Bn = (double*)bn;
   if (dir == 0)

@@ -310,6 +310,29 @@ __device__ __forceinline__ int helio_side(const DevParams& P, const RunParams& R
   return (f == RP.dlo[DIR]) ? 0 : (f == RP.dhi[DIR] + 1) ? 1 : -1;
 }
 
+// With HELIOBC a warp with faces of the domain boundary, whose solver is
+// another one, and of the interior runs the two chains one after the other.
+// FP64 launches of at most a block per SM, which wait for the chain, therefore
+// run twice as many blocks, which find room: those of blockIdx.y 0 take the
+// interior faces, those of 1 the boundary's (fluxes of a 16^3 domain, two
+// stages, fast FP64: 520 -> 385 us; of 64^3, in blocks that fill the chip, the
+// idle halves would cost 3.38 -> 3.61 ms).
+template <typename R>
+inline unsigned helio_parts(const DevParams& P, unsigned blocks) {
+  if (sizeof(R) == sizeof(float) || !P.helio_bc) return 1;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  return blocks <= (unsigned)sms ? 2 : 1;
+}
+template <typename R, int DIR>
+__device__ __forceinline__ bool helio_other(const DevParams& P, const RunParams& RP, int i, int j,
+                                            int k) {
+  if (sizeof(R) == sizeof(float) || gridDim.y == 1) return false;
+  return (helio_side<DIR>(P, RP, i, j, k) >= 0) != (blockIdx.y == 1);
+}
+
 // Fluids whose fluxes a face takes here: where the neutral populations have a
 // launch of their own (neutrals_apart), those of a HELIOBC face alone.
 template <typename R>
@@ -337,6 +360,7 @@ __device__ __forceinline__ void flux_face(const DevParams& P, const double* __re
   fnb[DIR] += 1;
   int i, j, k;
   decode(lin, D.vlo, fnb, i, j, k);
+  if (helio_other<R, DIR>(P, RP, i, j, k)) return;
   const long long cs = (long long)D.fn[0] * D.fn[1] * D.fn[2];
   const long long st = (DIR == 0) ? 1 : (DIR == 1) ? (long long)D.fn[0]
                                                    : (long long)D.fn[0] * D.fn[1];
@@ -410,7 +434,8 @@ __device__ __forceinline__ void flux_face(const DevParams& P, const double* __re
     }
   }
   R g[9];
-  plasma_flux<R, DIR>(P, wl, wr, g);
+  if (sizeof(R) == sizeof(float) || helio_side<DIR>(P, RP, i, j, k) < 0)
+    plasma_flux<R, DIR>(P, wl, wr, g);  // (HELIOBC sets every one of these)
   if (P.glm) {
     R fbn, fpsi;
     dedner_2x2<R>(R(states[D.run].ch), wl[5 + DIR], wl[8], wr[5 + DIR], wr[8], fbn, fpsi);
@@ -535,7 +560,8 @@ __device__ __forceinline__ void riemann_face(const DevParams& P, const RunParams
     wr[v] = on ? R(fs(1, v)) : R(0);
   }
   R g[9];
-  plasma_flux<R, DIR>(P, wl, wr, g);
+  if (sizeof(R) == sizeof(float) || helio_side<DIR>(P, RP, i, j, k) < 0)
+    plasma_flux<R, DIR>(P, wl, wr, g);  // (HELIOBC sets every one of these)
   if (P.glm) {
     R fbn, fpsi;
     dedner_2x2<R>(R(states[D.run].ch), wl[5 + DIR], wl[8], wr[5 + DIR], wr[8], fbn, fpsi);
@@ -638,6 +664,7 @@ __global__ void __launch_bounds__(kMaxBlock)
   const long long cr = loc(D.slo, D.sn, i, j, k);
   const long long cl = cr - ((DIR == 0) ? 1 : (DIR == 1) ? (long long)D.sn[0]
                                                          : (long long)D.sn[0] * D.sn[1]);
+  if (helio_other<R, DIR>(P, RP, i, j, k)) return;
   const int nc = P.nc;
   riemann_face<R, DIR>(P, RP, D, i, j, k, W, F, Bn, states, [&](int side, int v) -> double {
     return side ? fv[v * scs + cr] : fv[(nc + v) * scs + cl];
@@ -796,7 +823,8 @@ cudaError_t launch_hflux_t(const DevParams& P, int dir, const double* w, const d
   const int tot = b.tot_f[dir];
   if (tot <= 0) return cudaSuccess;
   const int nt = b.nt[1];
-  const unsigned g = flat_blocks(tot, nt);
+  const unsigned nb = flat_blocks(tot, nt);
+  const dim3 g(nb, helio_parts<R>(P, nb));
   R* F = (R*)f;
   R* Bn = (R*)bn;
   if (dir == 0) k_hflux<R, 0><<<g, nt, 0, s>>>(P, w, fv, F, Bn, b.desc, b.ndesc, tot, b.runs, state);

@@ -294,9 +294,9 @@ inline bool flux_split(const DevParams& P, int precision) {
 // run first in launch_neutral_* and k_flux adds the plasma (HELIOBC faces: and
 // their own neutral fluxes).  Fluxes of a 16^3 patch's two stages in fast FP64
 // with tracking surfaces 380 -> 289 us, characteristic 659 -> 567; of 64^3 cells
-// 3.67 -> 3.11 ms (the step with characteristic limiting 8.07 -> 7.60).  Not where characteristic face values decide
-// the positivity fallback of the neutral ones (limited before the predictor in
-// the Hancock step).
+// 3.67 -> 3.11 ms (the step with characteristic limiting 8.07 -> 7.60).  Not
+// where characteristic face values decide the positivity fallback of the neutral
+// ones (limited before the predictor in the Hancock step).
 inline bool neutrals_apart(const DevParams& P, int precision, bool hancock) {
   return precision != MF_PREC_MIXED && !flux_split(P, precision) && P.nf > 1 &&
          (hancock || !(P.char_rec && P.check_pos));
